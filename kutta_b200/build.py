@@ -39,6 +39,7 @@ CXX_FLAGS = ["-O3", "-std=c++17", "-fPIC", "-ffp-contract=off", "-Wall", "-Wextr
 
 PRODUCT_CU = {
     "exact_kernels.cu": EXACT,
+    "coarse_rows.cu": EXACT,
     "mixed_kernels.cu": [],
     "tail_cycle.cu": [],
     "learned.cu": [],

@@ -151,15 +151,62 @@ __device__ __forceinline__ float product_error(float a, float b, float product) 
   return ((ah * bh - product) + ah * bl + al * bh) + al * bl;
 }
 
-// One term of the Neumaier + Dekker residual sum: sum -= v*x, with both the
-// addition error and the product error carried in `error`.
-__device__ __forceinline__ void residual_term(float& sum, float& error, float v, float x) {
-  const float product = v * x;
+// product_error by one FMA where that gives the same bits: away from
+// underflow Dekker's split and the FMA both return the exact error. The split's
+// smallest partial product has its last bit no lower than |a b| 2^-46, which
+// stays representable for |a b| >= 2^-96; below that, and beyond the split's
+// 1e30 guard, the split itself runs. (An overflowing product leaves NaN in the
+// sum's error term either way.)
+__device__ __forceinline__ float product_error_fma(float a, float b, float product) {
+  if (fabsf(product) >= 0x1p-96f && fabsf(a) <= 1.0e30f && fabsf(b) <= 1.0e30f)
+    return fmaf(a, b, -product);
+  return product_error(a, b, product);
+}
+
+// product_error_fma of N independent products with one branch for all, so
+// that their loads and products overlap.
+template <int N>
+__device__ __forceinline__ void products(const float (&a)[N], const float (&b)[N],
+                                         float (&product)[N], float (&error)[N]) {
+  bool fast = true;
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    product[k] = a[k] * b[k];
+    error[k] = fmaf(a[k], b[k], -product[k]);
+    fast = fast && fabsf(product[k]) >= 0x1p-96f && fabsf(a[k]) <= 1.0e30f &&
+           fabsf(b[k]) <= 1.0e30f;
+  }
+  if (!fast) {
+#pragma unroll
+    for (int k = 0; k < N; ++k) error[k] = product_error_fma(a[k], b[k], product[k]);
+  }
+}
+
+// One term of the Neumaier + Dekker residual sum: sum -= product, with both
+// the addition error and the product's error carried in `error`.
+__device__ __forceinline__ void residual_add(float& sum, float& error, float product,
+                                             float product_error) {
   const float term = -product;
   const float next = sum + term;
   error += fabsf(sum) >= fabsf(term) ? (sum - next) + term : (term - next) + sum;
-  error -= product_error(v, x, product);
+  error -= product_error;
   sum = next;
+}
+__device__ __forceinline__ void residual_term(float& sum, float& error, float v, float x) {
+  const float product = v * x;
+  residual_add(sum, error, product, product_error_fma(v, x, product));
+}
+
+// amg_smooth_zero's row (linalg.kern.h:162-170): the caller has just cleared x,
+// so only a nonfinite b takes the ordinary path, with x = 0.
+__device__ __forceinline__ float zero_sweep_row(int i, const int* __restrict__ rows,
+                                                const float* __restrict__ vals, float bi,
+                                                float inv) {
+  if (!nonfinite(bi)) return 0.0f + (2.0f / 3.0f) * inv * (bi + 0.0f);
+  float sum = bi, error = 0.0f;
+  const int end = rows[i + 1];
+  for (int j = rows[i]; j < end; ++j) residual_term(sum, error, vals[j], 0.0f);
+  return 0.0f + (2.0f / 3.0f) * inv * (sum + error);
 }
 
 // One term of the Kahan SpMV sum (csr_spmv).

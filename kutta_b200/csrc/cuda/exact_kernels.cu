@@ -190,18 +190,6 @@ __global__ void k_residual(int n, const int* __restrict__ rows, const int* __res
   }
 }
 
-// amg_smooth_zero's row (linalg.kern.h:162-170): the caller has just cleared x,
-// so only a nonfinite b takes the ordinary path, with x = 0.
-__device__ __forceinline__ float zero_sweep_row(int i, const int* __restrict__ rows,
-                                                const float* __restrict__ vals, float bi,
-                                                float inv) {
-  if (!nonfinite(bi)) return 0.0f + (2.0f / 3.0f) * inv * (bi + 0.0f);
-  float sum = bi, error = 0.0f;
-  const int end = rows[i + 1];
-  for (int j = rows[i]; j < end; ++j) residual_term(sum, error, vals[j], 0.0f);
-  return 0.0f + (2.0f / 3.0f) * inv * (sum + error);
-}
-
 // amg_smooth (linalg.kern.h:150-156) and amg_smooth_zero (:162-170).
 template <bool kZero>
 __global__ void k_smooth(int n, const int* __restrict__ rows, const int* __restrict__ cols,
@@ -415,26 +403,43 @@ __global__ void k_pack_rows(int n, int width, const int* __restrict__ rows,
   }
 }
 
-// amg_coarse_solve, linalg.kern.h:126-147: whole <=24-row system in one thread.
+// amg_coarse_solve, linalg.kern.h:126-147: the whole <=24-row system in one
+// warp, a lane per row. Each lane sums its row in CSR order and the iterate is
+// exchanged through shared memory, so every value is the one-thread form's;
+// the operator is read once into shared memory. 32 sweeps of 8 rows took
+// 67 us in one thread (each entry a dependent load).
 __global__ void k_coarse_solve(int count, const int* __restrict__ rows,
                                const int* __restrict__ cols, const float* __restrict__ vals,
                                float* __restrict__ x, const float* __restrict__ b,
                                const float* __restrict__ inv, const int* __restrict__ status,
                                int sweeps) {
   pdl_entry();
-  if (threadIdx.x != 0 || blockIdx.x != 0 || status[0] != 0) return;
-  float current[24], r[24];
-  for (int row = 0; row < count; ++row) current[row] = 0.0f;
-  for (int sweep = 0; sweep < sweeps; ++sweep) {
-    for (int row = 0; row < count; ++row) {
-      float sum = b[row], error = 0.0f;
-      for (int j = rows[row]; j < rows[row + 1]; ++j)
-        residual_term(sum, error, vals[j], current[cols[j]]);
-      r[row] = sum + error;
-    }
-    for (int row = 0; row < count; ++row) current[row] += (2.0f / 3.0f) * inv[row] * r[row];
+  if (status[0] != 0) return;
+  constexpr int kMost = 24;
+  __shared__ float current[kMost];
+  __shared__ int col[kMost * kMost];
+  __shared__ float val[kMost * kMost];
+  const int row = threadIdx.x;
+  const bool owner = row < count;
+  const int nnz = rows[count];
+  for (int j = row; j < nnz; j += 32) {
+    col[j] = cols[j];
+    val[j] = vals[j];
   }
-  for (int row = 0; row < count; ++row) x[row] = current[row];
+  if (owner) current[row] = 0.0f;
+  const int begin = owner ? rows[row] : 0, end = owner ? rows[row + 1] : 0;
+  const float right = owner ? b[row] : 0.0f, scale = owner ? inv[row] : 0.0f;
+  __syncwarp();
+  for (int sweep = 0; sweep < sweeps; ++sweep) {
+    float sum = right, error = 0.0f;
+#pragma unroll 4
+    for (int j = begin; j < end; ++j) residual_term(sum, error, val[j], current[col[j]]);
+    const float r = sum + error;
+    __syncwarp();
+    if (owner) current[row] += (2.0f / 3.0f) * scale * r;
+    __syncwarp();
+  }
+  if (owner) x[row] = current[row];
 }
 
 // krylov_diagonal, linalg.kern.h:52-70, with the refresh's max_abs check of the
@@ -457,24 +462,6 @@ __global__ void k_diagonal(int n, const int* __restrict__ rows, const int* __res
 }
 
 // ---- AMG transfer and Galerkin, src/kutta/kernels/amg.kern.h ------------------
-// amg_restrict(_guarded) :5-16,84-87: Kahan sum over the aggregate's members.
-__global__ void k_restrict(int nc, const int* __restrict__ offsets,
-                           const int* __restrict__ members, const float* __restrict__ fine,
-                           float* __restrict__ coarse, const int* __restrict__ status) {
-  pdl_entry();
-  if (status[0] != 0) return;
-  ROWS(g, nc) {
-    float sum = 0.0f, error = 0.0f;
-    for (int j = offsets[g]; j < offsets[g + 1]; ++j) {
-      const float term = fine[members[j]] - error;
-      const float next = sum + term;
-      error = (next - sum) - term;
-      sum = next;
-    }
-    coarse[g] = sum;
-  }
-}
-
 // amg_prolong(_guarded) :18-21,88-91.
 __global__ void k_prolong(int nf, const int* __restrict__ aggregate,
                           const float* __restrict__ coarse, float* __restrict__ fine,
@@ -844,12 +831,6 @@ void diagonal(int n, const int* rows, const int* diag, const float* vals, float*
               int use_l1, DeviceReducer red, double* check, int slot, cudaStream_t s) {
   ++counter;
   pdl(k_diagonal, blocks(n), kBlock, 0, s, n, rows, diag, vals, inverse, use_l1, red, check, slot);
-}
-void restrict_(int nc, const int* offsets, const int* members, const float* fine, float* coarse,
-               const int* status, cudaStream_t s) {
-  if (nc <= 0) return;
-  ++counter;
-  pdl(k_restrict, blocks(nc), kBlock, 0, s, nc, offsets, members, fine, coarse, status);
 }
 void prolong(int nf, const int* aggregate, const float* coarse, float* fine, const int* status,
              cudaStream_t s) {

@@ -88,7 +88,7 @@ void smooth(int n, const int* rows, const int* cols, const float* vals, const fl
 void smooth_dot2(int n, const int* rows, const int* cols, const float* vals, const float* x,
                  const float* b, const float* inv, float* next, const float* q, DeviceReducer red,
                  float* scalars, int offset, int* status, Epilogue epi, cudaStream_t s);
-// <=24-row coarsest level, `sweeps` Jacobi sweeps in one thread (amg_coarse_solve).
+// <=24-row coarsest level, `sweeps` Jacobi sweeps in one warp (amg_coarse_solve).
 void coarse_solve(int count, const int* rows, const int* cols, const float* vals, float* x,
                   const float* b, const float* inv, const int* status, int sweeps,
                   cudaStream_t s);
@@ -98,8 +98,6 @@ void diagonal(int n, const int* rows, const int* diag, const float* vals, float*
               int use_l1, DeviceReducer red, double* check, int slot, cudaStream_t s);
 
 // ---- AMG transfer and Galerkin --------------------------------------------
-void restrict_(int nc, const int* offsets, const int* members, const float* fine, float* coarse,
-               const int* status, cudaStream_t s);
 void prolong(int nf, const int* aggregate, const float* coarse, float* fine, const int* status,
              cudaStream_t s);
 void galerkin(int nnz_c, const int* offsets, const int* entries, const float* fine, float* coarse,
@@ -108,6 +106,51 @@ void galerkin(int nnz_c, const int* offsets, const int* entries, const float* fi
 void m_matrix_diagonal(int nf, int nc, const int* offsets, const int* members, const int* fine_rows,
                        const int* fine_diag, const float* fine, const int* rows, const int* diag,
                        float* coarse, float* surplus, cudaStream_t s);
+
+// ---- plain coarse levels (coarse_rows.cu) -----------------------------------
+// The residual and sweep above for levels with long rows or few of them (the
+// same bits): all threads of a block form the products of its rows' entries,
+// one thread per row adds them. They load the operator before they wait for
+// the previous kernel, so that kernel must not be its writer. At most
+// kStagedSmall rows take blocks of 64 rows, more take 128 (see staged()).
+constexpr int kStagedSmall = 16384;
+void staged_residual(int n, const int* rows, const int* cols, const float* vals, const float* x,
+                     const float* b, float* r, const int* status, cudaStream_t s);
+// With aggregate != null the sweep starts from x + coarse[aggregate] (the
+// prolongation folded in; x itself is left as it is).
+void staged_smooth(int n, const int* rows, const int* cols, const float* vals, const float* x,
+                   const float* b, const float* inv, float* next, const int* status,
+                   const int* aggregate, const float* coarse, cudaStream_t s);
+// b_c = the Kahan sum of each aggregate's members of `fine`; with next != null the coarse level's zero-start sweep too.
+void restrict_rows(int nc, const int* offsets, const int* members, const float* fine,
+                   float* coarse, const int* rows, const float* vals, const float* inv,
+                   float* next, const int* status, cudaStream_t s);
+// The V-cycle of the smallest levels in one block: level[0].b restricted from
+// `fine`, the residual of the level above; its correction into `out`.
+constexpr int kPlainTailRows = 2048, kPlainTailSlots = 16384;
+constexpr int kPlainTailBytes = 227 * 1024;  // shared memory of a block
+struct PlainTail {
+  static constexpr int kMaxLevels = 16;
+  struct Level {
+    int n, at;                          // at: first float of its x, y and b
+    int slots, slot;                    // entries in slices of 32 rows; the first
+    const int* source;                  // CSR entry of each slot, -1 for padding
+    const int *order, *start;           // rows, longest first, and their first slots
+    const int *rows, *cols;
+    const float *vals, *inv;
+    const int *offsets, *members;       // aggregates of the level above
+    const int* aggregate;               // to the level below (null on the last)
+  };
+  Level level[kMaxLevels];
+  int levels, pre, post, coarsest;
+  int floats, slots;                    // of all levels
+  float2* entries;                      // value and 4 * column of each slot
+};
+// Writes t.entries from the levels' current values.
+void plain_tail_entries(const PlainTail& t, cudaStream_t s);
+int plain_tail_bytes(int floats, int slots);
+void plain_tail(const PlainTail& t, const float* fine, float* out, const int* status,
+                cudaStream_t s);
 
 // ---- Krylov vector updates (guarded by status) ----------------------------
 // x += a p; r -= a q; then r.r -> scalars[18] and solver_check(pcg = 1).

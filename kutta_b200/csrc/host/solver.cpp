@@ -155,8 +155,105 @@ Solver::Solver(Kind kind, const CsrView& a, const Options& options,
     choose_coarsest(host_values_[1]);
     if (options_.fused_tail && options_.coarse_bf16 && !nullspace_) plan_tail();
     if (options_.packed_fine) plan_packed(a, s);
+  } else if (amg()) {
+    plan_plain(s);
   }
   wait(s);
+}
+
+std::vector<int> Solver::row_pointers(const DevLevel& l, cudaStream_t s) {
+  std::vector<int> rows(static_cast<std::size_t>(l.n) + 1);
+  cuda_check(cudaMemcpyAsync(rows.data(), l.row_ptr.get(), sizeof(int) * rows.size(),
+                             cudaMemcpyDeviceToHost, s),
+             "row lengths");
+  wait(s);
+  return rows;
+}
+
+// Staged row kernels measured faster than a thread per row on every level of
+// at most 65,536 rows (512 rows: 1.8 against 2.5 us per sweep; 12,571 rows
+// with a longest of 165: 3.8 against 18.4 us; 48,848 with 123: 5.2 against 18.8
+// us) and, above, on levels whose longest row has more than 8 entries (159,785
+// rows of up to 18: 5.6 against 8.6 us). Short rows on many threads are faster
+// direct (262,144 rows of up to 7: 5.0 against 6.7 us). The one-block tail takes
+// the levels from the first with at most kPlainTailRows rows and
+// kPlainTailSlots entries: beyond that one SM is slower than a launch per
+// sweep.
+void Solver::plan_plain(cudaStream_t s) {
+  constexpr int kDirectRows = 1 << 16, kDirectLongest = 8;
+  for (std::size_t i = 0; i < levels_.size(); ++i) {
+    auto& l = levels_[i];
+    l.staged = l.n <= kDirectRows;
+    if (i == 0 || l.staged) continue;
+    const std::vector<int> rows = row_pointers(l, s);
+    for (int k = 0; k < l.n && !l.staged; ++k) l.staged = rows[k + 1] - rows[k] > kDirectLongest;
+  }
+  if (nullspace_ || options_.cycle != Cycle::V) return;
+  launch::PlainTail t{};
+  std::size_t start = levels_.size();
+  while (start > 1 && levels_.size() - start < launch::PlainTail::kMaxLevels) {
+    auto& l = levels_[start - 1];
+    if (l.n > launch::kPlainTailRows || l.nnz > launch::kPlainTailSlots) break;
+    // Rows in order of length, their entries in slices of 32 rows.
+    const std::vector<int> rows = row_pointers(l, s);
+    std::vector<int> order(static_cast<std::size_t>(l.n)), first(order.size());
+    std::iota(order.begin(), order.end(), 0);
+    std::stable_sort(order.begin(), order.end(), [&](int p, int q) {
+      return rows[p + 1] - rows[p] > rows[q + 1] - rows[q];
+    });
+    int slots = 0;
+    for (int k = 0; k < l.n; k += 32) slots += 32 * (rows[order[k] + 1] - rows[order[k]]);
+    const int floats = t.floats + 3 * l.n;
+    if (launch::plain_tail_bytes(floats, t.slots + slots) > launch::kPlainTailBytes) break;
+    std::vector<int> source(static_cast<std::size_t>(slots), -1);
+    for (int k = 0, slice = 0; k < l.n; ++k) {
+      const int i = order[k], lane = k % 32;
+      if (k > 0 && lane == 0) slice += 32 * (rows[order[k - 32] + 1] - rows[order[k - 32]]);
+      first[k] = slice + lane;
+      for (int j = rows[i]; j < rows[i + 1]; ++j)
+        source[static_cast<std::size_t>(first[k] + 32 * (j - rows[i]))] = j;
+    }
+    l.tail_order.upload(order, s);
+    l.tail_start.upload(first, s);
+    l.tail_source.upload(source, s);
+    wait(s);  // the host arrays are released here
+    t.floats = floats;
+    t.slots += slots;
+    --start;
+  }
+  if (start == levels_.size()) return;
+  t.levels = static_cast<int>(levels_.size() - start);
+  t.pre = options_.pre_sweeps;
+  t.post = options_.post_sweeps;
+  t.coarsest = options_.coarse_sweeps;
+  int at = 0, slot = 0;
+  for (int k = 0; k < t.levels; ++k) {
+    const auto& above = levels_[start + static_cast<std::size_t>(k) - 1];
+    const auto& l = levels_[start + static_cast<std::size_t>(k)];
+    auto& v = t.level[k];
+    v.n = l.n;
+    v.at = at;
+    v.slots = static_cast<int>(l.tail_source.size());
+    v.slot = slot;
+    v.source = l.tail_source.get();
+    v.order = l.tail_order.get();
+    v.start = l.tail_start.get();
+    v.rows = l.row_ptr.get();
+    v.cols = l.col.get();
+    v.vals = l.val.get();
+    v.inv = l.l1.get();
+    v.offsets = above.member_offsets.get();
+    v.members = above.members.get();
+    v.aggregate = k + 1 == t.levels ? nullptr : l.aggregate.get();
+    at += 3 * l.n;
+    slot += v.slots;
+    plain_tail_bytes_ += 8.0 * l.nnz + 28.0 * l.n;
+  }
+  plain_tail_entries_.reset(static_cast<std::size_t>(t.slots));
+  t.entries = plain_tail_entries_.get();
+  launch::plain_tail_entries(t, s);
+  plain_tail_ = t;
+  plain_tail_start_ = start;
 }
 
 // The packed rows' pattern: each row's off-diagonal column offsets in column
@@ -406,9 +503,10 @@ void Solver::reset(int iterations) { launch::solver_reset(scalars_.get(), status
 
 // ------------------------------------------------------------ preconditioner --
 void Solver::smooth(DevLevel& l, const int* rows, const int* cols, const float* vals,
-                    const float* b, float*& x, int sweeps, bool zero_start, const int* status) {
+                    const float* b, float*& x, int sweeps, bool zero_start, const int* status,
+                    bool swept, const float* coarse) {
   const bool fine = &l == &levels_[0];
-  for (int sweep = 0; sweep < sweeps; ++sweep) {
+  for (int sweep = swept ? 1 : 0; sweep < sweeps; ++sweep) {
     const bool zero = zero_start && sweep == 0;
     // Every 8th fine-level sweep is bracketed by events: enough samples for the
     // average launch time, little added host work inside a timed solve.
@@ -440,6 +538,9 @@ void Solver::smooth(DevLevel& l, const int* rows, const int* cols, const float* 
     else if (with_dots)
       launch::smooth_dot2(l.n, rows, cols, vals, x, b, l.l1.get(), l.r, q_, reducer(),
                           scalars_.get(), 4, status_.get(), Epilogue::PcgBetaFlexible, stream_);
+    else if (l.staged && !zero)
+      launch::staged_smooth(l.n, rows, cols, vals, x, b, l.l1.get(), l.r, status,
+                            sweep == 0 && coarse ? l.aggregate.get() : nullptr, coarse, stream_);
     else
       launch::smooth(l.n, rows, cols, vals, x, b, l.l1.get(), l.r, status, zero, stream_);
     if (timed) cuda_check(cudaEventRecord(events_[events_used_++], stream_), "cudaEventRecord");
@@ -449,7 +550,8 @@ void Solver::smooth(DevLevel& l, const int* rows, const int* cols, const float* 
 }
 
 // Aggregation::cycle, amg.cpp:283-310.
-void Solver::cycle(std::size_t index, const float* b, float*& x, const int* status) {
+void Solver::cycle(std::size_t index, const float* b, float*& x, const int* status,
+                   bool swept) {
   auto& l = levels_[index];
   const int* rows = l.row_ptr.get();
   const int* cols = l.col.get();
@@ -478,33 +580,50 @@ void Solver::cycle(std::size_t index, const float* b, float*& x, const int* stat
       launch::coarse_solve(l.n, rows, cols, vals, x, b, l.l1.get(), status,
                            options_.coarse_sweeps, stream_);
     } else {
-      smooth(l, rows, cols, vals, b, x, options_.coarse_sweeps, true, status);
+      smooth(l, rows, cols, vals, b, x, options_.coarse_sweeps, true, status, swept);
     }
   } else {
-    smooth(l, rows, cols, vals, b, x, options_.pre_sweeps, true, status);
+    smooth(l, rows, cols, vals, b, x, options_.pre_sweeps, true, status, swept);
     if (l.v16.allocated())
       launch::bf16_residual(l.n, rows, cols, l.v16.get(), l.scale.get(), x, b, l.r, status,
                             stream_);
     else if (index == 0 && packed_.width > 0)
       launch::packed_residual(l.n, packed(), x, b, l.r, status, stream_);
+    else if (l.staged)
+      launch::staged_residual(l.n, rows, cols, vals, x, b, l.r, status, stream_);
     else
       launch::residual(l.n, rows, cols, vals, x, b, l.r, status, stream_);
     auto& c = levels_[index + 1];
-    if (mixed())
+    const bool inner_next =
+        options_.cycle == Cycle::K && index + 2 < levels_.size() && inner_level(index + 1);
+    const bool tail_next = plain_tail_start_ != 0 && index + 1 == plain_tail_start_;
+    // The coarse level's zero-start sweep rides on the restriction that writes
+    // its right-hand side, unless something comes between or there is none.
+    const bool sweep_next = !mixed() && !nullspace_ && !inner_next &&
+                            (index + 2 < levels_.size() || c.n > 24);
+    if (tail_next) {
+      launch::plain_tail(plain_tail_, l.r, c.x, status, stream_);
+      tally(plain_tail_bytes_);
+    } else if (!mixed()) {
+      launch::restrict_rows(c.n, l.member_offsets.get(), l.members.get(), l.r, c.b.get(),
+                            c.row_ptr.get(), c.val.get(), c.l1.get(), sweep_next ? c.r : nullptr,
+                            status, stream_);
+      if (sweep_next) std::swap(c.x, c.r);
+    } else
       launch::restrict_lanes(c.n, l.member_offsets.get(), l.members.get(), l.r, c.b.get(), status,
                              stream_);
-    else
-      launch::restrict_(c.n, l.member_offsets.get(), l.members.get(), l.r, c.b.get(), status,
-                        stream_);
     tally(8.0 * l.nnz + 4.0 * (l.n + 1) + 12.0 * l.n + 4.0 * (c.n + 1) + 8.0 * l.n + 4.0 * c.n);
     if (nullspace_) project(c.b.get(), c.n, c.projection.get());
-    if (options_.cycle == Cycle::K && index + 2 < levels_.size() && inner_level(index + 1))
+    if (inner_next)
       inner(index + 1, status);
-    else
-      cycle(index + 1, c.b.get(), c.x, status);
-    launch::prolong(l.n, l.aggregate.get(), c.x, x, status, stream_);
+    else if (!tail_next)
+      cycle(index + 1, c.b.get(), c.x, status, sweep_next);
+    // On staged levels the first post-sweep adds the correction as it reads x.
+    const bool fold = l.staged && options_.post_sweeps > 0;
+    if (!fold) launch::prolong(l.n, l.aggregate.get(), c.x, x, status, stream_);
     tally(12.0 * l.n + 4.0 * c.n);
-    smooth(l, rows, cols, vals, b, x, options_.post_sweeps, false, status);
+    smooth(l, rows, cols, vals, b, x, options_.post_sweeps, false, status, false,
+           fold ? c.x : nullptr);
   }
   if (nullspace_ && index != 0) project(x, l.n, l.projection.get());
 }
@@ -810,6 +929,7 @@ void Solver::refresh_levels(const float* val, bool fine_done, cudaStream_t s) {
   if (packed_.width > 0)
     launch::pack_rows(n_, packed_.width, rows0(), cols0(), levels_[0].diag.get(), val,
                       packed_.vals.get(), packed_.diag.get(), s);
+  if (plain_tail_start_ != 0) launch::plain_tail_entries(plain_tail_, s);
   if (mixed()) prepare_mixed(s, slots);
   cuda_check(cudaMemcpyAsync(host_values_.get(), values_.get(),
                              sizeof(double) * (slots + (mixed() ? 2 : 0)), cudaMemcpyDeviceToHost, s),

@@ -82,6 +82,11 @@ struct DevLevel {
   DArray<unsigned short> v16;
   DArray<float> scale;
   DArray<double> dense_lower, dense_inverse;
+  // The plain solve's row kernels form the row's products with all threads of a
+  // block (launch::staged_smooth) instead of a thread per row.
+  bool staged = false;
+  // Levels of the one-block tail (launch::PlainTail::Level).
+  DArray<int> tail_order, tail_start, tail_source;
   // transfer to level + 1
   DArray<int> aggregate, member_offsets, members, entry_offsets, entries;
 };
@@ -149,6 +154,14 @@ class Solver {
   std::size_t tail_start_ = 0;
   double tail_bytes_ = 0;
   launch::TailPlan tail_{};
+  // The plain V-cycle's choice of row kernels per level, and its smallest
+  // levels (>= plain_tail_start_, 0: none) in one block.
+  void plan_plain(cudaStream_t s);
+  static std::vector<int> row_pointers(const DevLevel& l, cudaStream_t s);
+  std::size_t plain_tail_start_ = 0;
+  double plain_tail_bytes_ = 0;
+  launch::PlainTail plain_tail_{};
+  DArray<float2> plain_tail_entries_;
   bool mixed() const { return options_.coarse_bf16 || options_.dense_coarsest; }
   // The mixed solve's packed copy of the fine operator (width 0: CSR kernels).
   struct Packed {
@@ -246,10 +259,13 @@ class Solver {
   cudaStream_t capture_ = nullptr;
   // Work queued by cycle/smooth/inner is skipped on the device while
   // status[0] != 0 (the outer solve's status, or a K-cycle level's own).
-  void cycle(std::size_t index, const float* b, float*& x, const int* status);
+  // swept: the level's first (zero-start) sweep is already in x.
+  void cycle(std::size_t index, const float* b, float*& x, const int* status,
+             bool swept = false);
   void inner(std::size_t index, const int* parent);
   void smooth(DevLevel& l, const int* rows, const int* cols, const float* vals, const float* b,
-              float*& x, int sweeps, bool zero_start, const int* status);
+              float*& x, int sweeps, bool zero_start, const int* status, bool swept = false,
+              const float* coarse = nullptr);
   void reduce_into(ReduceMode mode, int n, const float* x, const float* y, const float* u,
                    const float* v, float* scalars, int offset, const int* guard);
 

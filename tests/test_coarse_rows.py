@@ -1,0 +1,108 @@
+"""The plain solve's coarse-level kernels (kutta_b200/csrc/cuda/coarse_rows.cu):
+rows whose products a block forms together, the folded transfers and the small
+levels in one block must give the thread-per-row kernels' values, so whole
+solves must match the oracle as before; and one FMA must give the bits of the
+reference's split product error wherever it is used for it."""
+import numpy as np
+import pytest
+
+from kutta_b200 import harness
+from kutta_b200 import linalg as L
+from oracle import kutta_oracle as O
+
+M = L.OperatorStructure.SymmetricMMatrix
+f32 = np.float32
+
+
+def _split_error(a, b, product):
+    """Dekker's product error with the 4097 split, in float32 throughout."""
+    ca, cb = f32(4097) * a, f32(4097) * b
+    ah, bh = ca - (ca - a), cb - (cb - b)
+    al, bl = a - ah, b - bh
+    return ((ah * bh - product) + ah * bl + al * bh) + al * bl
+
+
+@pytest.mark.parametrize("low, high", [(-96, -90), (-60, 60), (60, 126)])
+def test_fma_error_equals_split_error_above_2_to_minus_96(low, high):
+    """For |a b| >= 2^-96 and factors up to 1e30 both are the exact error: a b
+    has 48 bits, so float64 holds the product and its difference exactly."""
+    rng = np.random.default_rng(low + 200)
+    n = 400_000
+    exponent = rng.integers(low, high, n)
+    share = rng.integers(-40, 41, n)
+    ea = np.clip(exponent // 2 + share, -126, 99)
+    eb = np.clip(exponent - ea, -126, 99)
+    a = np.ldexp(rng.uniform(1, 2, n), ea).astype(f32) * rng.choice([f32(-1), f32(1)], n)
+    b = np.ldexp(rng.uniform(1, 2, n), eb).astype(f32)
+    with np.errstate(over="ignore", invalid="ignore"):
+        product = a * b
+        used = np.isfinite(product) & (np.abs(product) >= f32(2.0 ** -96)) & \
+            (np.abs(a) <= f32(1e30)) & (np.abs(b) <= f32(1e30))
+        a, b, product = a[used], b[used], product[used]
+        split = _split_error(a, b, product)
+    exact = a.astype(np.float64) * b.astype(np.float64) - product.astype(np.float64)
+    assert len(a) > n // 8
+    assert np.array_equal(exact.astype(f32).astype(np.float64), exact)  # one FMA returns it
+    assert np.array_equal(split, exact.astype(f32))
+
+
+def _hub(n, degree, hubs, seed):
+    """An M-matrix with a few rows of `degree` entries among rows of 3 to 6."""
+    rng = np.random.default_rng(seed)
+    pairs = {(i, i + 1) for i in range(n - 1)}
+    for h in rng.choice(n, hubs, replace=False):
+        for j in rng.choice(n, degree, replace=False):
+            if h != j:
+                pairs.add((min(h, j), max(h, j)))
+    i, j = np.array(sorted(pairs)).T
+    w = np.exp(rng.uniform(-3, 0, len(i))).astype(f32).astype(np.float64)
+    row = np.concatenate([i, j, np.arange(n)])
+    col = np.concatenate([j, i, np.arange(n)])
+    total = np.bincount(np.concatenate([i, j]), np.concatenate([w, w]), n) * 1.001 + 1e-3
+    diagonal = np.nextafter(total.astype(f32), f32(np.inf)).astype(np.float64)
+    val = np.concatenate([-w, -w, diagonal])
+    order = np.lexsort((col, row))
+    row, col, val = row[order], col[order].astype(np.int32), val[order]
+    row_ptr = np.concatenate([[0], np.cumsum(np.bincount(row, minlength=n))]).astype(np.int32)
+    diag = np.nonzero(row == col)[0].astype(np.int32)
+    return harness.HostSystem(row_ptr, col, diag, val, rng.standard_normal(n).astype(f32))
+
+
+CASES = {
+    # Rows at and around a block's 32, 64 and 128, and one small level only.
+    **{f"poisson{n}": lambda n=n: harness.poisson(n, 1) for n in (25, 33, 64, 65, 129, 257)},
+    "poisson2d": lambda: harness.poisson(47, 43, 1, 100.0),
+    # The one-block levels' edges: 2,048 and 2,049 rows below the fine level.
+    "hex": lambda: harness.box_system(27, 23, 26, tet=False, seed=4),
+    "tet": lambda: harness.box_system(13, 17, 11, tet=True, seed=5),
+    # Rows longer than what a block stages at once (1,024 and 2,048 entries).
+    "hub_small": lambda: _hub(3_000, 1_400, 3, 1),
+    "hub_large": lambda: _hub(20_000, 5_000, 4, 2),
+}
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("point", [False, True], ids=["", "point"])
+@pytest.mark.parametrize("name", CASES)
+def test_solve_matches_oracle(cuda, name, point):
+    """point: a single source, whose iterates are zero or tiny far from it, so
+    that products fall below 2^-96, where the split itself runs. x within
+    relative 1e-5 and equal iterations, as the solver parity tests require (the
+    FP64 reductions alone may round otherwise)."""
+    import torch
+    s = CASES[name]()
+    b = s.b.astype(f32)
+    if point:
+        b = np.zeros(s.n, f32)
+        b[s.n // 3] = 1
+    a = L.upload(s)
+    solver = L.make_amg_solver(L.SolverKind.AmgPcg, s, L.AmgOptions(structure=M, pre_sweeps=3,
+                                                                    post_sweeps=3))
+    solver.refresh(a)
+    x = torch.zeros(s.n, device="cuda")
+    st = solver.solve(a, x, torch.from_numpy(b).cuda(), L.SolveControl(1e-4, 1e-38, 200))
+    o = O.solve(s, O.AMG_PCG, m_matrix=True, b=b, rel_tol=1e-4, abs_tol=1e-38, max_iter=200,
+                opts=O.options(O.AMG_PCG, pre_sweeps=3, post_sweeps=3, m_matrix=True))
+    got = x.cpu().numpy().astype(np.float64)
+    assert (st.iterations, st.converged) == (o.iterations, o.converged)
+    assert np.linalg.norm(got - o.x) <= 1e-5 * np.linalg.norm(o.x.astype(np.float64))
