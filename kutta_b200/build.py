@@ -48,6 +48,7 @@ PRODUCT_CU = {
     "fv_kernels.cu": EXACT,
     "noalloc.cu": [],
     "coupled_kernels.cu": EXACT,
+    "coupled_coarse.cu": EXACT,
 }
 PRODUCT_CPP = ["host/setup.cpp", "host/solver.cpp", "host/device_setup.cpp", "host/mixed.cpp",
                "host/learned.cpp", "host/coupled_setup.cpp", "host/coupled.cpp", "capi.cpp"]

@@ -994,14 +994,22 @@ int b2_coupled_level_copy(const b2_coupled* s, int level, int32_t* rows, int32_t
     read_back(rows, l.rows, n + 1, st);
     read_back(cols, l.cols, nnz, st);
     read_back(diag, l.diag, n, st);
-    read_back(a, static_cast<const float*>(l.a), nnz, st);
-    read_back(c_out, static_cast<const float*>(l.c), nnz, st);
-    read_back(g, static_cast<const float*>(l.g), 3 * nnz, st);
-    read_back(h, static_cast<const float*>(l.h), 3 * nnz, st);
+    // The device keeps one record (a, gx, gy, gz, c, hx, hy, hz) per entry.
+    std::vector<float> entry(a || c_out || g || h ? 8 * nnz : 0);
+    read_back(entry.data(), reinterpret_cast<const float*>(l.entry), entry.size(), st);
     read_back(d, static_cast<const float*>(l.d), 11 * n, st);
     read_back(aggregate, c.transfer(level - 1).aggregate,
               static_cast<std::size_t>(c.level_rows(level - 1)), st);
     kb2::wait(st);
+    for (std::size_t e = 0; e < nnz && !entry.empty(); ++e) {
+      const float* v = &entry[8 * e];
+      if (a) a[e] = v[0];
+      if (c_out) c_out[e] = v[4];
+      for (std::size_t k = 0; k < 3; ++k) {
+        if (g) g[k * nnz + e] = v[1 + k];
+        if (h) h[k * nnz + e] = v[5 + k];
+      }
+    }
   });
 }
 

@@ -50,18 +50,24 @@ struct CoupledFine {
   const float4* face;   // per face: (sx, sy, sz, Rhie-Chow coefficient)
 };
 
-// One coarse level: CSR with a, c per entry, G and H as 3 nnz [x | y | z],
-// and 11 planes of n per row (du dv dw cs iu iv iw hx iu hy iv hz iw schur).
+// One coarse level: CSR with two float4 per entry, (a, gx, gy, gz) and
+// (c, hx, hy, hz) (a of a diagonal entry is 0: its momentum part is in d), and
+// 11 planes of n per row (du dv dw cs iu iv iw hx iu hy iv hz iw schur).
 struct CoupledLevel {
   int n = 0, nnz = 0;
   const int* rows = nullptr;
   const int* cols = nullptr;
   const int* diag = nullptr;
-  float *a = nullptr, *c = nullptr, *g = nullptr, *h = nullptr, *d = nullptr;
-  // Rows long enough (a hub aggregate bordering a hundred others) that the
-  // separately launched row kernels give each row a warp instead of a
-  // thread; the results are the same bits either way.
-  int wide = 0;
+  float4* entry = nullptr;
+  float* d = nullptr;
+  // The contributions of each entry's Galerkin sum, in the reference's order:
+  // terms [term_at[e], term_at[e + 1]). From the fine level a term is an ELL slot
+  // of the fine operator, from a coarse one 2 * entry, + 1 for a diagonal entry;
+  // ~row says that a member row's own data comes next (diagonal entries only,
+  // whose lists begin with one).
+  const int* term_at = nullptr;
+  const int* terms = nullptr;
+  const int* term_faces = nullptr;  // from the fine level: each term's face
 };
 
 // Level k -> k+1: aggregate of each fine row, member lists of each coarse row.
@@ -71,22 +77,19 @@ struct CoupledTransfer {
   const int* members = nullptr;
 };
 
-// The V-cycle of the small coarse levels (by default each at most kMaxRows
-// rows; the kernel itself takes any size, its block looping over the rows) as
-// one single-block launch: levels 0 .. levels-1 of the tail, the first receiving
-// its right-hand side from the level above; x/tmp are each level's current
-// ping-pong roles.
+// The V-cycle of the small coarse levels, each of at most kMaxRows rows and
+// kMaxEntries entries, as one single-block launch: levels 0 .. levels-1 of the
+// tail, the first one's right-hand side from b, its correction into x.
 struct CoupledTail {
-  static constexpr int kMaxLevels = 12;
-  static constexpr int kMaxRows = 1024;
+  static constexpr int kMaxLevels = 8;
+  static constexpr int kMaxRows = 128, kMaxEntries = 2048;
   int levels = 0;
   int pre = 1, post = 2, coarsest = 8;
   float omega = 0.7f;
   CoupledLevel op[kMaxLevels];
   CoupledTransfer down[kMaxLevels];  // down[k]: tail level k -> k + 1
-  float4* x[kMaxLevels];
-  float4* tmp[kMaxLevels];
-  float4* b[kMaxLevels];
+  const float4* b = nullptr;
+  float4* x = nullptr;
 };
 
 namespace launch {
@@ -100,11 +103,18 @@ void cpl_copy_diagonal(int n, const int* rows, const int* diag, const float* val
 void cpl_assemble(const CoupledMeshDevice& m, const CoupledSolveInputs& in, float* cell,
                   float* coefficient, float4* b, float* scratch, CoupledFine op, float wc,
                   float coefficient_scale, float continuity_scale, int reference, cudaStream_t s);
-void cpl_galerkin_fine(const CoupledLevel& l, const CoupledTransfer& t, const CoupledMeshDevice& m,
-                       const CoupledSolveInputs& in, const float* coefficient, const float* cell,
+// Galerkin operators: the fine level's contributions come from its packed
+// records (cpl_assemble first), a coarse level's from its entries.
+void cpl_galerkin_fine(const CoupledLevel& l, const CoupledFine& op, const float* cell, int cells,
                        float wc, cudaStream_t s);
-void cpl_galerkin_coarse(const CoupledLevel& l, const CoupledTransfer& t, const CoupledLevel& f,
-                         cudaStream_t s);
+void cpl_galerkin_coarse(const CoupledLevel& l, const CoupledLevel& f, cudaStream_t s);
+// The term lists, a thread per coarse row: first each entry's count of terms,
+// then (after an exclusive scan into term_at) the terms. Fine level: its
+// adjacency through the mesh; coarse: the level above's CSR.
+void cpl_terms_fine(const CoupledLevel& l, const CoupledTransfer& t, const CoupledMeshDevice& m,
+                    int* count, int* terms, int* term_faces, cudaStream_t s);
+void cpl_terms_coarse(const CoupledLevel& l, const CoupledTransfer& t, const CoupledLevel& f,
+                      int* count, int* terms, cudaStream_t s);
 // |G| row sums into scratch (3n), then cs and the block inverse.
 void cpl_coarse_prepare(const CoupledLevel& l, float* scratch, cudaStream_t s);
 
@@ -116,10 +126,16 @@ void cpl_fine_smooth(int n, const CoupledFine& op, int width, const float4* x, c
                      float4* next, float omega, bool first, cudaStream_t s);
 void cpl_coarse_residual(const CoupledLevel& l, const float4* x, const float4* b, float4* r,
                          cudaStream_t s);
+// One sweep; with aggregate != null from x + coarse[aggregate] (the prolongation
+// folded in).
 void cpl_coarse_smooth(const CoupledLevel& l, const float4* x, const float4* b, float4* next,
-                       float omega, bool first, cudaStream_t s);
+                       float omega, bool first, const int* aggregate, const float4* coarse,
+                       cudaStream_t s);
+// coarse = the sum of each aggregate's members; with next != null also level
+// l's (the coarse one's) first sweep from zero.
 void cpl_restrict(int nc, const int* offsets, const int* members, const float4* fine,
-                  float4* coarse, cudaStream_t s);
+                  float4* coarse, const CoupledLevel* l, float omega, float4* next,
+                  cudaStream_t s);
 void cpl_prolong(int nf, const int* aggregate, const float4* coarse, float4* fine,
                  cudaStream_t s);
 

@@ -80,35 +80,22 @@ CoupledSolver::CoupledSolver(const CoupledMeshHost& m, int reference,
   own(link_, slots);
   own(face_, nf);
 
-  // A level whose longest row has at least this many entries gets a warp per
-  // row in its separately launched row kernels (KUTTA_B200_COUPLED_WIDE_ROWS,
-  // 0 for never; the same bits either way; the one-block tail keeps a thread
-  // per row): a thread walking a hub row of ~150 entries stalls a whole sweep
-  // behind it.
-  const char* wide_env = std::getenv("KUTTA_B200_COUPLED_WIDE_ROWS");
-  const int wide_rows = wide_env ? std::atoi(wide_env) : 32;
   for (std::size_t k = 0; k < setup.levels.size(); ++k) {
     auto& src = setup.levels[k];
-    int longest = 0;
-    for (int i = 0; i < src.n; ++i) longest = std::max(longest, src.rows[i + 1] - src.rows[i]);
     Level l;
     own(l.rows, src.rows, s);
     own(l.cols, src.cols, s);
     own(l.diag, src.diag, s);
     const std::size_t cn = src.n, nnz = src.nnz;
-    own(l.a, nnz);
-    own(l.c, nnz);
-    own(l.g, 3 * nnz);
-    own(l.h, 3 * nnz);
+    own(l.entry, 2 * nnz);
     own(l.d, 11 * cn);
     own(l.b, cn);
     own(l.store[0], cn);
     own(l.store[1], cn);
     l.x = l.store[0].get();
     l.tmp = l.store[1].get();
-    l.op = CoupledLevel{src.n, src.nnz, l.rows.get(), l.cols.get(), l.diag.get(),
-                        l.a.get(),  l.c.get(),   l.g.get(),    l.h.get(),    l.d.get()};
-    l.op.wide = wide_rows > 0 && longest >= wide_rows ? 1 : 0;
+    l.op = CoupledLevel{src.n,        src.nnz,       l.rows.get(), l.cols.get(),
+                        l.diag.get(), l.entry.get(), l.d.get()};
     levels_.push_back(std::move(l));
     auto& tsrc = setup.transfers[k];
     Transfer t;
@@ -118,15 +105,18 @@ CoupledSolver::CoupledSolver(const CoupledMeshHost& m, int reference,
     t.view = CoupledTransfer{t.aggregate.get(), t.offsets.get(), t.members.get()};
     transfers_.push_back(std::move(t));
   }
+  build_terms(s);
   // Levels from `tail_` down are small enough for the one-block V-cycle
   // (KUTTA_B200_COUPLED_TAIL=0: separate launches, the same results;
-  // KUTTA_B200_COUPLED_TAIL_ROWS: the largest level it takes).
+  // KUTTA_B200_COUPLED_TAIL_ROWS: only levels of at most so many rows).
   const char* tail = std::getenv("KUTTA_B200_COUPLED_TAIL");
   const char* tail_rows = std::getenv("KUTTA_B200_COUPLED_TAIL_ROWS");
-  const int max_rows = tail_rows ? std::atoi(tail_rows) : CoupledTail::kMaxRows;
+  const int max_rows = std::min(tail_rows ? std::atoi(tail_rows) : CoupledTail::kMaxRows,
+                                CoupledTail::kMaxRows);
   tail_ = levels_.size();
   if (!(tail && std::string(tail) == "0"))
     while (tail_ > 0 && levels_[tail_ - 1].op.n <= max_rows &&
+           levels_[tail_ - 1].op.nnz <= CoupledTail::kMaxEntries &&
            levels_.size() - (tail_ - 1) <= static_cast<std::size_t>(CoupledTail::kMaxLevels))
       --tail_;
   for (auto* v : {&b_, &r_, &shadow_, &p_, &q_, &sv_, &t_}) own(*v, n);
@@ -259,12 +249,25 @@ void CoupledSolver::fine_smooth(float4*& out, const float4* rhs, int sweeps, boo
   }
 }
 
-void CoupledSolver::coarse_smooth(Level& l, int sweeps, bool first) {
-  for (int k = 0; k < sweeps; ++k) {
+void CoupledSolver::coarse_smooth(std::size_t k, int sweeps, bool first, bool swept,
+                                  const float4* coarse) {
+  auto& l = levels_[k];
+  for (int s = swept ? 1 : 0; s < sweeps; ++s) {
+    const bool fold = s == 0 && coarse != nullptr;
     launch::cpl_coarse_smooth(l.op, l.x, l.b.get(), l.tmp, options_.smoother_damping,
-                              first && k == 0, stream_);
+                              first && s == 0, fold ? transfers_[k + 1].view.aggregate : nullptr,
+                              coarse, stream_);
     std::swap(l.x, l.tmp);
   }
+}
+
+void CoupledSolver::descend(std::size_t k, const float4* fine) {
+  auto& c = levels_[k];
+  const auto& t = transfers_[k].view;
+  const bool first = k != tail_;
+  launch::cpl_restrict(c.op.n, t.offsets, t.members, fine, c.b.get(), &c.op,
+                       options_.smoother_damping, first ? c.tmp : nullptr, stream_);
+  if (first) std::swap(c.x, c.tmp);
 }
 
 // Coarse level k receives its right-hand side in levels_[k].b
@@ -280,33 +283,27 @@ void CoupledSolver::cycle(std::size_t k) {
     for (int j = 0; j < t.levels; ++j) {
       auto& l = levels_[k + j];
       t.op[j] = l.op;
-      t.x[j] = l.x;
-      t.tmp[j] = l.tmp;
-      t.b[j] = l.b.get();
       if (j + 1 < t.levels) t.down[j] = transfers_[k + j + 1].view;
     }
+    t.b = levels_[k].b.get();
+    t.x = levels_[k].x;
     launch::cpl_tail(t, stream_);
-    // The roles the separate launches would leave: each level swaps once per
-    // sweep.
-    for (int j = 0; j < t.levels; ++j) {
-      const int sweeps = j + 1 < t.levels ? t.pre + t.post : t.coarsest;
-      if (sweeps % 2) std::swap(levels_[k + j].x, levels_[k + j].tmp);
-    }
     return;
   }
   auto& l = levels_[k];
   if (k + 1 == levels_.size()) {
-    coarse_smooth(l, options_.coarsest_sweeps, true);
+    coarse_smooth(k, options_.coarsest_sweeps, true, true, nullptr);
     return;
   }
   auto& c = levels_[k + 1];
-  coarse_smooth(l, options_.pre_sweeps, true);
+  coarse_smooth(k, options_.pre_sweeps, true, true, nullptr);
   launch::cpl_coarse_residual(l.op, l.x, l.b.get(), l.tmp, stream_);
-  const auto& t = transfers_[k + 1].view;
-  launch::cpl_restrict(c.op.n, t.offsets, t.members, l.tmp, c.b.get(), stream_);
+  descend(k + 1, l.tmp);
   cycle(k + 1);
-  launch::cpl_prolong(l.op.n, t.aggregate, c.x, l.x, stream_);
-  coarse_smooth(l, options_.post_sweeps, false);
+  // The first post-sweep adds the correction as it reads x.
+  if (options_.post_sweeps == 0)
+    launch::cpl_prolong(l.op.n, transfers_[k + 1].view.aggregate, c.x, l.x, stream_);
+  coarse_smooth(k, options_.post_sweeps, false, false, c.x);
 }
 
 // out = V-cycle(rhs), a fixed linear preconditioner (coupled_solver.cpp:349-360).
@@ -316,21 +313,56 @@ void CoupledSolver::precondition(const float4* rhs, float4*& out) {
     auto& c = levels_[0];
     const auto& t = transfers_[0].view;
     launch::cpl_fine_residual(n_, fine(), width_, out, rhs, tmp_, stream_);
-    launch::cpl_restrict(c.op.n, t.offsets, t.members, tmp_, c.b.get(), stream_);
+    descend(0, tmp_);
     cycle(0);
     launch::cpl_prolong(n_, t.aggregate, c.x, out, stream_);
   }
   fine_smooth(out, rhs, options_.post_sweeps, false);
 }
 
+// The contributions of every Galerkin entry, listed once for the pattern.
+void CoupledSolver::build_terms(cudaStream_t s) {
+  for (std::size_t k = 0; k < levels_.size(); ++k) {
+    auto& l = levels_[k];
+    const auto& t = transfers_[k].view;
+    const std::size_t entries = l.op.nnz;
+    // The fine level numbers its terms by ELL slot, a coarse one by 2 x entry.
+    KB2_REQUIRE(k == 0 ? static_cast<long long>(width_) * n_ <= 0x7fffffffLL
+                       : levels_[k - 1].op.nnz < (1 << 30),
+                "coupled: operator exceeds the 32-bit index range");
+    DArray<int> count(entries + 1), scratch(launch::scan_scratch(l.op.nnz));
+    const auto list = [&](int* terms) {
+      cuda_check(cudaMemsetAsync(count.get(), 0, (entries + 1) * sizeof(int), s), "memset");
+      if (k == 0)
+        launch::cpl_terms_fine(l.op, t, mesh_, count.get(), terms, l.term_faces.get(), s);
+      else
+        launch::cpl_terms_coarse(l.op, t, levels_[k - 1].op, count.get(), terms, s);
+    };
+    list(nullptr);
+    own(l.term_at, entries + 1);
+    launch::exclusive_scan(l.op.nnz, count.get(), l.term_at.get(), scratch.get(), s);
+    l.op.term_at = l.term_at.get();
+    int total = 0;
+    cuda_check(cudaMemcpyAsync(&total, l.term_at.get() + entries, sizeof(int),
+                               cudaMemcpyDeviceToHost, s),
+               "readback");
+    wait(s);
+    own(l.terms, static_cast<std::size_t>(total));
+    if (k == 0) own(l.term_faces, static_cast<std::size_t>(total));
+    list(l.terms.get());
+    l.op.terms = l.terms.get();
+    l.op.term_faces = l.term_faces.get();
+    wait(s);  // count and scratch are released here
+  }
+}
+
 // Galerkin operators from the fine level down, then each level's smoother
 // bound and block inverse (coupled_solver.cpp:361-384).
-void CoupledSolver::galerkin(const CoupledSolveInputs& in) {
+void CoupledSolver::galerkin() {
   if (levels_.empty()) return;
-  launch::cpl_galerkin_fine(levels_[0].op, transfers_[0].view, mesh_, in, coefficient_.get(),
-                            cell_.get(), wc_, stream_);
+  launch::cpl_galerkin_fine(levels_[0].op, fine(), cell_.get(), n_, wc_, stream_);
   for (std::size_t k = 1; k < levels_.size(); ++k)
-    launch::cpl_galerkin_coarse(levels_[k].op, transfers_[k].view, levels_[k - 1].op, stream_);
+    launch::cpl_galerkin_coarse(levels_[k].op, levels_[k - 1].op, stream_);
   for (auto& l : levels_)
     launch::cpl_coarse_prepare(l.op, reinterpret_cast<float*>(l.tmp), stream_);
 }
@@ -459,7 +491,7 @@ Stats CoupledSolver::solve(const CoupledSolveInputs& in, double density, double 
   launch::cpl_assemble(mesh_, in, cell_.get(), coefficient_.get(), b_.get(),
                        scratch_.get(), fine(), wc_, static_cast<float>(wc * wc),
                        static_cast<float>(wc / density), reference_, s);
-  galerkin(in);
+  galerkin();
   cuda_check(cudaGetLastError(), "coupled assembly");
   return bicgstab(control);
 }
@@ -511,9 +543,12 @@ void CoupledSolver::level_apply(int k, int op, const float* x, const float* b, f
     case 1: launch::cpl_coarse_residual(l, x4, b4, y4, s); break;
     case 2:
     case 3:
-      launch::cpl_coarse_smooth(l, x4, b4, y4, options_.smoother_damping, op == 3, s);
+      launch::cpl_coarse_smooth(l, x4, b4, y4, options_.smoother_damping, op == 3, nullptr,
+                                nullptr, s);
       break;
-    case 4: launch::cpl_restrict(l.n, t.offsets, t.members, x4, y4, s); break;
+    case 4:
+      launch::cpl_restrict(l.n, t.offsets, t.members, x4, y4, nullptr, 0.0f, nullptr, s);
+      break;
     case 5: launch::cpl_prolong(level_rows(k - 1), t.aggregate, x4, y4, s); break;
     default: KB2_REQUIRE(false, "coupled: unknown level operator");
   }

@@ -74,8 +74,9 @@ class CoupledSolver {
  private:
   struct Level {
     CoupledLevel op;
-    DArray<int> rows, cols, diag;
-    DArray<float> a, c, g, h, d;
+    DArray<int> rows, cols, diag, term_at, terms, term_faces;
+    DArray<float4> entry;
+    DArray<float> d;
     DArray<float4> b, store[2];
     float4 *x = nullptr, *tmp = nullptr;  // the smoother's ping-pong roles over store
   };
@@ -102,10 +103,16 @@ class CoupledSolver {
   }
   CoupledFine fine() const;
   void fine_smooth(float4*& out, const float4* rhs, int sweeps, bool first);
-  void coarse_smooth(Level& l, int sweeps, bool first);
+  // swept: the first sweep is already in l.x; coarse: the first one also adds
+  // this correction (by level k's aggregates).
+  void coarse_smooth(std::size_t k, int sweeps, bool first, bool swept, const float4* coarse);
+  // Restricts `fine` into coarse level k, with its first sweep from zero
+  // unless the tail makes it.
+  void descend(std::size_t k, const float4* fine);
   void cycle(std::size_t k);
+  void build_terms(cudaStream_t s);
   void precondition(const float4* rhs, float4*& out);
-  void galerkin(const CoupledSolveInputs& in);
+  void galerkin();
   double norm(const float4* v);
   std::vector<float4*> roles() const;
   void set_roles(const std::vector<float4*>& r);

@@ -1,0 +1,108 @@
+"""The Coupled solve's coarse-level kernels (kutta_b200/csrc/cuda/coupled_coarse.cu)
+on boxes whose levels reach both launch shapes and rows of a hundred entries:
+row kernels and Galerkin sums bit for bit against numpy restatements of the
+reference's order, on the operators that the device assembled."""
+import numpy as np
+import pytest
+
+from kutta_b200 import coupled_harness as H
+from kutta_b200 import linalg as L
+from oracle import coupled as O
+
+pytestmark = pytest.mark.gpu
+f32 = np.float32
+
+BOXES = {
+    # More than 16,384 rows on level 1, a ragged last block on every level.
+    "hex": lambda: H.box_hex(53, 51, 49),
+    # Hub rows on the small levels, and levels at the one-block tail's edges.
+    "tet": lambda: H.box_tet(12, 11, 9),
+}
+
+
+def bits(a):
+    return np.ascontiguousarray(a, f32).view(np.uint32)
+
+
+def _solved(name):
+    import torch
+    mesh = BOXES[name]()
+    fields = H.flow_fields(mesh, 3)
+    dev = {k: torch.from_numpy(v).cuda() if isinstance(v, np.ndarray) else v
+           for k, v in fields.items()}
+    s = L.CoupledSolver(mesh, -1, L.CoupledOptions())
+    rows, diag = (torch.from_numpy(mesh[k]).cuda() for k in ("pattern_row_ptr", "pattern_diag"))
+    for k, c in enumerate("uvw"):
+        s.capture_diagonal(k, rows, diag, dev["momentum_" + c], dev["physical_" + c])
+    s.solve(dev, L.SolveControl(0.1, 1e-12, 20))
+    return s
+
+
+@pytest.mark.parametrize("name", BOXES)
+def test_level_rows_match_oracle(cuda, name):
+    import torch
+    s = _solved(name)
+    omega = L.CoupledOptions().smoother_damping
+    rng = np.random.default_rng(5)
+    for k in range(1, s.levels()):
+        lv = s.level(k)
+        n = len(lv["diag"])
+        x, b = (rng.standard_normal(4 * n).astype(f32) for _ in range(2))
+        dx, db = (torch.from_numpy(np.ascontiguousarray(v.reshape(4, n).T).reshape(-1)).cuda()
+                  for v in (x, b))
+        want = {"residual": (b - O.coarse_row(lv, x)).astype(f32),
+                "smooth": O.coarse_smooth(lv, x, b, omega, False),
+                "smooth_zero": O.coarse_smooth(lv, x, b, omega, True)}
+        for op, w in want.items():
+            y = torch.full((4 * n,), float("nan"), device="cuda")
+            s.level_apply(k, op, dx, db, y)
+            got = y.cpu().numpy().reshape(n, 4).T.reshape(-1)
+            assert np.array_equal(bits(got), bits(w)), (k, op)
+
+
+def _add(sum_, error, value):
+    """One term of the Neumaier sum that the reference's diagonals take."""
+    total = f32(sum_ + value)
+    if abs(sum_) >= abs(value):
+        error = f32(error + f32(f32(sum_ - total) + value))
+    else:
+        error = f32(error + f32(f32(value - total) + sum_))
+    return total, error
+
+
+def test_galerkin_sums_match_their_order(cuda):
+    """Level 2 from level 1 (fv_coupled.kern.h:490-524): off-diagonal entries
+    are plain sums in member and entry order, the diagonal's ten compensated."""
+    s = _solved("tet")
+    f, c = s.level(1), s.level(2)
+    agg = c["aggregate"]
+    n, nc, fz, cz = len(f["diag"]), len(c["diag"]), len(f["cols"]), len(c["cols"])
+    entry = np.concatenate([[f["a"], f["c"]], f["g"].reshape(3, fz), f["h"].reshape(3, fz)])
+    want = np.zeros((8, cz), f32)
+    momentum = np.zeros((3, nc), f32)
+    where = [{int(c["cols"][e]): e for e in range(c["rows"][i], c["rows"][i + 1])}
+             for i in range(nc)]
+    for i in range(nc):
+        sums = np.zeros(10, f32)
+        errors = np.zeros(10, f32)
+        for row in np.nonzero(agg == i)[0]:
+            for k in range(3):
+                sums[k], errors[k] = _add(sums[k], errors[k], f["d"][k * n + row])
+            for j in range(f["rows"][row], f["rows"][row + 1]):
+                target = int(agg[f["cols"][j]])
+                if j == f["diag"][row] or target == i:
+                    if j != f["diag"][row]:
+                        for k in range(3):
+                            sums[k], errors[k] = _add(sums[k], errors[k], entry[0, j])
+                    for k in range(7):
+                        sums[3 + k], errors[3 + k] = _add(sums[3 + k], errors[3 + k],
+                                                          entry[1 + k, j])
+                else:
+                    want[:, where[i][target]] += entry[:, j]
+        total = (sums + errors).astype(f32)
+        momentum[:, i] = total[:3]
+        want[1:, c["diag"][i]] = total[3:]
+        want[0, c["diag"][i]] = 0
+    got = np.concatenate([[c["a"], c["c"]], c["g"].reshape(3, cz), c["h"].reshape(3, cz)])
+    assert np.array_equal(bits(got), bits(want))
+    assert np.array_equal(bits(c["d"][:3 * nc]), bits(momentum.reshape(-1)))
