@@ -281,10 +281,11 @@ void gnn_store_gate_grad(const double* dots, float* grad, cudaStream_t s);
 // H0, reduced on the device in between).
 void gnn_input(int n, const float* r, const float* node_scale, float* H0, cudaStream_t s);
 void gnn_normalize(int n, float* H0, const double* sum2, cudaStream_t s);
-// M = W H for C <= 32 channels (row-major n x C).
+// out = W H, with add != null add + W H, for C = 1 (no add) or 32 channels
+// (row-major n x C).
 void gnn_aggregate(int n, int C, const int* rows, const int* cols, const float* edge,
-                   const float* H, float* M, cudaStream_t s);
-// out = relu(Ws H + Wn M + b), Cin -> 32 channels.
+                   const float* H, const float* add, float* out, cudaStream_t s);
+// out = relu(Ws H + Wn M + b), Cin = 1 or 32 -> 32 channels.
 void gnn_dense(int n, int Cin, const float* H, const float* M, const float* Ws, const float* Wn,
                const float* bias, float* out, cudaStream_t s);
 // z = beta z + rho node_scale * (H wo).
@@ -296,11 +297,15 @@ void gnn_energy(int n, const float* t, const float* q, const double* dots, float
                 cudaStream_t s);
 void gnn_output_back(int n, const float* H, const float* wo, const float* node_scale,
                      const double* sum2, const float* dz, float* dH, float* dwo, cudaStream_t s);
-void gnn_dense_back(int n, int Cin, const float* H, const float* M, const float* out,
-                    const float* dOut, const float* Ws, const float* Wn, float* dH, float* dM,
-                    float* dWs, float* dWn, float* db, cudaStream_t s);
-void gnn_add(std::size_t count, const float* a, const float* b, float* out, cudaStream_t s);
-// The same backward as gnn_dense_back for a 32-wide input (Cin = 32) on the
+// 32 inputs.
+void gnn_dense_back(int n, const float* H, const float* M, const float* out, const float* dOut,
+                    const float* Ws, const float* Wn, float* dH, float* dM, float* dWs, float* dWn,
+                    float* db, cudaStream_t s);
+// One input (the first layer): no dH; dM may be null.
+void gnn_dense_back1(int n, const float* H, const float* M, const float* out, const float* dOut,
+                     const float* Wn, float* dM, float* dWs, float* dWn, float* db,
+                     cudaStream_t s);
+// The same backward as gnn_dense_back on the
 // tensor cores (learned_tc.cu): [dH | dM] = G [Ws | Wn] per 128-row tile, and
 // [dWs^T; dWn^T; db] = [H | M | 1]^T G accumulated in tensor memory, BF16
 // operands and FP32 accumulation; dWs, dWn, db are added to (not

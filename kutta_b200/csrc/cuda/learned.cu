@@ -126,49 +126,155 @@ __global__ void k_gnn_store_gate_grad(const double* __restrict__ dots, float* __
   if (blockIdx.x == 0 && threadIdx.x < 2) grad[threadIdx.x] = static_cast<float>(dots[threadIdx.x]);
 }
 
-// M = W H (C channels).
-__global__ void k_gnn_aggregate(int n, int C, const int* __restrict__ rows,
-                                const int* __restrict__ cols, const float* __restrict__ edge,
-                                const float* __restrict__ H, float* __restrict__ M) {
-  const int lane = threadIdx.x & 31;
-  WARP_ROWS(i, n) {
+// M = W H, or with `add` out = add + W H, for C = 32: eight lanes per row, four
+// channels each, so a gathered row is one 128-byte read and a warp has four
+// rows' reads in flight; the row's entries are loaded eight at a time, a lane
+// each, and passed by shuffle. L2-bound on the gathered rows (262,144 rows of 7:
+// 235 MB), 38 us there; a lane per channel, one
+// entry after another, took 109 us and left the addition to a kernel of 23 us.
+__global__ void __launch_bounds__(kBlock) k_gnn_aggregate(int n, const int* __restrict__ rows,
+                                                          const int* __restrict__ cols,
+                                                          const float* __restrict__ edge,
+                                                          const float4* __restrict__ H,
+                                                          const float4* __restrict__ add,
+                                                          float4* __restrict__ out) {
+  const int part = threadIdx.x & 7, lane0 = threadIdx.x & 24;
+  const unsigned mask = 0xffu << lane0;
+  for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 3; i < n;
+       i += (gridDim.x * blockDim.x) >> 3) {
+    float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    const int end = rows[i + 1];
+    for (int base = rows[i]; base < end; base += 8) {
+      const int j = base + part;
+      const int c = j < end ? cols[j] : 0;
+      const float w = j < end ? edge[j] : 0.0f;
+      float4 v[8];
+      float wk[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        wk[k] = __shfl_sync(mask, w, lane0 + k);
+        const int ck = __shfl_sync(mask, c, lane0 + k);
+        if (wk[k] != 0.0f) v[k] = H[8 * static_cast<std::size_t>(ck) + part];
+      }
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        if (wk[k] != 0.0f) {
+          acc.x = fmaf(wk[k], v[k].x, acc.x);
+          acc.y = fmaf(wk[k], v[k].y, acc.y);
+          acc.z = fmaf(wk[k], v[k].z, acc.z);
+          acc.w = fmaf(wk[k], v[k].w, acc.w);
+        }
+    }
+    const std::size_t at = 8 * static_cast<std::size_t>(i) + part;
+    if (add != nullptr) {
+      const float4 a = add[at];
+      acc = make_float4(a.x + acc.x, a.y + acc.y, a.z + acc.z, a.w + acc.w);
+    }
+    out[at] = acc;
+  }
+}
+
+// The same for one channel: a thread per row.
+__global__ void k_gnn_aggregate1(int n, const int* __restrict__ rows, const int* __restrict__ cols,
+                                 const float* __restrict__ edge, const float* __restrict__ H,
+                                 float* __restrict__ M) {
+  ROWS(i, n) {
     float acc = 0.0f;
     const int end = rows[i + 1];
     for (int j = rows[i]; j < end; ++j) {
       const float w = edge[j];
-      if (lane < C && w != 0.0f) acc = fmaf(w, H[static_cast<std::size_t>(cols[j]) * C + lane], acc);
+      if (w != 0.0f) acc = fmaf(w, H[cols[j]], acc);
     }
-    if (lane < C) M[static_cast<std::size_t>(i) * C + lane] = acc;
+    M[i] = acc;
   }
 }
 
-// H'_i = relu(Ws H_i + Wn M_i + b): weights [Cout=32][Cin] held transposed in
-// shared memory (lane = output channel reads consecutive words, no bank
-// conflicts); the row's inputs are broadcast by shuffles.
-__global__ void k_gnn_dense(int n, int Cin, const float* __restrict__ H,
-                            const float* __restrict__ M, const float* __restrict__ Ws,
-                            const float* __restrict__ Wn, const float* __restrict__ bias,
-                            float* __restrict__ out) {
-  __shared__ float ws[kHidden * kHidden], wn[kHidden * kHidden], bs[kHidden];
-  for (int k = threadIdx.x; k < kHidden * Cin; k += blockDim.x) {
-    const int c = k / Cin, j = k % Cin;  // Ws[c][j] -> ws[j][c]
+// H'_i = relu(Ws H_i + Wn M_i + b) for 32 inputs: a warp takes eight rows, lane
+// = output channel. The weights lie transposed in shared memory (consecutive
+// words, no bank conflicts) and the rows' inputs beside them, read four at a
+// time as broadcasts: 24 shared loads for 64 FMAs, where a row at a time with
+// its inputs passed by shuffle took two shuffles and two loads for two (58 us
+// against 150 at 262,144 rows).
+constexpr int kDenseRows = 8;  // of a warp
+__global__ void __launch_bounds__(kBlock) k_gnn_dense(int n, const float4* __restrict__ H,
+                                                      const float4* __restrict__ M,
+                                                      const float* __restrict__ Ws,
+                                                      const float* __restrict__ Wn,
+                                                      const float* __restrict__ bias,
+                                                      float* __restrict__ out) {
+  constexpr int kWarps = kBlock / 32;
+  __shared__ float ws[kHidden * kHidden], wn[kHidden * kHidden];
+  __shared__ float4 in[kWarps][2][kDenseRows * kHidden / 4];
+  for (int k = threadIdx.x; k < kHidden * kHidden; k += blockDim.x) {
+    const int c = k / kHidden, j = k % kHidden;  // Ws[c][j] -> ws[j][c]
     ws[j * kHidden + c] = Ws[k];
     wn[j * kHidden + c] = Wn[k];
   }
-  if (threadIdx.x < kHidden) bs[threadIdx.x] = bias[threadIdx.x];
   __syncthreads();
-  const int lane = threadIdx.x & 31;
-  WARP_ROWS(i, n) {
-    const float h = lane < Cin ? H[static_cast<std::size_t>(i) * Cin + lane] : 0.0f;
-    const float m = lane < Cin ? M[static_cast<std::size_t>(i) * Cin + lane] : 0.0f;
-    float acc = bs[lane];
-    for (int k = 0; k < Cin; ++k) {
-      const float hk = __shfl_sync(0xffffffffu, h, k);
-      const float mk = __shfl_sync(0xffffffffu, m, k);
-      acc = fmaf(ws[k * kHidden + lane], hk, acc);
-      acc = fmaf(wn[k * kHidden + lane], mk, acc);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const float b = bias[lane];
+  float4* h = in[warp][0];
+  float4* m = in[warp][1];
+  const int groups = (n + kDenseRows - 1) / kDenseRows;
+  for (int group = blockIdx.x * kWarps + warp; group < groups; group += gridDim.x * kWarps) {
+    const int row0 = group * kDenseRows, count = min(kDenseRows, n - row0);
+    __syncwarp();
+    for (int k = lane; k < kDenseRows * kHidden / 4; k += 32)
+      if (k < count * kHidden / 4) {
+        h[k] = H[static_cast<std::size_t>(row0) * (kHidden / 4) + k];
+        m[k] = M[static_cast<std::size_t>(row0) * (kHidden / 4) + k];
+      }
+    __syncwarp();
+    float acc[kDenseRows];
+#pragma unroll
+    for (int r = 0; r < kDenseRows; ++r) acc[r] = b;
+#pragma unroll 2
+    for (int q = 0; q < kHidden / 4; ++q) {
+      float s4[4], n4[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        s4[u] = ws[(4 * q + u) * kHidden + lane];
+        n4[u] = wn[(4 * q + u) * kHidden + lane];
+      }
+#pragma unroll
+      for (int r = 0; r < kDenseRows; ++r) {
+        const float4 hr = h[r * (kHidden / 4) + q], mr = m[r * (kHidden / 4) + q];
+        acc[r] = fmaf(s4[0], hr.x, acc[r]);
+        acc[r] = fmaf(n4[0], mr.x, acc[r]);
+        acc[r] = fmaf(s4[1], hr.y, acc[r]);
+        acc[r] = fmaf(n4[1], mr.y, acc[r]);
+        acc[r] = fmaf(s4[2], hr.z, acc[r]);
+        acc[r] = fmaf(n4[2], mr.z, acc[r]);
+        acc[r] = fmaf(s4[3], hr.w, acc[r]);
+        acc[r] = fmaf(n4[3], mr.w, acc[r]);
+      }
     }
-    out[static_cast<std::size_t>(i) * kHidden + lane] = fmaxf(acc, 0.0f);
+#pragma unroll
+    for (int r = 0; r < kDenseRows; ++r)
+      if (r < count)
+        out[static_cast<std::size_t>(row0 + r) * kHidden + lane] = fmaxf(acc[r], 0.0f);
+  }
+}
+
+// The same for one input (the first layer): a thread per row and four channels.
+__global__ void k_gnn_dense1(int n, const float* __restrict__ H, const float* __restrict__ M,
+                             const float* __restrict__ Ws, const float* __restrict__ Wn,
+                             const float* __restrict__ bias, float4* __restrict__ out) {
+  const int part = threadIdx.x & 7;
+  float s[4], w[4], b[4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    s[u] = Ws[4 * part + u];
+    w[u] = Wn[4 * part + u];
+    b[u] = bias[4 * part + u];
+  }
+  for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 3; i < n;
+       i += (gridDim.x * blockDim.x) >> 3) {
+    const float h = H[i], m = M[i];
+    float v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) v[u] = fmaxf(fmaf(w[u], m, fmaf(s[u], h, b[u])), 0.0f);
+    out[8 * static_cast<std::size_t>(i) + part] = make_float4(v[0], v[1], v[2], v[3]);
   }
 }
 
@@ -312,12 +418,56 @@ __global__ void k_gnn_dense_back(int n, int Cin, const float* __restrict__ H,
   if (threadIdx.x < kHidden) atomicAdd(db + threadIdx.x, gb[threadIdx.x]);
 }
 
-// out = a + b (elementwise).
-__global__ void k_gnn_add(std::size_t count, const float* __restrict__ a,
-                          const float* __restrict__ b, float* __restrict__ out) {
-  for (std::size_t k = blockIdx.x * blockDim.x + threadIdx.x; k < count;
-       k += static_cast<std::size_t>(gridDim.x) * blockDim.x)
-    out[k] = a[k] + b[k];
+// The backward of the one-input layer, whose input is the residual itself: no
+// dH, and dM only for the gate (dM != null). Lane = channel, a warp per row;
+// bound by reading the two wide arrays (the general kernel's 64 accumulators
+// and its shuffles took 403 us at 262,144 rows, this 19). Each block adds its
+// warps' sums before the atomics.
+__global__ void __launch_bounds__(kBlock) k_gnn_dense_back1(
+    int n, const float* __restrict__ H, const float* __restrict__ M, const float* __restrict__ out,
+    const float* __restrict__ dOut, const float* __restrict__ Wn, float* __restrict__ dM,
+    float* __restrict__ dWs, float* __restrict__ dWn, float* __restrict__ db) {
+  __shared__ float sums[3][kBlock / 32][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const float wn = Wn[lane];
+  float as = 0.0f, an = 0.0f, ab = 0.0f;
+  const int stride = static_cast<int>((gridDim.x * blockDim.x) >> 5);
+  constexpr int kAhead = 4;
+  for (int i0 = static_cast<int>((blockIdx.x * blockDim.x + threadIdx.x) >> 5); i0 < n;
+       i0 += kAhead * stride) {
+    float o[kAhead], g[kAhead], h[kAhead], m[kAhead];
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) {
+      const int i = i0 + k * stride;
+      const bool in = i < n;
+      const std::size_t at = static_cast<std::size_t>(in ? i : 0) * kHidden + lane;
+      o[k] = in ? out[at] : 0.0f;
+      g[k] = in ? dOut[at] : 0.0f;
+      h[k] = in ? H[i] : 0.0f;
+      m[k] = in ? M[i] : 0.0f;
+    }
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) {
+      const float v = o[k] > 0.0f ? g[k] : 0.0f;
+      ab += v;
+      as = fmaf(v, h[k], as);
+      an = fmaf(v, m[k], an);
+      if (dM != nullptr) {
+        float d = wn * v;
+        for (int u = 16; u > 0; u >>= 1) d += __shfl_down_sync(0xffffffffu, d, u);
+        if (lane == 0 && i0 + k * stride < n) dM[i0 + k * stride] = d;
+      }
+    }
+  }
+  sums[0][warp][lane] = as;
+  sums[1][warp][lane] = an;
+  sums[2][warp][lane] = ab;
+  __syncthreads();
+  if (warp >= 3) return;
+  float total = 0.0f;
+#pragma unroll
+  for (int k = 0; k < kBlock / 32; ++k) total += sums[warp][k][lane];
+  atomicAdd((warp == 0 ? dWs : warp == 1 ? dWn : db) + lane, total);
 }
 
 // z += alpha c with alpha = max(0, dots[0] / dots[1]) (dots = c.t, c.A c in
@@ -409,16 +559,27 @@ void gnn_normalize(int n, float* H0, const double* sum2, cudaStream_t s) {
   k_gnn_normalize<<<grid_for(n), kBlock, 0, s>>>(n, H0, sum2);
 }
 void gnn_aggregate(int n, int C, const int* rows, const int* cols, const float* edge,
-                   const float* H, float* M, cudaStream_t s) {
+                   const float* H, const float* add, float* out, cudaStream_t s) {
   if (n <= 0) return;
   ++counter;
-  k_gnn_aggregate<<<warp_grid(n), kBlock, 0, s>>>(n, C, rows, cols, edge, H, M);
+  if (C == 1)
+    k_gnn_aggregate1<<<grid_for(n), kBlock, 0, s>>>(n, rows, cols, edge, H, out);
+  else
+    k_gnn_aggregate<<<grid_for(8LL * n), kBlock, 0, s>>>(
+        n, rows, cols, edge, reinterpret_cast<const float4*>(H),
+        reinterpret_cast<const float4*>(add), reinterpret_cast<float4*>(out));
 }
 void gnn_dense(int n, int Cin, const float* H, const float* M, const float* Ws, const float* Wn,
                const float* bias, float* out, cudaStream_t s) {
   if (n <= 0) return;
   ++counter;
-  k_gnn_dense<<<warp_grid(n), kBlock, 0, s>>>(n, Cin, H, M, Ws, Wn, bias, out);
+  if (Cin == 1)
+    k_gnn_dense1<<<grid_for(8LL * n), kBlock, 0, s>>>(n, H, M, Ws, Wn, bias,
+                                                      reinterpret_cast<float4*>(out));
+  else
+    k_gnn_dense<<<grid_for(32LL * ((n + kDenseRows - 1) / kDenseRows)), kBlock, 0, s>>>(
+        n, reinterpret_cast<const float4*>(H), reinterpret_cast<const float4*>(M), Ws, Wn, bias,
+        out);
 }
 void gnn_output(int n, const float* H, const float* wo, const float* node_scale,
                 const double* sum2, float* z, float beta, cudaStream_t s) {
@@ -438,19 +599,20 @@ void gnn_output_back(int n, const float* H, const float* wo, const float* node_s
   ++counter;
   k_gnn_output_back<<<warp_grid(n), kBlock, 0, s>>>(n, H, wo, node_scale, sum2, dz, dH, dwo);
 }
-void gnn_dense_back(int n, int Cin, const float* H, const float* M, const float* out,
-                    const float* dOut, const float* Ws, const float* Wn, float* dH, float* dM,
-                    float* dWs, float* dWn, float* db, cudaStream_t s) {
+void gnn_dense_back(int n, const float* H, const float* M, const float* out, const float* dOut,
+                    const float* Ws, const float* Wn, float* dH, float* dM, float* dWs, float* dWn,
+                    float* db, cudaStream_t s) {
   if (n <= 0) return;
   ++counter;
-  k_gnn_dense_back<<<warp_grid(n), kBlock, 0, s>>>(n, Cin, H, M, out, dOut, Ws, Wn, dH, dM, dWs,
-                                                   dWn, db);
+  k_gnn_dense_back<<<warp_grid(n), kBlock, 0, s>>>(n, kHidden, H, M, out, dOut, Ws, Wn, dH, dM,
+                                                   dWs, dWn, db);
 }
-void gnn_add(std::size_t count, const float* a, const float* b, float* out, cudaStream_t s) {
-  if (count == 0) return;
+void gnn_dense_back1(int n, const float* H, const float* M, const float* out, const float* dOut,
+                     const float* Wn, float* dM, float* dWs, float* dWn, float* db,
+                     cudaStream_t s) {
+  if (n <= 0) return;
   ++counter;
-  const int blocks = static_cast<int>(std::min<std::size_t>((count + kBlock - 1) / kBlock, kMaxBlocks));
-  k_gnn_add<<<blocks, kBlock, 0, s>>>(count, a, b, out);
+  k_gnn_dense_back1<<<warp_grid(n), kBlock, 0, s>>>(n, H, M, out, dOut, Wn, dM, dWs, dWn, db);
 }
 void gnn_step(int n, float* z, const float* c, const double* dots, cudaStream_t s) {
   if (n <= 0) return;

@@ -616,6 +616,8 @@ __global__ void k_gnn_dense_back_reduce(int blocks, const float* __restrict__ pa
   if (e >= kBackPartialRows * kC) return;
   const int mrow = e / kC, c = e % kC;
   float sum = 0.0f;
+  // In block order, sixteen loads in flight.
+#pragma unroll 16
   for (int b = 0; b < blocks; ++b)
     sum += partials[(static_cast<std::size_t>(b) * kBackPartialRows + mrow) * kC + c];
   if (mrow < kC) dWs[c * kC + mrow] += sum;

@@ -97,7 +97,6 @@ void Gnn::bind(int n, const int* rows, const int* cols, const int* diag, const f
     dh_.reset(wide);
     dhs_.reset(wide);
     dm_.reset(wide);
-    dagg_.reset(wide);
     scale_.reset(rows_n);
     uv_.reset(2 * rows_n);
     h2_.reset(wide);
@@ -165,7 +164,8 @@ void Gnn::forward32(const float* r, float* z, cudaStream_t s) {
                        DeviceReducer{partials_.get(), ticket_.get()}, sums_.get(), 0, s);
   launch::gnn_normalize(n_, h_[0].get(), sums_.get(), s);
   for (int l = 0; l < kLayers; ++l) {
-    launch::gnn_aggregate(n_, cin(l), rows_, cols_, edge_.get(), h_[l].get(), m_agg_[l].get(), s);
+    launch::gnn_aggregate(n_, cin(l), rows_, cols_, edge_.get(), h_[l].get(), nullptr,
+                          m_agg_[l].get(), s);
     launch::gnn_dense(n_, cin(l), h_[l].get(), m_agg_[l].get(), p.ws[l], p.wn[l], p.b[l],
                       h_[l + 1].get(), s);
   }
@@ -202,18 +202,20 @@ void Gnn::backward(const float* t, const float* e, bool tensor_cores, cudaStream
       launch::gnn_dense_back_tc(n_, h_[l].get(), m_agg_[l].get(), h_[l + 1].get(), dh_.get(),
                                 p.ws[l], p.wn[l], dhs_.get(), dm_.get(), g.ws[l], g.wn[l],
                                 g.b[l], back_partials_.get(), fault_.get(), s);
+    } else if (cin(l) == kHidden) {
+      launch::gnn_dense_back(n_, h_[l].get(), m_agg_[l].get(), h_[l + 1].get(), dh_.get(),
+                             p.ws[l], p.wn[l], dhs_.get(), dm_.get(), g.ws[l], g.wn[l], g.b[l], s);
     } else {
-      launch::gnn_dense_back(n_, cin(l), h_[l].get(), m_agg_[l].get(), h_[l + 1].get(),
-                             dh_.get(), p.ws[l], p.wn[l], dhs_.get(), dm_.get(), g.ws[l],
-                             g.wn[l], g.b[l], s);
+      launch::gnn_dense_back1(n_, h_[l].get(), m_agg_[l].get(), h_[l + 1].get(), dh_.get(),
+                              p.wn[l], gated_ ? dm_.get() : nullptr, g.ws[l], g.wn[l], g.b[l], s);
     }
     if (gated_)  // dL/dE from this layer's aggregation M = E h[l]
       launch::gnn_edge_grad(n_, cin(l), rows_, cols_, dm_.get(), h_[l].get(), dedge_.get(),
                             l != kLayers - 1, s);
     if (l > 0) {
       // dL/dh[l] = Ws^T G + W^T (Wn^T G); W is symmetric.
-      launch::gnn_aggregate(n_, cin(l), rows_, cols_, edge_.get(), dm_.get(), dagg_.get(), s);
-      launch::gnn_add(static_cast<std::size_t>(n_) * cin(l), dhs_.get(), dagg_.get(), dh_.get(), s);
+      launch::gnn_aggregate(n_, cin(l), rows_, cols_, edge_.get(), dm_.get(), dhs_.get(),
+                            dh_.get(), s);
     }
   }
   if (gated_) {

@@ -105,7 +105,7 @@ class Gnn {
   DArray<int> fault_;
   // h[0] = input (n), h[l] = layer l output (n x 32); m[l] = aggregation of h[l].
   DArray<float> h_[kLayers + 1], m_agg_[kLayers];
-  DArray<float> dz_, z_, q_, dh_, dhs_, dm_, dagg_;
+  DArray<float> dz_, z_, q_, dh_, dhs_, dm_;
   int step_ = 0;
   long long wait_polls_ = -1;
 };
