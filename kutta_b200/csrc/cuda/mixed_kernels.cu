@@ -448,15 +448,19 @@ __global__ void k_dense_copy(std::size_t count, const double* __restrict__ from,
     to[k] = from[k];
 }
 
-// The same Cholesky factor and inverse for n <= kSharedDense, on chip and
-// with short dependent chains: L and X = L^-1 live in shared memory; each
-// elimination step updates the trailing lower triangle in parallel over its
-// (i, j) pairs (each element sees the same updates in the same k order as a
-// row-by-row update); X is built one elimination step at a time over all
-// right-hand sides of the identity at once; W = X^T X (symmetric) is written
-// to global memory. `L` (global) is not used.
-constexpr int kSharedDense = 112;  // 2 n^2 doubles <= 200 KB
-constexpr int kDenseThreads = 256;
+// The inverse for n <= kSharedDense in one CTA: the root-free factorisation
+// A = L D L^T and X = L^-1 in one elimination, then W = X^T D^-1 X (symmetric).
+// Its length is the n dependent steps, so each step is kept short: warp w's lane
+// l holds elements (w + 32 a, l + 32 c) in registers (A right of the diagonal
+// step, X left of it), and a step needs one division, the current column of A and
+// the current row of X, which their owners put into shared memory as they
+// update them for the next step, and one barrier. `L` (global) is not used. (A
+// Cholesky factor and a separate substitution in shared memory, five barriers,
+// a root and a column of divisions per step, took 231 us at 94 rows; this 118.)
+constexpr int kSharedDense = 112;
+constexpr int kDenseThreads = 1024;
+constexpr int kDenseTile = 4;  // elements of a thread in each direction
+static_assert(32 * kDenseTile >= kSharedDense, "a thread's rows and columns");
 
 // Lower-triangle pair number p -> (i, j), j <= i, rows counted from 0.
 __device__ __forceinline__ void triangle_pair(int p, int& i, int& j) {
@@ -471,73 +475,87 @@ __global__ void __launch_bounds__(kDenseThreads)
                            const float* __restrict__ vals, double* __restrict__ W, double* error,
                            double* ratio) {
   pdl_entry();
-  extern __shared__ double dense[];
-  double* Ls = dense;          // n x n, lower triangle
-  double* Xs = dense + n * n;  // n x n, X = L^-1 (lower triangle)
-  const int t = threadIdx.x, T = blockDim.x;
-  __shared__ int failed;
-  __shared__ double smallest, pivot;
-  __shared__ double diag0[kSharedDense];
-  if (t == 0) {
-    failed = 0;
-    smallest = 1.0;
-  }
-  for (int k = t; k < n * n; k += T) {
-    Ls[k] = 0.0;
-    Xs[k] = (k / n == k % n) ? 1.0 : 0.0;
-  }
+  extern __shared__ double dense[];  // n x n
+  __shared__ double column[2][kSharedDense], row[2][kSharedDense];
+  __shared__ double inverse[kSharedDense], diag0[kSharedDense];
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  bool failed = false;
+  double smallest = 1.0;  // thread 0's
+  for (int k = t; k < n * n; k += kDenseThreads) dense[k] = 0.0;
   __syncthreads();
-  for (int i = t; i < n; i += T)
+  for (int i = t; i < n; i += kDenseThreads)
     for (int j = rows[i]; j < rows[i + 1]; ++j) {
-      if (cols[j] <= i) Ls[i * n + cols[j]] = vals[j];
+      if (cols[j] <= i) dense[i * n + cols[j]] = vals[j];
       if (cols[j] == i) diag0[i] = vals[j];
     }
   __syncthreads();
+  double m[kDenseTile][kDenseTile];
+#pragma unroll
+  for (int a = 0; a < kDenseTile; ++a)
+#pragma unroll
+    for (int c = 0; c < kDenseTile; ++c) {
+      const int i = warp + 32 * a, j = lane + 32 * c;
+      m[a][c] = i < n && j <= i ? dense[i * n + j] : 0.0;
+      if (c == 0 && lane == 0 && i < n) column[0][i] = m[a][0];
+    }
+  __syncthreads();
   for (int k = 0; k < n; ++k) {
+    const int now = k & 1, next = now ^ 1;
+    double d = column[now][k];
+    const bool positive = d > 0.0;
     if (t == 0) {
-      double d = Ls[k * n + k];
-      if (!(d > 0.0)) {
-        failed = 1;
-        d = 1.0;
-      } else {
-        smallest = fmin(smallest, d / diag0[k]);
+      if (positive) smallest = fmin(smallest, d / diag0[k]);
+      else failed = true;
+    }
+    if (!positive) d = 1.0;
+    const double inv = 1.0 / d;
+    if (t == 0) inverse[k] = inv;
+    double s[kDenseTile];
+#pragma unroll
+    for (int c = 0; c < kDenseTile; ++c) {
+      const int j = lane + 32 * c;
+      s[c] = j >= n || j == k ? 0.0 : j < k ? row[now][j] : column[now][j];
+    }
+#pragma unroll
+    for (int a = 0; a < kDenseTile; ++a) {
+      const int i = warp + 32 * a;
+      if (i <= k || i >= n) continue;
+      const double f = column[now][i] * inv;
+#pragma unroll
+      for (int c = 0; c < kDenseTile; ++c) {
+        const int j = lane + 32 * c;
+        if (j > i) continue;
+        m[a][c] = j == k ? -f : fma(-f, s[c], m[a][c]);
+        if (j == k + 1) column[next][i] = m[a][c];
+        if (i == k + 1 && j <= k) row[next][j] = m[a][c];
       }
-      pivot = sqrt(d);
-      Ls[k * n + k] = pivot;
-    }
-    __syncthreads();
-    for (int i = k + 1 + t; i < n; i += T) Ls[i * n + k] /= pivot;
-    __syncthreads();
-    const int m = n - k - 1;  // trailing rows k+1 .. n-1
-    for (int p = t; p < m * (m + 1) / 2; p += T) {
-      int a, b;
-      triangle_pair(p, a, b);
-      const int i = k + 1 + a, j = k + 1 + b;
-      Ls[i * n + j] -= Ls[i * n + k] * Ls[j * n + k];
     }
     __syncthreads();
   }
-  // X = L^-1: step k scales row k of X by 1 / L_kk, then removes L_ik X_k from
-  // the rows below (only columns j <= k of X are nonzero at that point).
-  for (int k = 0; k < n; ++k) {
-    const double inv = 1.0 / Ls[k * n + k];
-    for (int j = t; j <= k; j += T) Xs[k * n + j] *= inv;
-    __syncthreads();
-    const int below = n - k - 1;
-    for (int p = t; p < below * (k + 1); p += T) {
-      const int i = k + 1 + p / (k + 1), j = p % (k + 1);
-      Xs[i * n + j] -= Ls[i * n + k] * Xs[k * n + j];
+#pragma unroll
+  for (int a = 0; a < kDenseTile; ++a)
+#pragma unroll
+    for (int c = 0; c < kDenseTile; ++c) {
+      const int i = warp + 32 * a, j = lane + 32 * c;
+      if (i < n && j < n) dense[i * n + j] = j < i ? m[a][c] : j == i ? 1.0 : 0.0;
     }
-    __syncthreads();
-  }
-  // W = X^T X: W_ij = sum_{k >= max(i, j)} X_ki X_kj.
-  for (int p = t; p < n * (n + 1) / 2; p += T) {
-    int i, j;
-    triangle_pair(p, i, j);
-    double acc = 0.0;
-    for (int k = i; k < n; ++k) acc += Xs[k * n + i] * Xs[k * n + j];
-    W[static_cast<std::size_t>(i) * n + j] = acc;
-    W[static_cast<std::size_t>(j) * n + i] = acc;
+  __syncthreads();
+  // W_ij = sum_{k >= i} X_ki X_kj / d_k for j <= i, a warp per row i.
+  for (int i = warp; i < n; i += 32) {
+    double acc[kDenseTile] = {};
+    for (int k = i; k < n; ++k) {
+      const double f = dense[k * n + i] * inverse[k];
+#pragma unroll
+      for (int c = 0; c < kDenseTile; ++c)
+        if (lane + 32 * c <= i) acc[c] = fma(f, dense[k * n + lane + 32 * c], acc[c]);
+    }
+#pragma unroll
+    for (int c = 0; c < kDenseTile; ++c) {
+      const int j = lane + 32 * c;
+      if (j > i) continue;
+      W[static_cast<std::size_t>(i) * n + j] = acc[c];
+      W[static_cast<std::size_t>(j) * n + i] = acc[c];
+    }
   }
   if (t == 0) {
     *error = failed ? 1.0 : 0.0;
@@ -744,10 +762,10 @@ void dense_inverse(int n, const int* rows, const int* cols, const float* vals, d
   if (n <= 0) return;
   ++counter;
   if (n <= kSharedDense) {
-    const int bytes = 2 * n * n * static_cast<int>(sizeof(double));
+    const int bytes = n * n * static_cast<int>(sizeof(double));
     static std::atomic<unsigned long long> raised{0};
     raise_shared_limit(reinterpret_cast<const void*>(k_dense_inverse_shared),
-                       2 * kSharedDense * kSharedDense * static_cast<int>(sizeof(double)), raised);
+                       kSharedDense * kSharedDense * static_cast<int>(sizeof(double)), raised);
     pdl(k_dense_inverse_shared, 1, kDenseThreads, bytes, s, n, rows, cols, vals, inverse, error,
                                                             ratio);
     return;
