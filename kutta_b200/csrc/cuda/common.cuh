@@ -272,8 +272,7 @@ __device__ __forceinline__ double nan_max(double a, double b) { return (b > a ||
 // 1 zero diagonal, 2 nonfinite, 3 negative diagonal under L1).
 __device__ __forceinline__ float diagonal_row(int i, const int* __restrict__ rows,
                                               const int* __restrict__ diag,
-                                              const float* __restrict__ vals,
-                                              float* __restrict__ inverse, int use_l1) {
+                                              const float* vals, float* inverse, int use_l1) {
   const float d = vals[diag[i]];
   float off = 0.0f, bad = 0.0f;
   for (int j = rows[i]; j < rows[i + 1]; ++j) {
@@ -287,6 +286,15 @@ __device__ __forceinline__ float diagonal_row(int i, const int* __restrict__ row
   return (bad != 0.0f || inv - inv != 0.0f || l1 - l1 != 0.0f)
              ? 2.0f
              : (use_l1 != 0 && d < 0.0f ? 3.0f : (d == 0.0f ? 1.0f : 0.0f));
+}
+// amg_m_matrix_diagonal's share of fine row i (src/kutta/kernels/amg.kern.h:44-58):
+// its diagonal plus its off-diagonals, upward rounded.
+__device__ __forceinline__ float row_surplus(int i, const int* __restrict__ rows,
+                                             const int* __restrict__ diag, const float* vals) {
+  UpperSum sum{vals[diag[i]], 0.0f};
+  for (int j = rows[i]; j < rows[i + 1]; ++j)
+    if (j != diag[i]) sum = upper_add(sum, vals[j]);
+  return upper_value(sum);
 }
 __device__ __forceinline__ double warp_max(double v) {
 #pragma unroll

@@ -6,6 +6,8 @@
 // fixed tree; they are fused into the kernel that produces their operand and the
 // last block runs the reference's single-thread scalar update as an epilogue,
 // so a PCG iteration is a handful of launches instead of a dozen.
+#include <cuda_bf16.h>
+
 #include "common.cuh"
 #include "kernels.hpp"
 
@@ -495,12 +497,7 @@ __global__ void k_galerkin(int nnz_c, const int* __restrict__ offsets,
 __global__ void k_row_surplus(int n, const int* __restrict__ rows, const int* __restrict__ diag,
                               const float* __restrict__ fine, float* __restrict__ surplus) {
   pdl_entry();
-  ROWS(i, n) {
-    UpperSum sum{fine[diag[i]], 0.0f};
-    for (int j = rows[i]; j < rows[i + 1]; ++j)
-      if (j != diag[i]) sum = upper_add(sum, fine[j]);
-    surplus[i] = upper_value(sum);
-  }
+  ROWS(i, n) surplus[i] = row_surplus(i, rows, diag, fine);
 }
 
 __global__ void k_m_matrix_combine(int nc, const int* __restrict__ offsets,
@@ -515,6 +512,56 @@ __global__ void k_m_matrix_combine(int nc, const int* __restrict__ offsets,
     for (int j = rows[g]; j < rows[g + 1]; ++j)
       if (j != diag[g]) diagonal = upper_add(diagonal, -coarse[j]);
     coarse[diag[g]] = upper_value(diagonal);
+  }
+}
+
+// A level's row data in one pass of a refresh, where each was a launch of its
+// own: with kCombine the M-matrix diagonal (k_m_matrix_combine), then the
+// inverse L1 diagonal and its invalid flag (k_diagonal), and where wanted the
+// row's surplus for the level below (k_row_surplus) and its BF16 copy
+// (k_bf16_pack). A thread's row stays in L1 between the parts, and every part
+// is the same operations in the same order. Assembly, refresh and corrections on
+// the 1.57M-row tet hierarchy take 15 launches instead of 30, 440 us instead of
+// 462.
+template <bool kCombine>
+__global__ void k_level_rows(int n, const int* __restrict__ rows, const int* __restrict__ diag,
+                             float* vals, const int* __restrict__ offsets,
+                             const int* __restrict__ members,
+                             const float* __restrict__ fine_surplus, float* __restrict__ inverse,
+                             float* __restrict__ surplus, unsigned short* __restrict__ v16,
+                             float* __restrict__ scale, DeviceReducer red, double* check,
+                             int slot) {
+  pdl_entry();
+  double worst = 0;
+  ROWS(i, n) {
+    if constexpr (kCombine) {
+      UpperSum diagonal{0.0f, 0.0f};
+      for (int m = offsets[i]; m < offsets[i + 1]; ++m)
+        diagonal = upper_add(diagonal, fine_surplus[members[m]]);
+      for (int j = rows[i]; j < rows[i + 1]; ++j)
+        if (j != diag[i]) diagonal = upper_add(diagonal, -vals[j]);
+      vals[diag[i]] = upper_value(diagonal);
+    }
+    worst = nan_max(worst, diagonal_row(i, rows, diag, vals, inverse, 1));
+    if (surplus != nullptr) surplus[i] = row_surplus(i, rows, diag, vals);
+    if (v16 != nullptr) {
+      float most = 0.0f;
+      for (int j = rows[i]; j < rows[i + 1]; ++j) most = fmaxf(most, fabsf(vals[j]));
+      const float s = most > 0.0f ? most : 1.0f;
+      scale[i] = s;
+      const float inv = 1.0f / s;
+      for (int j = rows[i]; j < rows[i + 1]; ++j)
+        v16[j] = __bfloat16_as_ushort(__float2bfloat16_rn(vals[j] * inv));
+    }
+  }
+  __shared__ double shared[32];
+  worst = block_max(worst, shared);
+  const Reducer r = as_reducer(red);
+  if (!publish(r, worst, 0, false)) return;
+  const double total = gather_max(r, shared);
+  if (threadIdx.x == 0) {
+    check[slot] = total;
+    *r.ticket = 0;
   }
 }
 
@@ -853,6 +900,16 @@ void m_matrix_diagonal(int nf, int nc, const int* offsets, const int* members, c
   ++counter;
   pdl(k_m_matrix_combine, full_grid(nc), kBlock, 0, s, nc, offsets, members, surplus, rows, diag,
                                                       coarse);
+}
+void level_rows(int n, const int* rows, const int* diag, float* vals, const LevelRows& p,
+                DeviceReducer red, double* check, int slot, cudaStream_t s) {
+  ++counter;
+  if (p.members != nullptr)
+    pdl(k_level_rows<true>, blocks(n), kBlock, 0, s, n, rows, diag, vals, p.offsets, p.members,
+        p.fine_surplus, p.inverse, p.surplus, p.v16, p.scale, red, check, slot);
+  else
+    pdl(k_level_rows<false>, blocks(n), kBlock, 0, s, n, rows, diag, vals, p.offsets, p.members,
+        p.fine_surplus, p.inverse, p.surplus, p.v16, p.scale, red, check, slot);
 }
 void pcg_step_dot(int n, float* x, float* r, const float* p, const float* q, DeviceReducer red,
                   float* scalars, int* status, cudaStream_t s) {

@@ -65,13 +65,18 @@ __global__ void k_fv_pressure_assemble(int n, const int* __restrict__ offsets,
                                        const float* __restrict__ coefficient,
                                        const float* __restrict__ flux, float* __restrict__ values,
                                        float* __restrict__ rhs, int reference,
-                                       float* __restrict__ inverse, DeviceReducer red,
+                                       float* __restrict__ inverse,
+                                       float* __restrict__ surplus, DeviceReducer red,
                                        double* check, int slot) {
+  pdl_entry();
   double worst = 0;
   ROWS(i, n) {
     rhs[i] = assemble_row(i, offsets, faces, sign, adjacent, entry, rows, diag, coefficient, flux,
                           values, reference);
-    if constexpr (kFused) worst = nan_max(worst, diagonal_row(i, rows, diag, values, inverse, 1));
+    if constexpr (kFused) {
+      worst = nan_max(worst, diagonal_row(i, rows, diag, values, inverse, 1));
+      if (surplus != nullptr) surplus[i] = row_surplus(i, rows, diag, values);
+    }
   }
   if constexpr (kFused) {
     __shared__ double shared[32];
@@ -91,6 +96,7 @@ __global__ void k_fv_correct_flux(int n, const int* __restrict__ owner,
                                   const float* __restrict__ correction,
                                   const float* __restrict__ coefficient, float* __restrict__ flux,
                                   int internal) {
+  pdl_entry();
   ROWS(i, n) {
     const float pc = correction[owner[i]];
     const float pn = i < internal ? correction[neighbour[i]] : 0.0f;
@@ -106,6 +112,7 @@ __global__ void k_fv_correct_velocity(int n, const float* __restrict__ volume,
                                       const float* __restrict__ correction, float* __restrict__ u,
                                       float* __restrict__ v, float* __restrict__ w,
                                       float* __restrict__ p, float alpha) {
+  pdl_entry();
   ROWS(i, n) {
     const float d = volume[i] * inverse[i];
     u[i] -= d * gx[i];
@@ -128,29 +135,30 @@ void fv_pressure_assemble(int n, const int* offsets, const int* faces, const flo
                           int reference, cudaStream_t s) {
   if (n <= 0) return;
   ++counter;
-  k_fv_pressure_assemble<false><<<grid_for(n), kBlock, 0, s>>>(
-      n, offsets, faces, sign, adjacent, entry, rows, diag, coefficient, flux, values, rhs,
-      reference, nullptr, DeviceReducer{nullptr, nullptr}, nullptr, 0);
+  pdl(k_fv_pressure_assemble<false>, grid_for(n), kBlock, 0, s, n, offsets, faces, sign, adjacent,
+      entry, rows, diag, coefficient, flux, values, rhs, reference, static_cast<float*>(nullptr),
+      static_cast<float*>(nullptr), DeviceReducer{nullptr, nullptr}, static_cast<double*>(nullptr),
+      0);
 }
 
 void fv_pressure_assemble_l1(int n, const int* offsets, const int* faces, const float* sign,
                              const int* adjacent, const int* entry, const int* rows,
                              const int* diag, const float* coefficient, const float* flux,
                              float* values, float* rhs, int reference, float* inverse,
-                             DeviceReducer red, double* check, int slot, cudaStream_t s) {
+                             float* surplus, DeviceReducer red, double* check, int slot, cudaStream_t s) {
   if (n <= 0) return;
   ++counter;
-  k_fv_pressure_assemble<true><<<grid_for(n), kBlock, 0, s>>>(
-      n, offsets, faces, sign, adjacent, entry, rows, diag, coefficient, flux, values, rhs,
-      reference, inverse, red, check, slot);
+  pdl(k_fv_pressure_assemble<true>, grid_for(n), kBlock, 0, s, n, offsets, faces, sign, adjacent,
+      entry, rows, diag, coefficient, flux, values, rhs, reference, inverse, surplus, red, check,
+      slot);
 }
 
 void fv_correct_flux(int n, const int* owner, const int* neighbour, const float* correction,
                      const float* coefficient, float* flux, int internal, cudaStream_t s) {
   if (n <= 0) return;
   ++counter;
-  k_fv_correct_flux<<<grid_for(n), kBlock, 0, s>>>(n, owner, neighbour, correction, coefficient,
-                                                   flux, internal);
+  pdl(k_fv_correct_flux, grid_for(n), kBlock, 0, s, n, owner, neighbour, correction, coefficient,
+      flux, internal);
 }
 
 void fv_correct_velocity(int n, const float* volume, const float* inverse, const float* diagonal,
@@ -159,8 +167,8 @@ void fv_correct_velocity(int n, const float* volume, const float* inverse, const
                          float alpha, cudaStream_t s) {
   if (n <= 0) return;
   ++counter;
-  k_fv_correct_velocity<<<grid_for(n), kBlock, 0, s>>>(n, volume, inverse, diagonal, gx, gy, gz,
-                                                       correction, u, v, w, p, alpha);
+  pdl(k_fv_correct_velocity, grid_for(n), kBlock, 0, s, n, volume, inverse, diagonal, gx, gy, gz,
+      correction, u, v, w, p, alpha);
 }
 
 }  // namespace launch

@@ -107,6 +107,22 @@ void m_matrix_diagonal(int nf, int nc, const int* offsets, const int* members, c
                        const int* fine_diag, const float* fine, const int* rows, const int* diag,
                        float* coarse, float* surplus, cudaStream_t s);
 
+// A level's row data in one refresh pass: with members the M-matrix diagonal
+// into vals (from the level above's fine_surplus), the inverse L1 diagonal with
+// its invalid flags' maximum in check[slot], and where not null the rows'
+// surplus and BF16 copy (v16, scale).
+struct LevelRows {
+  const int* offsets;
+  const int* members;
+  const float* fine_surplus;
+  float* inverse;
+  float* surplus;
+  unsigned short* v16;
+  float* scale;
+};
+void level_rows(int n, const int* rows, const int* diag, float* vals, const LevelRows& p,
+                DeviceReducer red, double* check, int slot, cudaStream_t s);
+
 // ---- plain coarse levels (coarse_rows.cu) -----------------------------------
 // The residual and sweep above for levels with long rows or few of them (the
 // same bits): all threads of a block form the products of its rows' entries,
@@ -345,7 +361,7 @@ void gnn_layer_b(int n, const int* rows, const int* cols, const float* edge,
 
 // ---- finite-volume steps around the pressure solve (fv_kernels.cu) ---------
 // fv_pressure_assemble (fv_flow.kern.h:164-183); the _l1 form also writes
-// the rows' inverse L1 diagonal and the max invalid flag into check[slot].
+// the rows' inverse L1 diagonal, the max invalid flag into check[slot] and, with surplus, row surpluses.
 void fv_pressure_assemble(int n, const int* offsets, const int* faces, const float* sign,
                           const int* adjacent, const int* entry, const int* rows, const int* diag,
                           const float* coefficient, const float* flux, float* values, float* rhs,
@@ -354,7 +370,8 @@ void fv_pressure_assemble_l1(int n, const int* offsets, const int* faces, const 
                              const int* adjacent, const int* entry, const int* rows,
                              const int* diag, const float* coefficient, const float* flux,
                              float* values, float* rhs, int reference, float* inverse,
-                             DeviceReducer red, double* check, int slot, cudaStream_t s);
+                             float* surplus, DeviceReducer red, double* check, int slot,
+                             cudaStream_t s);
 void fv_correct_flux(int n, const int* owner, const int* neighbour, const float* correction,
                      const float* coefficient, float* flux, int internal, cudaStream_t s);
 void fv_correct_velocity(int n, const float* volume, const float* inverse, const float* diagonal,

@@ -371,14 +371,15 @@ void Solver::plan_tail() {
   }
 }
 
-// BF16 copies of the coarse operators and the dense inverse of the coarsest,
-// from the current FP32 coarse values; the dense SPD check lands in values_[0].
-void Solver::prepare_mixed(cudaStream_t s, int slot) {
+// BF16 copies of the coarse operators (unless the refresh's row pass has made
+// them) and the dense inverse of the coarsest, from the current FP32 coarse
+// values; the dense SPD check lands in values_[slot].
+void Solver::prepare_mixed(cudaStream_t s, int slot, bool packed) {
   double* error = values_.get() + slot;
   cuda_check(cudaMemsetAsync(error, 0, 2 * sizeof(double), s), "memset");
   for (std::size_t i = 1; i < levels_.size(); ++i) {
     auto& l = levels_[i];
-    if (l.v16.allocated())
+    if (l.v16.allocated() && !packed)
       launch::bf16_pack(l.n, l.row_ptr.get(), l.val.get(), l.v16.get(), l.scale.get(), s);
     if (dense(l))
       launch::dense_inverse(l.n, l.row_ptr.get(), l.col.get(), l.val.get(), l.dense_lower.get(),
@@ -900,37 +901,53 @@ void Solver::assemble_refresh(const FvPressure& fv, float* values, float* rhs, c
   auto& l = levels_[0];
   launch::fv_pressure_assemble_l1(n_, fv.offsets, fv.faces, fv.sign, fv.adjacent, fv.entry,
                                   l.row_ptr.get(), l.diag.get(), fv.coefficient, fv.flux, values,
-                                  rhs, fv.reference, l.l1.get(), reducer(), values_.get(), 0, s);
+                                  rhs, fv.reference, l.l1.get(), surplus(0), reducer(),
+                                  values_.get(), 0, s);
   refresh_levels(values, true, s);
+}
+
+// Scratch for level i's row surpluses, which level i + 1's pass reads while it
+// writes its own: two buffers in turn. Null where nothing needs them.
+float* Solver::surplus(std::size_t i) {
+  if (!options_.m_matrix || i + 1 >= levels_.size()) return nullptr;
+  auto& buffer = surplus_[i % 2];
+  if (!buffer.allocated()) buffer.reset(static_cast<std::size_t>(levels_[i % 2].n));
+  return buffer.get();
 }
 
 void Solver::refresh_levels(const float* val, bool fine_done, cudaStream_t s) {
   const float* matrix = val;
   std::vector<double> allowed;
-  if (options_.m_matrix && !surplus_.allocated() && levels_.size() > 1)
-    surplus_.reset(static_cast<std::size_t>(n_));
   for (std::size_t i = 0; i < levels_.size(); ++i) {
     auto& l = levels_[i];
-    if (i > 0 || !fine_done)
-      launch::diagonal(l.n, l.row_ptr.get(), l.diag.get(), matrix, l.l1.get(), 1, reducer(),
-                       values_.get(), static_cast<int>(i), s);
     allowed.push_back(nullspace_ && l.n == 1 ? 1 : 0);
-    if (i + 1 < levels_.size()) {
-      auto& c = levels_[i + 1];
-      launch::galerkin(c.nnz, l.entry_offsets.get(), l.entries.get(), matrix, c.val.get(), s);
-      if (options_.m_matrix)
-        launch::m_matrix_diagonal(l.n, c.n, l.member_offsets.get(), l.members.get(),
-                                  l.row_ptr.get(), l.diag.get(), matrix, c.row_ptr.get(),
-                                  c.diag.get(), c.val.get(), surplus_.get(), s);
-      matrix = c.val.get();
+    launch::LevelRows p{};
+    p.inverse = l.l1.get();
+    p.surplus = i + 1 < levels_.size() ? surplus(i) : nullptr;
+    if (i > 0) {
+      auto& above = levels_[i - 1];
+      launch::galerkin(l.nnz, above.entry_offsets.get(), above.entries.get(), matrix, l.val.get(),
+                       s);
+      if (options_.m_matrix) {
+        p.offsets = above.member_offsets.get();
+        p.members = above.members.get();
+        p.fine_surplus = surplus(i - 1);
+      }
+      p.v16 = l.v16.get();
+      p.scale = l.scale.get();
+      matrix = l.val.get();
     }
+    // Without members the pass writes no values, so the caller's stay untouched.
+    if (i > 0 || !fine_done)
+      launch::level_rows(l.n, l.row_ptr.get(), l.diag.get(), const_cast<float*>(matrix), p,
+                         reducer(), values_.get(), static_cast<int>(i), s);
   }
   const int slots = static_cast<int>(levels_.size());
   if (packed_.width > 0)
     launch::pack_rows(n_, packed_.width, rows0(), cols0(), levels_[0].diag.get(), val,
                       packed_.vals.get(), packed_.diag.get(), s);
   if (plain_tail_start_ != 0) launch::plain_tail_entries(plain_tail_, s);
-  if (mixed()) prepare_mixed(s, slots);
+  if (mixed()) prepare_mixed(s, slots, true);
   cuda_check(cudaMemcpyAsync(host_values_.get(), values_.get(),
                              sizeof(double) * (slots + (mixed() ? 2 : 0)), cudaMemcpyDeviceToHost, s),
              "refresh readback");

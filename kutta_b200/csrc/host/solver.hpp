@@ -145,7 +145,8 @@ class Solver {
   // Refresh from the level-0 values; fine_done: level 0's L1 diagonal and
   // check slot are already written (by the fused assembly).
   void refresh_levels(const float* val, bool fine_done, cudaStream_t s);
-  void prepare_mixed(cudaStream_t s, int error_slot);
+  void prepare_mixed(cudaStream_t s, int error_slot, bool packed = false);
+  float* surplus(std::size_t level);
   void choose_coarsest(double smallest_pivot);
   bool dense_ok_ = false;  // the dense coarsest inverse is used (well conditioned)
   // Cluster-fused tail of the mixed V-cycle: levels >= tail_start_ in one launch.
@@ -298,7 +299,7 @@ class Solver {
   std::vector<DevLevel> levels_;
   double complexity_ = 0;
   DArray<float> jacobi_inverse_;  // Jacobi preconditioner
-  DArray<float> surplus_;         // M-matrix diagonal scratch (fine rows)
+  DArray<float> surplus_[2];      // M-matrix diagonal scratch (levels in turn)
   float *r_ = nullptr, *z_ = nullptr, *p_ = nullptr, *q_ = nullptr, *shadow_ = nullptr,
         *s_ = nullptr, *t_ = nullptr, *zs_ = nullptr, *best_ = nullptr, *scratch_ = nullptr;
   DArray<float> scalars_, projection_;
