@@ -98,9 +98,10 @@ __device__ __forceinline__ Pair kp_add(Pair a, Pair b) {
   return kp(h, e - (h - s));
 }
 __device__ __forceinline__ Pair kp_neg(Pair a) { return kp(-a.hi, -a.lo); }
+// The products are rounded before they are added, also where contraction is on.
 __device__ __forceinline__ Pair kp_mul(Pair a, Pair b) {
-  const float h = a.hi * b.hi;
-  const float l = fmaf(a.hi, b.hi, -h) + a.hi * b.lo + a.lo * b.hi;
+  const float h = __fmul_rn(a.hi, b.hi);
+  const float l = fmaf(a.hi, b.hi, -h) + __fmul_rn(a.hi, b.lo) + __fmul_rn(a.lo, b.hi);
   return kp_add(kp(h, 0.0f), kp(l, 0.0f));
 }
 __device__ __forceinline__ Pair kp_div(Pair a, Pair b) {

@@ -209,14 +209,21 @@ void bf16_residual(int n, const int* rows, const int* cols, const unsigned short
 // Restriction for the mixed V-cycle: plain FP32 sums, four lanes per aggregate.
 void restrict_lanes(int nc, const int* offsets, const int* members, const float* fine,
                     float* coarse, const int* status, cudaStream_t s);
-// K-cycle inner step on a BF16 level: q = A p with p.q and w.p (gcr: q.q and
-// w.q) -> scalars[0..3], skipped while status[0] != 0.
+// K-cycle inner step on a BF16 level: q = A p, p.q and w.p -> scalars[0..3],
+// then alpha (inner_alpha). With copy != null the first step of a cycle: p is
+// copied there, the guard is the parent's status and the level's own starts.
 void bf16_spmv_dot2(int n, const int* rows, const int* cols, const unsigned short* v16,
-                    const float* scale, const float* p, const float* w, float* q, bool gcr,
-                    DeviceReducer red, float* scalars, const int* status, cudaStream_t s);
-// inner_first fused with the t.t, b.b reduction -> scalars[4..7].
+                    const float* scale, const float* p, const float* w, float* q, float* copy,
+                    DeviceReducer red, float* scalars, const int* parent, int* status,
+                    cudaStream_t s);
+// bf16_smooth from x with next.q -> scalars[4..5] and beta (inner_beta).
+void bf16_smooth_dot(int n, const int* rows, const int* cols, const unsigned short* v16,
+                     const float* scale, const float* x, const float* b, const float* inv,
+                     float* next, const float* q, DeviceReducer red, float* scalars, int* status,
+                     cudaStream_t s);
+// inner_first, t.t and b.b -> scalars[4..7] and the exit check (inner_check).
 void inner_first_dot(int n, const float* b, const float* p, const float* q, float* x, float* t,
-                     float* scalars, const int* status, DeviceReducer red, cudaStream_t s);
+                     float* scalars, int* status, DeviceReducer red, cudaStream_t s);
 // Dense FP64 Cholesky of an n <= 1024 CSR operator and its explicit inverse
 // (n x n, row-major, into `inverse`; `lower` is n x n scratch); *error = 1 if
 // the operator is not SPD.

@@ -160,57 +160,121 @@ __global__ void k_restrict_lanes(int nc, const int* __restrict__ offsets,
   });
 }
 
-// The last block stores the two FP64 totals as (hi, lo) pairs at
-// scalars[offset] and scalars[offset + 2].
-__device__ __forceinline__ void finish_dot2(DeviceReducer red, double a, double b,
+// The last block stores the FP64 totals as (hi, lo) pairs at scalars[offset]
+// and scalars[offset + 2]; returns true in its thread 0, which may then run the
+// scalar step that follows (every block has read the status by then).
+__device__ __forceinline__ bool finish_dot2(DeviceReducer red, double a, double b,
                                             float* scalars, int offset) {
   __shared__ double shared[32];
   a = block_sum(a, shared);
   b = block_sum(b, shared);
   const Reducer r{red.partials, red.ticket};
-  if (!publish(r, a, b, true)) return;
+  if (!publish(r, a, b, true)) return false;
   const double total_a = gather(r, 0, shared);
   const double total_b = gather(r, 1, shared);
-  if (threadIdx.x == 0) {
-    store_pair(scalars, offset, total_a);
-    store_pair(scalars, offset + 2, total_b);
-    *r.ticket = 0;
-  }
+  if (threadIdx.x != 0) return false;
+  store_pair(scalars, offset, total_a);
+  store_pair(scalars, offset + 2, total_b);
+  *r.ticket = 0;
+  return true;
+}
+
+// The K-cycle's scalar steps (scalars.kern.h:154-186), each run by the last
+// block of the reduction that produces its operands: as kernels of one thread
+// they cost a launch of 1.1 us each, four times per inner step.
+__device__ __forceinline__ void inner_alpha(float* scalars, int* status, bool first) {
+  const Pair denom = kp_load(scalars, 0);
+  const Pair alpha = kp_div(kp_load(scalars, 2), denom);
+  if (!kp_positive(denom) || !kp_coefficient(alpha) ||
+      (kp_zero(alpha) && !kp_zero(kp_load(scalars, 2))))
+    status[0] = first ? 2 : 1;
+  else
+    kp_store(scalars, 8, alpha);
+}
+// Adaptive exit: keep the first correction when |t|^2 <= |b|^2 / 16.
+__device__ __forceinline__ void inner_check(const float* scalars, int* status) {
+  if (kp_le(kp_load(scalars, 4), kp_mul(kp(0.0625f, 0.0f), kp_load(scalars, 6)))) status[0] = 1;
+}
+__device__ __forceinline__ void inner_beta(float* scalars, int* status) {
+  const Pair beta = kp_div(kp_neg(kp_load(scalars, 4)), kp_load(scalars, 0));
+  if (!kp_coefficient(beta) || (kp_zero(beta) && !kp_zero(kp_load(scalars, 4))))
+    status[0] = 1;
+  else
+    kp_store(scalars, 10, beta);
 }
 
 // K-cycle inner step on a BF16 level: q = A p and, in the same pass, the two
-// products its step length needs -> scalars[0..3]: p.q and w.p (A-conjugate,
-// SPD) or q.q and w.q (GCR). Skipped while status[0] != 0.
+// products its step length needs, p.q and w.p -> scalars[0..3], then alpha.
+// kFirst: p is the level's z, copied to `copy` on the way, `status` is the
+// parent's, and the level's own status starts here (2, the plain cycle, while
+// the parent has stopped); otherwise status is the level's own.
+template <bool kFirst>
 __global__ void k_bf16_spmv_dot2(int n, const int* __restrict__ rows, const int* __restrict__ cols,
                                  const unsigned short* __restrict__ v16,
                                  const float* __restrict__ scale, const float* __restrict__ p,
-                                 const float* __restrict__ w, float* __restrict__ q, bool gcr,
-                                 DeviceReducer red, float* scalars,
-                                 const int* __restrict__ status) {
+                                 const float* __restrict__ w, float* __restrict__ q,
+                                 float* __restrict__ copy, DeviceReducer red, float* scalars,
+                                 const int* status, int* own) {
   pdl_entry();
-  if (status[0] != 0) return;
+  if (status[0] != 0) {
+    if (kFirst && blockIdx.x == 0 && threadIdx.x == 0) own[0] = 2;
+    return;
+  }
   double a = 0.0, b = 0.0;
   for_rows(n, [&](int i, int lane, bool valid) {
     const float acc = row_total(valid ? bf16_row_part(i, lane, rows, cols, v16, p) : 0.0f);
     if (valid && lane == 0) {
-      const float qi = scale[i] * acc;
+      const float qi = scale[i] * acc, pi = p[i];
       q[i] = qi;
-      const double d = gcr ? static_cast<double>(qi) : static_cast<double>(p[i]);
-      a += d * static_cast<double>(qi);
-      b += static_cast<double>(w[i]) * d;
+      if (kFirst) copy[i] = pi;
+      a += static_cast<double>(pi) * static_cast<double>(qi);
+      b += static_cast<double>(w[i]) * static_cast<double>(pi);
     }
   });
-  finish_dot2(red, a, b, scalars, 0);
+  if (!finish_dot2(red, a, b, scalars, 0)) return;
+  if (kFirst) own[0] = 0;
+  inner_alpha(scalars, own, kFirst);
+}
+
+// The last sweep of the second inner cycle with z.q -> scalars[4..5] (q = A p of
+// the first) and beta.
+__global__ void k_bf16_smooth_dot(int n, const int* __restrict__ rows,
+                                  const int* __restrict__ cols,
+                                  const unsigned short* __restrict__ v16,
+                                  const float* __restrict__ scale, const float* __restrict__ x,
+                                  const float* __restrict__ b, const float* __restrict__ inv,
+                                  float* __restrict__ next, const float* __restrict__ q,
+                                  DeviceReducer red, float* scalars, int* status) {
+  pdl_entry();
+  if (status[0] != 0) return;
+  double a = 0.0;
+  for_rows(n, [&](int i, int lane, bool valid) {
+    const float acc = row_total(valid ? bf16_row_part(i, lane, rows, cols, v16, x) : 0.0f);
+    if (valid && lane == 0) {
+      const float z = x[i] + (2.0f / 3.0f) * inv[i] * (b[i] - scale[i] * acc);
+      next[i] = z;
+      a += static_cast<double>(z) * static_cast<double>(q[i]);
+    }
+  });
+  __shared__ double shared[32];
+  a = block_sum(a, shared);
+  const Reducer r{red.partials, red.ticket};
+  if (!publish(r, a, 0.0, false)) return;
+  const double total = gather(r, 0, shared);
+  if (threadIdx.x != 0) return;
+  store_pair(scalars, 4, total);
+  *r.ticket = 0;
+  inner_beta(scalars, status);
 }
 
 // amg_inner_first with the next reduction fused: x = alpha p, t = b - alpha q
 // (or x = p, t = 0 when the level's status is not running), then t.t and b.b
-// -> scalars[4..7]. Skipped (reduction included) while status[0] != 0, as
-// every reader of those slots is.
+// -> scalars[4..7] and the exit check. Skipped (reduction included) while
+// status[0] != 0, as every reader of those slots is.
 __global__ void k_inner_first_dot(int n, const float* __restrict__ b, const float* __restrict__ p,
                                   const float* __restrict__ q, float* __restrict__ x,
-                                  float* __restrict__ t, float* scalars,
-                                  const int* __restrict__ status, DeviceReducer red) {
+                                  float* __restrict__ t, float* scalars, int* status,
+                                  DeviceReducer red) {
   pdl_entry();
   const bool running = status[0] == 0;
   const float alpha = kp_float(kp_load(scalars, 8));
@@ -223,7 +287,7 @@ __global__ void k_inner_first_dot(int n, const float* __restrict__ b, const floa
     bb += static_cast<double>(b[i]) * static_cast<double>(b[i]);
   }
   if (!running) return;
-  finish_dot2(red, tt, bb, scalars, 4);
+  if (finish_dot2(red, tt, bb, scalars, 4)) inner_check(scalars, status);
 }
 
 // Dense FP64 Cholesky of the coarsest operator and its explicit inverse for
@@ -736,15 +800,29 @@ void restrict_lanes(int nc, const int* offsets, const int* members, const float*
                                                             status);
 }
 void bf16_spmv_dot2(int n, const int* rows, const int* cols, const unsigned short* v16,
-                    const float* scale, const float* p, const float* w, float* q, bool gcr,
-                    DeviceReducer red, float* scalars, const int* status, cudaStream_t s) {
+                    const float* scale, const float* p, const float* w, float* q, float* copy,
+                    DeviceReducer red, float* scalars, const int* parent, int* status,
+                    cudaStream_t s) {
   if (n <= 0) return;
   ++counter;
-  pdl(k_bf16_spmv_dot2, lanes_grid(n, true), kBlock, 0, s, n, rows, cols, v16, scale, p, w, q,
-                                                          gcr, red, scalars, status);
+  if (copy != nullptr)
+    pdl(k_bf16_spmv_dot2<true>, lanes_grid(n, true), kBlock, 0, s, n, rows, cols, v16, scale, p, w,
+        q, copy, red, scalars, parent, status);
+  else
+    pdl(k_bf16_spmv_dot2<false>, lanes_grid(n, true), kBlock, 0, s, n, rows, cols, v16, scale, p, w,
+        q, copy, red, scalars, static_cast<const int*>(status), status);
+}
+void bf16_smooth_dot(int n, const int* rows, const int* cols, const unsigned short* v16,
+                     const float* scale, const float* x, const float* b, const float* inv,
+                     float* next, const float* q, DeviceReducer red, float* scalars, int* status,
+                     cudaStream_t s) {
+  if (n <= 0) return;
+  ++counter;
+  pdl(k_bf16_smooth_dot, lanes_grid(n, true), kBlock, 0, s, n, rows, cols, v16, scale, x, b, inv,
+      next, q, red, scalars, status);
 }
 void inner_first_dot(int n, const float* b, const float* p, const float* q, float* x, float* t,
-                     float* scalars, const int* status, DeviceReducer red, cudaStream_t s) {
+                     float* scalars, int* status, DeviceReducer red, cudaStream_t s) {
   if (n <= 0) return;
   ++counter;
   pdl(k_inner_first_dot, grid_for(n), kBlock, 0, s, n, b, p, q, x, t, scalars, status, red);

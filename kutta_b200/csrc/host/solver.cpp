@@ -529,7 +529,10 @@ void Solver::smooth(DevLevel& l, const int* rows, const int* cols, const float* 
              : (packed_rows ? fine_operator_bytes() : 8.0 * l.nnz + 4.0 * (l.n + 1)) +
                    (with_dots ? 20.0 : 16.0) * l.n;
     if (timed) event_bytes_.push_back(bytes);
-    if (l.v16.allocated())
+    if (inner_dot_ == &l && !zero_start && sweep + 1 == sweeps)
+      launch::bf16_smooth_dot(l.n, rows, cols, l.v16.get(), l.scale.get(), x, b, l.l1.get(), l.r,
+                              l.q.get(), reducer(), l.scalars.get(), l.status.get(), stream_);
+    else if (l.v16.allocated())
       launch::bf16_smooth(l.n, rows, cols, l.v16.get(), l.scale.get(), x, b, l.l1.get(), l.r,
                           status, zero, stream_);
     else if (packed_rows)
@@ -660,45 +663,47 @@ void Solver::inner(std::size_t index, const int* parent) {
   const double bf16_bytes = 6.0 * l.nnz + 4.0 * (n + 1) + 16.0 * n;
 
   cycle(index, l.b.get(), l.z, parent);
-  copy(p, l.z, n);
   if (bf16) {
-    launch::bf16_spmv_dot2(n, rows, cols, l.v16.get(), l.scale.get(), p, l.b.get(), q, false,
-                           reducer(), sc, parent, stream_);
-    tally(bf16_bytes);
+    // The scalar steps ride on the reductions that produce their operands.
+    launch::bf16_spmv_dot2(n, rows, cols, l.v16.get(), l.scale.get(), l.z, l.b.get(), q, p,
+                           reducer(), sc, parent, st, stream_);
+    tally(bf16_bytes + 4.0 * n);
+    launch::inner_first_dot(n, l.b.get(), p, q, l.x, t, sc, st, reducer(), stream_);
+    tally(24.0 * n);
+    const DevLevel* outer = inner_dot_;
+    inner_dot_ = &l;
+    cycle(index, t, l.z, st);
+    inner_dot_ = outer;
   } else {
+    copy(p, l.z, n);
     launch::spmv(n, rows, cols, vals, p, q, parent, stream_);
     tally(spmv_bytes);
     reduce_into(ReduceMode::Dot2, n, spd ? p : q, q, l.b.get(), spd ? p : q, sc, 0, parent);
-  }
-  launch::inner_alpha(sc, st, parent, 1, stream_);
-  if (bf16) {
-    launch::inner_first_dot(n, l.b.get(), p, q, l.x, t, sc, st, reducer(), stream_);
-    tally(24.0 * n);
-  } else {
+    launch::inner_alpha(sc, st, parent, 1, stream_);
     launch::inner_first(n, l.b.get(), p, q, l.x, t, sc, st, stream_);
     tally(24.0 * n);
     reduce_into(ReduceMode::Dot2, n, t, t, l.b.get(), l.b.get(), sc, 4, st);
+    launch::inner_check(sc, st, stream_);
+    cycle(index, t, l.z, st);
+    if (!spd) {
+      launch::spmv(n, rows, cols, vals, l.z, l.r, st, stream_);
+      tally(spmv_bytes);
+    }
+    reduce_into(ReduceMode::Dot, n, spd ? l.z : l.r, q, nullptr, nullptr, sc, 4, st);
+    launch::inner_beta(sc, st, stream_);
   }
-  launch::inner_check(sc, st, stream_);
-  cycle(index, t, l.z, st);
-  if (!spd) {
-    launch::spmv(n, rows, cols, vals, l.z, l.r, st, stream_);
-    tally(spmv_bytes);
-  }
-  reduce_into(ReduceMode::Dot, n, spd ? l.z : l.r, q, nullptr, nullptr, sc, 4, st);
-  launch::inner_beta(sc, st, stream_);
   launch::direction(n, l.z, p, sc, st, stream_);
   tally(12.0 * n);
   if (bf16) {
-    launch::bf16_spmv_dot2(n, rows, cols, l.v16.get(), l.scale.get(), p, t, q, false, reducer(),
-                           sc, st, stream_);
+    launch::bf16_spmv_dot2(n, rows, cols, l.v16.get(), l.scale.get(), p, t, q, nullptr, reducer(),
+                           sc, st, st, stream_);
     tally(bf16_bytes);
   } else {
     launch::spmv(n, rows, cols, vals, p, q, st, stream_);
     tally(spmv_bytes);
     reduce_into(ReduceMode::Dot2, n, spd ? p : q, q, t, spd ? p : q, sc, 0, st);
+    launch::inner_alpha(sc, st, parent, 0, stream_);
   }
-  launch::inner_alpha(sc, st, parent, 0, stream_);
   launch::inner_step(n, l.x, p, sc, st, stream_);
   tally(12.0 * n);
 }

@@ -264,6 +264,8 @@ class Solver {
   void cycle(std::size_t index, const float* b, float*& x, const int* status,
              bool swept = false);
   void inner(std::size_t index, const int* parent);
+  // The K-cycle level whose next post-smoothing ends in z.q and beta.
+  const DevLevel* inner_dot_ = nullptr;
   void smooth(DevLevel& l, const int* rows, const int* cols, const float* vals, const float* b,
               float*& x, int sweeps, bool zero_start, const int* status, bool swept = false,
               const float* coarse = nullptr);
