@@ -947,17 +947,18 @@ long long b2_coupled_copy(const b2_coupled* s, int what, float* out, void* strea
       count = static_cast<long long>(27 * n);
       if (!out) return;
       read_back(out, c.cell_data(), 20 * n, st);
-      std::vector<float> inv(4 * n), inv_h(4 * n);
-      c.copy_inverse(inv.data(), inv_h.data(), st);
+      // The block inverse as the sweep forms it, in the same float operations.
+      std::vector<float> diag(4 * n), coupling(4 * n), yz(2 * n), schur(n);
+      c.copy_inverse(diag.data(), coupling.data(), yz.data(), schur.data(), st);
       kb2::wait(st);
       for (std::size_t i = 0; i < n; ++i) {
-        out[20 * n + i] = inv[4 * i];
-        out[21 * n + i] = inv[4 * i + 1];
-        out[22 * n + i] = inv[4 * i + 2];
-        out[23 * n + i] = inv_h[4 * i];
-        out[24 * n + i] = inv_h[4 * i + 1];
-        out[25 * n + i] = inv_h[4 * i + 2];
-        out[26 * n + i] = inv[4 * i + 3];
+        const float h[3] = {coupling[4 * i + 3], yz[2 * i], yz[2 * i + 1]};
+        for (std::size_t k = 0; k < 3; ++k) {
+          const float inverse = 1.0f / diag[4 * i + k];
+          out[(20 + k) * n + i] = inverse;
+          out[(23 + k) * n + i] = h[k] * inverse;
+        }
+        out[26 * n + i] = schur[i];
       }
     } else if (what == 3) {
       count = c.faces();

@@ -16,9 +16,8 @@
 //   fine Galerkin reads them;
 // - the fine operator used every iteration is repacked once per solve into
 //   per-cell records, 16-byte aligned: (du, dv, dw, cd), (wc Gx, wc Gy, wc Gz,
-//   wc Hx), (wc Hy, wc Hz), the block inverse (iu, iv, iw, schur) and
-//   (Hx iu, Hy iv, Hz iw, 0) with Hx = wc Hx, and ELL slots in slot-major
-//   order for the internal faces of each cell in cell-face order: (a, gx, gy,
+//   wc Hx), (wc Hy, wc Hz) and the block inverse's Schur denominator, and ELL
+//   slots in slot-major order for the internal faces of each cell in cell-face order: (a, gx, gy,
 //   gz), h and (neighbour, face) per slot, plus one (sx, sy, sz, rc) record
 //   per face. A warp's slot loads are then contiguous 512-byte lines;
 // - coarse levels (coupled_coarse.cu) keep the reference's CSR pattern with one
@@ -26,11 +25,13 @@
 //   n per row (du dv dw cs iu iv iw hx iu hy iv hz iw schur).
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 
 #include "common.cuh"
 #include "coupled_kernels.hpp"
 #include "coupled_rows.cuh"
+#include "epilogues.cuh"
 
 namespace kb2 {
 namespace {
@@ -225,8 +226,7 @@ __global__ void k_cpl_fine_pack(int n, int width, FineGeometry m, const float* _
     op.diag[i] = make_float4(du, dv, dw, cd);
     op.coupling[i] = make_float4(ex, ey, ez, hx);
     op.coupling_yz[i] = make_float2(hy, hz);
-    op.inverse[i] = make_float4(inv.iu, inv.iv, inv.iw, inv.schur);
-    op.inverse_h[i] = make_float4(inv.hu, inv.hv, inv.hw, 0.0f);
+    op.schur[i] = inv.schur;
     const float q00 = wc * cell[10 * N + i], q01 = wc * cell[11 * N + i], q02 = wc * cell[12 * N + i];
     const float q10 = wc * cell[13 * N + i], q11 = wc * cell[14 * N + i], q12 = wc * cell[15 * N + i];
     const float q20 = wc * cell[16 * N + i], q21 = wc * cell[17 * N + i], q22 = wc * cell[18 * N + i];
@@ -293,6 +293,35 @@ __global__ void __launch_bounds__(kBlock, 8) k_cpl_fine_spmv(int n, int width, C
     y[i] = fine_row(i, n, width, op, x);
 }
 
+// y = J x with the BiCGStab's reduction of y fused in: w.y and alpha, or (kDual)
+// y.y, y.w and omega. The FP64 sums need more than 32 registers, so the grid is
+// sized for six blocks per SM (still one wave).
+constexpr int kDotBlocks = 6;
+template <bool kDual>
+__global__ void __launch_bounds__(kBlock, kDotBlocks)
+    k_cpl_fine_spmv_dot(int n, int width, CoupledFine op, const float4* __restrict__ x,
+                        const float4* __restrict__ w, float4* __restrict__ y, DeviceReducer red,
+                        float* scalars, int* status) {
+  pdl_entry();
+  if (status[0] != 0) return;
+  double a = 0.0, b = 0.0;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const float4 v = fine_row(i, n, width, op, x), u = w[i];
+    y[i] = v;
+    const double dot = static_cast<double>(u.x) * v.x + static_cast<double>(u.y) * v.y +
+                       static_cast<double>(u.z) * v.z + static_cast<double>(u.w) * v.w;
+    if (kDual) {
+      a += static_cast<double>(v.x) * v.x + static_cast<double>(v.y) * v.y +
+           static_cast<double>(v.z) * v.z + static_cast<double>(v.w) * v.w;
+      b += dot;
+    } else {
+      a += dot;
+    }
+  }
+  finish(as_reducer(red), a, b, kDual, scalars, 2, status,
+         kDual ? Epilogue::BicgOmega : Epilogue::BicgAlpha);
+}
+
 __global__ void __launch_bounds__(kBlock, 8) k_cpl_fine_residual(int n, int width, CoupledFine op,
                                                               const float4* __restrict__ x,
                                                               const float4* __restrict__ b,
@@ -321,8 +350,15 @@ __global__ void __launch_bounds__(kBlock, 8) k_cpl_fine_smooth(int n, int width,
       r = make_float4(r.x - y.x, r.y - y.y, r.z - y.z, r.w - y.w);
       base = x[i];
     }
-    const float4 e = op.coupling[i], iv = op.inverse[i], ih = op.inverse_h[i];
-    const float4 d = block_solve(r, e.x, e.y, e.z, iv.x, iv.y, iv.z, ih.x, ih.y, ih.z, iv.w);
+    // The block inverse's factors again from the diagonal (block_prepare's
+    // operations): three reciprocals per cell instead of 28 bytes. The records
+    // are read again (from L1) rather than held in registers over the row.
+    asm volatile("" ::: "memory");
+    const float4 m = op.diag[i], e = op.coupling[i];
+    const float2 h = op.coupling_yz[i];
+    const float iu = 1.0f / m.x, iv = 1.0f / m.y, iw = 1.0f / m.z;
+    const float4 d = block_solve(r, e.x, e.y, e.z, iu, iv, iw, e.w * iu, h.x * iv, h.y * iw,
+                                 op.schur[i]);
     next[i] = damped(base, d, omega);
   }
 }
@@ -472,6 +508,19 @@ void cpl_fine_spmv(int n, const CoupledFine& op, int width, const float4* x, flo
   if (n <= 0) return;
   ++counter;
   pdl(k_cpl_fine_spmv, grid_for(n), kBlock, 0, s, n, width, op, x, y);
+}
+
+void cpl_fine_spmv_dot(int n, const CoupledFine& op, int width, const float4* x, const float4* w,
+                       float4* y, bool dual, DeviceReducer red, float* scalars, int* status,
+                       cudaStream_t s) {
+  if (n <= 0) return;
+  ++counter;
+  const int grid = std::min(grid_for(n), kSms * kDotBlocks);
+  if (dual)
+    pdl(k_cpl_fine_spmv_dot<true>, grid, kBlock, 0, s, n, width, op, x, w, y, red, scalars, status);
+  else
+    pdl(k_cpl_fine_spmv_dot<false>, grid, kBlock, 0, s, n, width, op, x, w, y, red, scalars,
+        status);
 }
 
 void cpl_fine_residual(int n, const CoupledFine& op, int width, const float4* x, const float4* b,

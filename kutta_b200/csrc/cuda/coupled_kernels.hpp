@@ -42,8 +42,7 @@ struct CoupledFine {
   float4* diag;         // (du, dv, dw, cd)
   float4* coupling;     // (wc Gx, wc Gy, wc Gz, wc Hx)
   float2* coupling_yz;  // (wc Hy, wc Hz)
-  float4* inverse;      // (iu, iv, iw, schur)
-  float4* inverse_h;    // (Hx iu, Hy iv, Hz iw, 0)
+  float* schur;         // the block inverse's Schur denominator
   float4* edge;         // per slot: (a, gx, gy, gz)
   float* edge_h;        // per slot: h
   int2* link;           // per slot: (neighbour, face), neighbour -1 past the row's end
@@ -120,6 +119,11 @@ void cpl_coarse_prepare(const CoupledLevel& l, float* scratch, cudaStream_t s);
 
 void cpl_fine_spmv(int n, const CoupledFine& op, int width, const float4* x, float4* y,
                    cudaStream_t s);
+// y = J x, then w.y -> scalars[2] and solver_bicg_alpha, or (dual) y.y, y.w ->
+// scalars[2], scalars[4] and solver_bicg_omega; skipped while status[0] != 0.
+void cpl_fine_spmv_dot(int n, const CoupledFine& op, int width, const float4* x, const float4* w,
+                       float4* y, bool dual, DeviceReducer red, float* scalars, int* status,
+                       cudaStream_t s);
 void cpl_fine_residual(int n, const CoupledFine& op, int width, const float4* x, const float4* b,
                        float4* r, cudaStream_t s);
 void cpl_fine_smooth(int n, const CoupledFine& op, int width, const float4* x, const float4* b,

@@ -9,6 +9,7 @@
 #include <cuda_bf16.h>
 
 #include "common.cuh"
+#include "epilogues.cuh"
 #include "kernels.hpp"
 
 #include <algorithm>
@@ -30,114 +31,6 @@ using namespace dev;
 
 #define ROWS(i, n) \
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < (n); i += gridDim.x * blockDim.x)
-
-__device__ __forceinline__ Reducer as_reducer(DeviceReducer r) { return Reducer{r.partials, r.ticket}; }
-
-// ---- scalar updates, src/kutta/kernels/scalars.kern.h:51-121 -----------------
-__device__ void epilogue(Epilogue e, float* sc, int* st) {
-  switch (e) {
-    case Epilogue::None:
-      return;
-    case Epilogue::PcgAlpha: {  // solver_pcg_alpha :63-71
-      if (st[0] != 0) return;
-      const Pair rho = kp_load(sc, 0), pq = kp_load(sc, 2);
-      const Pair alpha = kp_div(rho, pq);
-      if (!kp_positive(rho) || !kp_positive(pq) || !kp_coefficient(alpha) || kp_zero(alpha))
-        st[0] = 2;
-      else
-        kp_store(sc, 8, alpha);
-      return;
-    }
-    case Epilogue::PcgBeta:
-    case Epilogue::PcgBetaFlexible: {  // solver_pcg_beta :72-80
-      if (st[0] != 0) return;
-      const Pair next = kp_load(sc, 4);
-      const Pair numer = e == Epilogue::PcgBetaFlexible
-                             ? kp_neg(kp_mul(kp_load(sc, 8), kp_load(sc, 6)))
-                             : next;
-      const Pair beta = kp_div(numer, kp_load(sc, 0));
-      if (!kp_positive(next) || !kp_coefficient(beta) || (kp_zero(beta) && !kp_zero(numer)))
-        st[0] = 2;
-      else {
-        kp_store(sc, 10, beta);
-        kp_store(sc, 0, next);
-      }
-      return;
-    }
-    case Epilogue::BicgBeta: {  // solver_bicg_beta :81-89
-      if (st[0] != 0) return;
-      const Pair rho = kp_load(sc, 0), omega = kp_load(sc, 12);
-      const Pair beta = kp_mul(kp_div(rho, kp_load(sc, 14)), kp_div(kp_load(sc, 8), omega));
-      if (kp_zero(rho) || !kp_finite(rho) || kp_zero(omega) || !kp_coefficient(omega) ||
-          !kp_coefficient(beta) || kp_zero(beta))
-        st[0] = 2;
-      else {
-        kp_store(sc, 10, beta);
-        st[2] = 0;
-      }
-      return;
-    }
-    case Epilogue::BicgAlpha: {  // solver_bicg_alpha :90-97
-      if (st[0] != 0) return;
-      const Pair rv = kp_load(sc, 2);
-      const Pair alpha = kp_div(kp_load(sc, 0), rv);
-      if (kp_zero(rv) || !kp_finite(rv) || !kp_coefficient(alpha) || kp_zero(alpha))
-        st[0] = 2;
-      else
-        kp_store(sc, 8, alpha);
-      return;
-    }
-    case Epilogue::BicgS: {  // solver_bicg_s :98-103
-      if (st[0] != 0) return;
-      ++st[1];
-      st[2] = kp_le(kp_load(sc, 16), kp_load(sc, 20)) ? 1 : 0;
-      return;
-    }
-    case Epilogue::BicgOmega: {  // solver_bicg_omega :104-112
-      if (st[0] != 0) return;
-      if (st[2] != 0) {
-        kp_store(sc, 12, kp(0.0f, 0.0f));
-        return;
-      }
-      const Pair tt = kp_load(sc, 2), ts = kp_load(sc, 4);
-      const Pair omega = kp_div(ts, tt);
-      if (!kp_positive(tt) || !kp_finite(tt) || kp_zero(omega) || !kp_coefficient(omega))
-        st[0] = 2;
-      else
-        kp_store(sc, 12, omega);
-      return;
-    }
-    case Epilogue::CheckPcg:
-    case Epilogue::CheckBicg: {  // solver_check :113-121
-      if (st[0] != 0) return;
-      const bool pcg = e == Epilogue::CheckPcg;
-      if (pcg) ++st[1];
-      const Pair rr = kp_load(sc, 18);
-      if (!kp_finite(rr) || kp_le(rr, kp_load(sc, 20)) || !kp_le(rr, kp_load(sc, 22)) ||
-          st[1] % 50 == 0)
-        st[0] = 1;
-      if (!pcg) kp_store(sc, 14, kp_load(sc, 0));
-      return;
-    }
-  }
-}
-
-// Block partial -> grid total -> pair store -> epilogue, in the last block.
-__device__ __forceinline__ void finish(const Reducer& red, double a, double b, bool dual,
-                                       float* scalars, int offset, int* status, Epilogue epi) {
-  __shared__ double shared[32];
-  a = block_sum(a, shared);
-  if (dual) b = block_sum(b, shared);
-  if (!publish(red, a, b, dual)) return;
-  const double total_a = gather(red, 0, shared);
-  const double total_b = dual ? gather(red, 1, shared) : 0.0;
-  if (threadIdx.x == 0) {
-    store_pair(scalars, offset, total_a);
-    if (dual) store_pair(scalars, offset + 2, total_b);
-    epilogue(epi, scalars, status);
-    *red.ticket = 0;
-  }
-}
 
 // ---- CSR row kernels --------------------------------------------------------
 // One row per thread: on the 5-entry fine rows this direct form measured
@@ -175,6 +68,25 @@ __global__ void k_spmv_dot(int n, const int* __restrict__ rows, const int* __res
     acc += static_cast<double>(w[i]) * static_cast<double>(sum);
   }
   finish(as_reducer(red), acc, 0, false, scalars, offset, status, epi);
+}
+
+// csr_spmv_guarded + dot2_into(t, t; t, s) + solver_bicg_omega (solver.cpp:343-347).
+__global__ void k_spmv_dot2(int n, const int* __restrict__ rows, const int* __restrict__ cols,
+                            const float* __restrict__ vals, const float* __restrict__ x,
+                            const float* __restrict__ sv, float* __restrict__ t, DeviceReducer red,
+                            float* scalars, int* status) {
+  pdl_entry();
+  if (status[0] != 0) return;
+  double tt = 0, ts = 0;
+  ROWS(i, n) {
+    float sum = 0.0f, error = 0.0f;
+    const int end = rows[i + 1];
+    for (int j = rows[i]; j < end; ++j) kahan_term(sum, error, vals[j], x[cols[j]]);
+    t[i] = sum;
+    tt += static_cast<double>(sum) * static_cast<double>(sum);
+    ts += static_cast<double>(sum) * static_cast<double>(sv[i]);
+  }
+  finish(as_reducer(red), tt, ts, true, scalars, 2, status, Epilogue::BicgOmega);
 }
 
 // csr_residual / csr_residual_guarded, linalg.kern.h:32-50,115-118.
@@ -566,9 +478,14 @@ __global__ void k_level_rows(int n, const int* __restrict__ rows, const int* __r
 }
 
 // ---- Krylov vector updates, scalars.kern.h:122-152 ---------------------------
-// solver_step :122-127 + dot_into(r, r -> 18) + solver_check(pcg) (solver.cpp:291-293).
+// solver_step :122-127 + dot_into(r, r -> 18) + solver_check(pcg) (solver.cpp:291-293);
+// with next != null also the fine level's zero-start sweep of the new r, which
+// the AMG cycle begins with (it reads r and writes the sweep: 4 of its 12 bytes a
+// row and a launch less).
 __global__ void k_pcg_step_dot(int n, float* __restrict__ x, float* __restrict__ r,
                                const float* __restrict__ p, const float* __restrict__ q,
+                               const int* __restrict__ rows, const float* __restrict__ vals,
+                               const float* __restrict__ inv, float* __restrict__ next,
                                DeviceReducer red, float* scalars, int* status) {
   pdl_entry();
   if (status[0] != 0) return;
@@ -578,6 +495,7 @@ __global__ void k_pcg_step_dot(int n, float* __restrict__ x, float* __restrict__
     x[i] += alpha * p[i];
     const float ri = r[i] - alpha * q[i];
     r[i] = ri;
+    if (next != nullptr) next[i] = zero_sweep_row(i, rows, vals, ri, inv[i]);
     acc += static_cast<double>(ri) * static_cast<double>(ri);
   }
   finish(as_reducer(red), acc, 0, false, scalars, 18, status, Epilogue::CheckPcg);
@@ -602,34 +520,48 @@ __global__ void k_bicg_direction(int n, const float* __restrict__ r, const float
   ROWS(i, n) p[i] = r[i] + beta * (p[i] - omega * v[i]);
 }
 
-// solver_bicg_difference :138-141.
+// solver_bicg_difference :138-141 + dot_into(s, s -> 16) + solver_bicg_s.
 __global__ void k_bicg_difference(int n, const float* __restrict__ r, const float* __restrict__ q,
-                                  float* __restrict__ sv, const float* __restrict__ scalars,
-                                  const int* __restrict__ status) {
+                                  float* __restrict__ sv, DeviceReducer red, float* scalars,
+                                  int* status) {
   pdl_entry();
   if (status[0] != 0) return;
   const float alpha = kp_float(kp_load(scalars, 8));
-  ROWS(i, n) sv[i] = r[i] - alpha * q[i];
+  double acc = 0;
+  ROWS(i, n) {
+    const float si = r[i] - alpha * q[i];
+    sv[i] = si;
+    acc += static_cast<double>(si) * static_cast<double>(si);
+  }
+  finish(as_reducer(red), acc, 0, false, scalars, 16, status, Epilogue::BicgS);
 }
 
-// solver_bicg_step :142-149.
+// solver_bicg_step :142-149 + dot_into(r, r -> 18) + solver_check, and the next
+// update's dot_into(rhat, r -> 0) + solver_bicg_beta.
 __global__ void k_bicg_step(int n, float* __restrict__ x, float* __restrict__ r,
                             const float* __restrict__ z, const float* __restrict__ zs,
                             const float* __restrict__ sv, const float* __restrict__ t,
-                            const float* __restrict__ scalars, const int* __restrict__ status) {
+                            const float* __restrict__ shadow, DeviceReducer red, float* scalars,
+                            int* status) {
   pdl_entry();
   if (status[0] != 0) return;
   const float alpha = kp_float(kp_load(scalars, 8)), omega = kp_float(kp_load(scalars, 12));
   const bool s_only = status[2] != 0;
+  double rr = 0, rho = 0;
   ROWS(i, n) {
+    float ri;
     if (s_only) {
       x[i] += alpha * z[i];
-      r[i] = sv[i];
+      ri = sv[i];
     } else {
       x[i] += alpha * z[i] + omega * zs[i];
-      r[i] = sv[i] - omega * t[i];
+      ri = sv[i] - omega * t[i];
     }
+    r[i] = ri;
+    rr += static_cast<double>(ri) * static_cast<double>(ri);
+    rho += static_cast<double>(shadow[i]) * static_cast<double>(ri);
   }
+  finish_bicg(as_reducer(red), rr, rho, scalars, status);
 }
 
 // krylov_multiply(_guarded), linalg.kern.h:72-75,119-122.
@@ -803,6 +735,12 @@ void spmv_dot(int n, const int* rows, const int* cols, const float* vals, const 
   pdl(k_spmv_dot, blocks(n), kBlock, 0, s, n, rows, cols, vals, p, w, q, red, scalars, offset,
                                           status, epi);
 }
+void spmv_dot2(int n, const int* rows, const int* cols, const float* vals, const float* x,
+               const float* sv, float* t, DeviceReducer red, float* scalars, int* status,
+               cudaStream_t s) {
+  ++counter;
+  pdl(k_spmv_dot2, blocks(n), kBlock, 0, s, n, rows, cols, vals, x, sv, t, red, scalars, status);
+}
 void residual(int n, const int* rows, const int* cols, const float* vals, const float* x,
               const float* b, float* r, const int* status, cudaStream_t s) {
   if (n <= 0) return;
@@ -911,10 +849,12 @@ void level_rows(int n, const int* rows, const int* diag, float* vals, const Leve
     pdl(k_level_rows<false>, blocks(n), kBlock, 0, s, n, rows, diag, vals, p.offsets, p.members,
         p.fine_surplus, p.inverse, p.surplus, p.v16, p.scale, red, check, slot);
 }
-void pcg_step_dot(int n, float* x, float* r, const float* p, const float* q, DeviceReducer red,
+void pcg_step_dot(int n, float* x, float* r, const float* p, const float* q, const int* rows,
+                  const float* vals, const float* inv, float* next, DeviceReducer red,
                   float* scalars, int* status, cudaStream_t s) {
   ++counter;
-  pdl(k_pcg_step_dot, blocks(n), kBlock, 0, s, n, x, r, p, q, red, scalars, status);
+  pdl(k_pcg_step_dot, blocks(n), kBlock, 0, s, n, x, r, p, q, rows, vals, inv, next, red, scalars,
+      status);
 }
 void direction(int n, const float* z, float* p, const float* scalars, const int* status,
                cudaStream_t s) {
@@ -928,17 +868,16 @@ void bicg_direction(int n, const float* r, const float* v, float* p, const float
   ++counter;
   pdl(k_bicg_direction, blocks(n), kBlock, 0, s, n, r, v, p, scalars, status);
 }
-void bicg_difference(int n, const float* r, const float* q, float* sv, const float* scalars,
-                     const int* status, cudaStream_t s) {
-  if (n <= 0) return;
+void bicg_difference(int n, const float* r, const float* q, float* sv, DeviceReducer red,
+                     float* scalars, int* status, cudaStream_t s) {
   ++counter;
-  pdl(k_bicg_difference, blocks(n), kBlock, 0, s, n, r, q, sv, scalars, status);
+  pdl(k_bicg_difference, blocks(n), kBlock, 0, s, n, r, q, sv, red, scalars, status);
 }
 void bicg_step(int n, float* x, float* r, const float* z, const float* zs, const float* sv,
-               const float* t, const float* scalars, const int* status, cudaStream_t s) {
-  if (n <= 0) return;
+               const float* t, const float* shadow, DeviceReducer red, float* scalars, int* status,
+               cudaStream_t s) {
   ++counter;
-  pdl(k_bicg_step, blocks(n), kBlock, 0, s, n, x, r, z, zs, sv, t, scalars, status);
+  pdl(k_bicg_step, blocks(n), kBlock, 0, s, n, x, r, z, zs, sv, t, shadow, red, scalars, status);
 }
 void multiply(int n, const float* r, const float* inverse, float* z, const int* status,
               cudaStream_t s) {

@@ -49,6 +49,10 @@ void spmv(int n, const int* rows, const int* cols, const float* vals, const floa
 void spmv_dot(int n, const int* rows, const int* cols, const float* vals, const float* p,
               const float* w, float* q, DeviceReducer red, float* scalars, int offset,
               int* status, Epilogue epi, cudaStream_t s);
+// t = A x, t.t and t.sv -> scalars[2], scalars[4] and solver_bicg_omega.
+void spmv_dot2(int n, const int* rows, const int* cols, const float* vals, const float* x,
+               const float* sv, float* t, DeviceReducer red, float* scalars, int* status,
+               cudaStream_t s);
 // The mixed solve's packed copy of the fine operator ("packed rows"): per
 // row i the diagonal value diag[i] and `width` (4 or 8) off-diagonal slots,
 // values vals[width i + k] and int16 column offsets offsets[width i + k] =
@@ -170,16 +174,23 @@ void plain_tail(const PlainTail& t, const float* fine, float* out, const int* st
 
 // ---- Krylov vector updates (guarded by status) ----------------------------
 // x += a p; r -= a q; then r.r -> scalars[18] and solver_check(pcg = 1).
-void pcg_step_dot(int n, float* x, float* r, const float* p, const float* q, DeviceReducer red,
+// With next != null also the zero-start sweep of the new r (rows, vals and inv of
+// the fine level) into next.
+void pcg_step_dot(int n, float* x, float* r, const float* p, const float* q, const int* rows,
+                  const float* vals, const float* inv, float* next, DeviceReducer red,
                   float* scalars, int* status, cudaStream_t s);
 void direction(int n, const float* z, float* p, const float* scalars, const int* status,
                cudaStream_t s);
 void bicg_direction(int n, const float* r, const float* v, float* p, const float* scalars,
                     const int* status, cudaStream_t s);
-void bicg_difference(int n, const float* r, const float* q, float* sv, const float* scalars,
-                     const int* status, cudaStream_t s);
+// sv = r - alpha q, s.s -> scalars[16] and solver_bicg_s.
+void bicg_difference(int n, const float* r, const float* q, float* sv, DeviceReducer red,
+                     float* scalars, int* status, cudaStream_t s);
+// The x and r update, r.r -> scalars[18] and solver_check; then, while the
+// iteration runs, shadow.r -> scalars[0] and the next update's solver_bicg_beta.
 void bicg_step(int n, float* x, float* r, const float* z, const float* zs, const float* sv,
-               const float* t, const float* scalars, const int* status, cudaStream_t s);
+               const float* t, const float* shadow, DeviceReducer red, float* scalars, int* status,
+               cudaStream_t s);
 void multiply(int n, const float* r, const float* inverse, float* z, const int* status,
               cudaStream_t s);
 void axpy(int n, float* y, const float* x, float a, cudaStream_t s);

@@ -72,8 +72,7 @@ CoupledSolver::CoupledSolver(const CoupledMeshHost& m, int reference,
   own(diag_, n);
   own(coupling_, n);
   own(coupling_yz_, n);
-  own(inverse_, n);
-  own(inverse_h_, n);
+  own(schur_, n);
   const std::size_t slots = static_cast<std::size_t>(width_) * n;
   own(edge_, slots);
   own(edge_h_, slots);
@@ -222,9 +221,8 @@ void CoupledSolver::iteration(Body body) {
 }
 
 CoupledFine CoupledSolver::fine() const {
-  return CoupledFine{diag_.get(),   coupling_.get(), coupling_yz_.get(), inverse_.get(),
-                     inverse_h_.get(), edge_.get(), edge_h_.get(),      link_.get(),
-                     face_.get()};
+  return CoupledFine{diag_.get(), coupling_.get(), coupling_yz_.get(), schur_.get(),
+                     edge_.get(), edge_h_.get(),   link_.get(),        face_.get()};
 }
 
 void CoupledSolver::capture_diagonal(int component, const int* rows, const int* diag,
@@ -415,30 +413,26 @@ Stats CoupledSolver::bicgstab(const Control& c) {
                "copy");
     launch::fill(n4, F(p_), 0.0f, stream_);
     launch::fill(n4, F(q_), 0.0f, stream_);
+    // Every later update's beta rides on the step before it.
+    launch::reduce_into(ReduceMode::Dot, n4, F(shadow_), F(r_), F(shadow_), F(r_), red, sc, 0, st,
+                        true, Epilogue::BicgBeta, stream_);
   };
   restart();
   int restarts = 0;
   Pinned<int>& state = host_status_;
   while (stats.iterations < c.max_iter) {
     iteration([&] {
-      launch::reduce_into(ReduceMode::Dot, n4, F(shadow_), F(r_), F(shadow_), F(r_), red, sc, 0, st,
-                          true, Epilogue::BicgBeta, stream_);
       launch::bicg_direction(n4, F(r_), F(q_), F(p_), sc, st, stream_);
       precondition(p_.get(), z_);
-      launch::cpl_fine_spmv(n_, fine(), width_, z_, q_.get(), stream_);
-      launch::reduce_into(ReduceMode::Dot, n4, F(shadow_), F(q_), F(shadow_), F(q_), red, sc, 2, st,
-                          true, Epilogue::BicgAlpha, stream_);
-      launch::bicg_difference(n4, F(r_), F(q_), F(sv_), sc, st, stream_);
-      launch::reduce_into(ReduceMode::Dot, n4, F(sv_), F(sv_), F(sv_), F(sv_), red, sc, 16, st, true,
-                          Epilogue::BicgS, stream_);
+      launch::cpl_fine_spmv_dot(n_, fine(), width_, z_, shadow_.get(), q_.get(), false, red, sc, st,
+                                stream_);
+      launch::bicg_difference(n4, F(r_), F(q_), F(sv_), red, sc, st, stream_);
       precondition(sv_.get(), zs_);
-      launch::cpl_fine_spmv(n_, fine(), width_, zs_, t_.get(), stream_);
-      launch::reduce_into(ReduceMode::Dot2, n4, F(t_), F(t_), F(t_), F(sv_), red, sc, 2, st, true,
-                          Epilogue::BicgOmega, stream_);
+      launch::cpl_fine_spmv_dot(n_, fine(), width_, zs_, sv_.get(), t_.get(), true, red, sc, st,
+                                stream_);
       launch::bicg_step(n4, reinterpret_cast<float*>(x_), F(r_), reinterpret_cast<float*>(z_),
-                        reinterpret_cast<float*>(zs_), F(sv_), F(t_), sc, st, stream_);
-      launch::reduce_into(ReduceMode::Dot, n4, F(r_), F(r_), F(r_), F(r_), red, sc, 18, st, true,
-                          Epilogue::CheckBicg, stream_);
+                        reinterpret_cast<float*>(zs_), F(sv_), F(t_), F(shadow_), red, sc, st,
+                        stream_);
     });
     cuda_check(cudaMemcpyAsync(state.get(), st, 3 * sizeof(int), cudaMemcpyDeviceToHost, stream_),
                "status readback");
@@ -554,11 +548,16 @@ void CoupledSolver::level_apply(int k, int op, const float* x, const float* b, f
   }
 }
 
-void CoupledSolver::copy_inverse(float* inverse, float* inverse_h, cudaStream_t s) const {
-  const std::size_t bytes = static_cast<std::size_t>(n_) * sizeof(float4);
-  cuda_check(cudaMemcpyAsync(inverse, inverse_.get(), bytes, cudaMemcpyDeviceToHost, s), "copy");
-  cuda_check(cudaMemcpyAsync(inverse_h, inverse_h_.get(), bytes, cudaMemcpyDeviceToHost, s),
-             "copy");
+void CoupledSolver::copy_inverse(float* diag, float* coupling, float* coupling_yz, float* schur,
+                                 cudaStream_t s) const {
+  const std::size_t n = n_;
+  const auto copy = [&](float* to, const void* from, std::size_t bytes) {
+    cuda_check(cudaMemcpyAsync(to, from, bytes, cudaMemcpyDeviceToHost, s), "copy");
+  };
+  copy(diag, diag_.get(), n * sizeof(float4));
+  copy(coupling, coupling_.get(), n * sizeof(float4));
+  copy(coupling_yz, coupling_yz_.get(), n * sizeof(float2));
+  copy(schur, schur_.get(), n * sizeof(float));
 }
 
 std::string CoupledSolver::describe() const {

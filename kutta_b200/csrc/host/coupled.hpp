@@ -47,9 +47,11 @@ class CoupledSolver {
   std::string describe() const;
   int cells() const { return n_; }
   int faces() const { return mesh_.n_faces; }
-  // The fine block inverse as two float4 per cell: (iu, iv, iw, schur) and
-  // (Hx iu, Hy iv, Hz iw, 0); asynchronous copies to host memory on `s`.
-  void copy_inverse(float* inverse, float* inverse_h, cudaStream_t s) const;
+  // What the fine block inverse is made of, per cell: (du, dv, dw, cd), (wc G,
+  // wc Hx), (wc Hy, wc Hz) and the Schur denominator; asynchronous copies to host
+  // memory on `s`.
+  void copy_inverse(float* diag, float* coupling, float* coupling_yz, float* schur,
+                    cudaStream_t s) const;
   int levels() const { return static_cast<int>(levels_.size()) + 1; }
   int level_rows(int k) const { return k == 0 ? n_ : levels_[k - 1].op.n; }
   // The last solution (float4 per cell, (du, dv, dw, dp~)), the right-hand
@@ -131,9 +133,9 @@ class CoupledSolver {
   DArray<int> owner_, neighbour_, offsets_, faces_, adjacent_, kind_;
   DArray<float> sign_, sx_, sy_, sz_, dx_, dy_, dz_, diffusion_, volume_;
   DArray<float> cell_, coefficient_, scratch_;
-  DArray<float4> diag_, coupling_, inverse_, inverse_h_, edge_, face_;
+  DArray<float4> diag_, coupling_, edge_, face_;
   DArray<float2> coupling_yz_;
-  DArray<float> edge_h_;
+  DArray<float> edge_h_, schur_;
   DArray<int2> link_;
   std::vector<Level> levels_;
   std::vector<Transfer> transfers_;

@@ -712,7 +712,7 @@ void Solver::inner(std::size_t index, const int* parent) {
 // (solver.cpp:65-68) preconditioner.
 void Solver::apply(const float* r, float*& z) {
   if (amg() && graphing()) {
-    graphed(r, z, fuse_dots_ ? 1 : 0, z, [&] { precondition(r, z); });
+    graphed(r, z, (fuse_dots_ ? 1 : 0) + (swept_ ? 2 : 0), z, [&] { precondition(r, z); });
   } else if (amg()) {
     precondition(r, z);
   } else {
@@ -728,7 +728,9 @@ void Solver::apply(const float* r, float*& z) {
 // preconditioner, so the Krylov driver must be the flexible one, as it is for
 // the mixed solve.
 void Solver::precondition(const float* r, float*& z) {
-  cycle(0, r, z, status_.get());
+  // The update before has left the first sweep in the fine level's spare buffer.
+  if (swept_) std::swap(z, levels_[0].r);
+  cycle(0, r, z, status_.get(), swept_);
   if (learned_ != nullptr && (learned_mode_ & kLearnedCycle)) {
     float* t = learned_residual_.get();
     launch::residual(n_, rows0(), cols0(), val_, z, r, t, status_.get(), stream_);
@@ -1048,13 +1050,19 @@ void Solver::pcg(float* x, const float* b, const Control& c, double target, Stat
       else
         launch::spmv_dot(n_, rows0(), cols0(), val_, p_, p_, q_, reducer(), scalars_.get(), 2,
                          status_.get(), Epilogue::PcgAlpha, stream_);
-      launch::pcg_step_dot(n_, x, r_, p_, q_, reducer(), scalars_.get(), status_.get(), stream_);
-      tally(fine_operator_bytes() + 8.0 * n_ + 24.0 * n_);
-      if (stats.iterations + j + 1 == c.max_iter) return;
+      const bool last = stats.iterations + j + 1 == c.max_iter;
+      const bool sweep = amg() && levels_.size() > 1 && !last;
+      auto& fine = levels_[0];
+      launch::pcg_step_dot(n_, x, r_, p_, q_, rows0(), val_, fine.l1.get(),
+                           sweep ? fine.r : nullptr, reducer(), scalars_.get(), status_.get(),
+                           stream_);
+      tally(fine_operator_bytes() + 8.0 * n_ + (sweep ? 32.0 : 24.0) * n_);
+      if (last) return;
       const bool fused = can_fuse_dots();
       fuse_dots_ = fused;
+      swept_ = sweep;
       apply(r_, z_);
-      fuse_dots_ = false;
+      fuse_dots_ = swept_ = false;
       tally((variable() ? (fused ? 4.0 : 12.0) : 8.0) * n_ + 12.0 * n_);
       if (variable()) {
         if (!fused)
@@ -1095,6 +1103,9 @@ void Solver::bicgstab(float* x, const float* b, const Control& c, double target,
     copy(shadow_, r_, n_);
     launch::fill(n_, p_, 0.0f, stream_);
     launch::fill(n_, q_, 0.0f, stream_);
+    // Every later update's beta rides on the step before it.
+    launch::reduce_into(ReduceMode::Dot, n_, shadow_, r_, shadow_, r_, reducer(), scalars_.get(),
+                        0, status_.get(), true, Epilogue::BicgBeta, stream_);
   };
   restart();
   int restarts = 0;
@@ -1107,23 +1118,17 @@ void Solver::bicgstab(float* x, const float* b, const Control& c, double target,
     speculated_.reset();
     for (int j = 0; j < batch; ++j) {
       (void)j;
-      launch::reduce_into(ReduceMode::Dot, n_, shadow_, r_, shadow_, r_, reducer(), sc, 0,
-                          status_.get(), true, Epilogue::BicgBeta, stream_);
       launch::bicg_direction(n_, r_, q_, p_, sc, status_.get(), stream_);
       apply(p_, z_);
       launch::spmv_dot(n_, rows0(), cols0(), val_, z_, shadow_, q_, reducer(), sc, 2,
                        status_.get(), Epilogue::BicgAlpha, stream_);
-      launch::bicg_difference(n_, r_, q_, s_, sc, status_.get(), stream_);
-      launch::reduce_into(ReduceMode::Dot, n_, s_, s_, s_, s_, reducer(), sc, 16, status_.get(),
-                          true, Epilogue::BicgS, stream_);
+      launch::bicg_difference(n_, r_, q_, s_, reducer(), sc, status_.get(), stream_);
       apply(s_, zs_);
-      launch::spmv(n_, rows0(), cols0(), val_, zs_, t_, status_.get(), stream_);
-      launch::reduce_into(ReduceMode::Dot2, n_, t_, t_, t_, s_, reducer(), sc, 2, status_.get(),
-                          true, Epilogue::BicgOmega, stream_);
-      launch::bicg_step(n_, x, r_, z_, zs_, s_, t_, sc, status_.get(), stream_);
-      launch::reduce_into(ReduceMode::Dot, n_, r_, r_, r_, r_, reducer(), sc, 18, status_.get(),
-                          true, Epilogue::CheckBicg, stream_);
-      tally(2.0 * (8.0 * nnz_ + 4.0 * (n_ + 1)) + 104.0 * n_);
+      launch::spmv_dot2(n_, rows0(), cols0(), val_, zs_, s_, t_, reducer(), sc, status_.get(),
+                        stream_);
+      launch::bicg_step(n_, x, r_, z_, zs_, s_, t_, shadow_, reducer(), sc, status_.get(),
+                        stream_);
+      tally(2.0 * (8.0 * nnz_ + 4.0 * (n_ + 1)) + 80.0 * n_);
     }
     const auto state = poll(x, b);
     stats.iterations = state[1];

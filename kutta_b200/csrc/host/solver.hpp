@@ -209,6 +209,8 @@ class Solver {
            !(learned_ != nullptr && (learned_mode_ & kLearnedCycle));
   }
   bool fuse_dots_ = false;
+  // The fine level's first sweep was made by the update before apply().
+  bool swept_ = false;
   void precondition(const float* r, float*& z);
   // c = G(t), q = A c and the dots {c.t, c.Ac} for the safeguarded step.
   void learned_direction(const float* t);
