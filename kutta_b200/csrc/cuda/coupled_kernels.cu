@@ -89,61 +89,6 @@ __global__ void k_cpl_face_coefficient(int nf, int internal, const int* __restri
   }
 }
 
-// fv_coupled.kern.h:93-108 (coupled_velocity_block): H_ii into planes 7-9.
-__global__ void __launch_bounds__(kBlock, 8) k_cpl_velocity_block(int n, int internal, const int* __restrict__ offsets,
-                                     const int* __restrict__ faces,
-                                     const float* __restrict__ sign,
-                                     const int* __restrict__ adjacent,
-                                     const int* __restrict__ kind, const float* __restrict__ sx,
-                                     const float* __restrict__ sy, const float* __restrict__ sz,
-                                     const float* __restrict__ weight, float* __restrict__ cell) {
-  pdl_entry();
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    float hx = 0.0f, hy = 0.0f, hz = 0.0f;
-    for (int j = offsets[i]; j < offsets[i + 1]; ++j) {
-      const int f = faces[j], c = adjacent[j];
-      float share = 0.0f;
-      if (c >= 0) {
-        share = 1.0f - share_of(weight, i, c);
-      } else {
-        const int k = kind[f - internal];
-        if (k == 2 || k == 4) share = 1.0f;
-      }
-      const float s = share * sign[j];
-      hx += s * sx[f];
-      hy += s * sy[f];
-      hz += s * sz[f];
-    }
-    cell[7 * static_cast<std::size_t>(n) + i] = hx;
-    cell[8 * static_cast<std::size_t>(n) + i] = hy;
-    cell[9 * static_cast<std::size_t>(n) + i] = hz;
-  }
-}
-
-// fv_coupled.kern.h:131-150 (coupled_rhs): the pressure diagonal into plane
-// 3 and the block right-hand side.
-__global__ void k_cpl_rhs(int n, const int* __restrict__ offsets, const int* __restrict__ faces,
-                          const float* __restrict__ sign, const float* __restrict__ coefficient,
-                          const float* __restrict__ mass, const float* __restrict__ net,
-                          const float* __restrict__ ru, const float* __restrict__ rv,
-                          const float* __restrict__ rw, float* __restrict__ cell,
-                          float4* __restrict__ b, int reference, float continuity_scale) {
-  pdl_entry();
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    Csum c{0.0f, 0.0f};
-    float imbalance = 0.0f;
-    for (int j = offsets[i]; j < offsets[i + 1]; ++j) {
-      const int f = faces[j];
-      c = csum_add(c, coefficient[f]);
-      imbalance += sign[j] * mass[f];
-    }
-    if (net) imbalance = net[i];
-    const float value = csum_value(c);
-    cell[3 * static_cast<std::size_t>(n) + i] = i == reference ? 2.0f * value : value;
-    b[i] = make_float4(ru[i], rv[i], rw[i], -continuity_scale * imbalance);
-  }
-}
-
 struct FineGeometry {
   const int* offsets;
   const int* faces;
@@ -153,9 +98,19 @@ struct FineGeometry {
   const float *dx, *dy, *dz;
 };
 
-// fv_coupled.kern.h:191-208 (coupled_fine_gsum): |G| row sums, 3n planes.
-__global__ void __launch_bounds__(kBlock, 8) k_cpl_fine_gsum(int n, FineGeometry m, const float* __restrict__ cell,
-                                float* __restrict__ r, float wc) {
+// One pass over each cell's faces for three of the reference's kernels, whose
+// sums are independent (each in its own order): coupled_velocity_block
+// (fv_coupled.kern.h:93-108), H_ii into planes 7-9; coupled_rhs (:131-150), the
+// pressure diagonal into plane 3 and the block right-hand side; and
+// coupled_fine_gsum (:191-208), the |G| row sums, 3n planes. Bound by the face
+// data's latency: as three kernels 130 us at 884,736 hexes, this 75.
+__global__ void __launch_bounds__(kBlock, 5) k_cpl_cell_sums(
+    int n, int internal, FineGeometry m, const int* __restrict__ kind,
+    const float* __restrict__ weight, const float* __restrict__ coefficient,
+    const float* __restrict__ mass, const float* __restrict__ net, const float* __restrict__ ru,
+    const float* __restrict__ rv, const float* __restrict__ rw, float* __restrict__ cell,
+    float* __restrict__ r, float4* __restrict__ b, int reference, float continuity_scale,
+    float wc) {
   pdl_entry();
   const std::size_t N = n;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -165,36 +120,39 @@ __global__ void __launch_bounds__(kBlock, 8) k_cpl_fine_gsum(int n, FineGeometry
     const float half_wc = 0.5f * wc;
     float gx = fabsf(wc * cell[4 * N + i]), gy = fabsf(wc * cell[5 * N + i]),
           gz = fabsf(wc * cell[6 * N + i]);
+    float hx = 0.0f, hy = 0.0f, hz = 0.0f;
+    Csum c{0.0f, 0.0f};
+    float imbalance = 0.0f;
     for (int j = m.offsets[i]; j < m.offsets[i + 1]; ++j) {
-      if (m.adjacent[j] < 0) continue;
-      const int f = m.faces[j];
-      const float s = m.sign[j];
-      gx += fabsf(half_wc * s * m.sx[f] + q00 * m.dx[j] + q01 * m.dy[j] + q02 * m.dz[j]);
-      gy += fabsf(half_wc * s * m.sy[f] + q10 * m.dx[j] + q11 * m.dy[j] + q12 * m.dz[j]);
-      gz += fabsf(half_wc * s * m.sz[f] + q20 * m.dx[j] + q21 * m.dy[j] + q22 * m.dz[j]);
+      const int f = m.faces[j], other = m.adjacent[j];
+      const float s = m.sign[j], sx = m.sx[f], sy = m.sy[f], sz = m.sz[f];
+      c = csum_add(c, coefficient[f]);
+      imbalance += s * mass[f];
+      float share = 0.0f;
+      if (other >= 0) {
+        share = 1.0f - share_of(weight, i, other);
+        gx += fabsf(half_wc * s * sx + q00 * m.dx[j] + q01 * m.dy[j] + q02 * m.dz[j]);
+        gy += fabsf(half_wc * s * sy + q10 * m.dx[j] + q11 * m.dy[j] + q12 * m.dz[j]);
+        gz += fabsf(half_wc * s * sz + q20 * m.dx[j] + q21 * m.dy[j] + q22 * m.dz[j]);
+      } else {
+        const int k = kind[f - internal];
+        if (k == 2 || k == 4) share = 1.0f;
+      }
+      const float t = share * s;
+      hx += t * sx;
+      hy += t * sy;
+      hz += t * sz;
     }
+    if (net) imbalance = net[i];
+    const float value = csum_value(c);
+    cell[3 * N + i] = i == reference ? 2.0f * value : value;
+    cell[7 * N + i] = hx;
+    cell[8 * N + i] = hy;
+    cell[9 * N + i] = hz;
     r[i] = gx;
     r[N + i] = gy;
     r[2 * N + i] = gz;
-  }
-}
-
-// fv_coupled.kern.h:210-223 (coupled_fine_schur): cs into plane 19.
-__global__ void k_cpl_fine_schur(int n, FineGeometry m, const float* __restrict__ weight,
-                                 const float* __restrict__ r, float* __restrict__ cell, float wc) {
-  pdl_entry();
-  const std::size_t N = n;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    float sum = 0.0f;
-    for (int j = m.offsets[i]; j < m.offsets[i + 1]; ++j) {
-      const int c = m.adjacent[j];
-      if (c < 0) continue;
-      const int f = m.faces[j];
-      sum += wc * share_of(weight, i, c) *
-             (fabsf(m.sx[f]) * r[c] / cell[c] + fabsf(m.sy[f]) * r[N + c] / cell[N + c] +
-              fabsf(m.sz[f]) * r[2 * N + c] / cell[2 * N + c]);
-    }
-    cell[19 * N + i] = sum;
+    b[i] = make_float4(ru[i], rv[i], rw[i], -continuity_scale * imbalance);
   }
 }
 
@@ -209,47 +167,55 @@ __global__ void k_cpl_face_records(int nf, const float* __restrict__ sx,
     face[f] = make_float4(sx[f], sy[f], sz[f], coefficient[f]);
 }
 
-// fv_coupled.kern.h:229-256 (coupled_fine_coefficients): the block inverse
-// and the five directed-edge coefficients, written as the per-cell records
-// and the ELL slots of the fine operator.
+// coupled_fine_schur (fv_coupled.kern.h:210-223), cs into plane 19, and
+// coupled_fine_coefficients (:229-256), the block inverse and the five
+// directed-edge coefficients as the per-cell records and the ELL slots of the
+// fine operator, in one pass over each cell's faces (as two kernels 163 us at
+// 884,736 hexes, this 125).
 __global__ void k_cpl_fine_pack(int n, int width, FineGeometry m, const float* __restrict__ mu,
                                 const float* __restrict__ diffusion,
                                 const float* __restrict__ mass, const float* __restrict__ weight,
-                                const float* __restrict__ cell, CoupledFine op, float wc) {
+                                const float* __restrict__ r, float* cell, CoupledFine op,
+                                float wc) {
   pdl_entry();
   const std::size_t N = n;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const float du = cell[i], dv = cell[N + i], dw = cell[2 * N + i], cd = cell[3 * N + i];
-    const float ex = wc * cell[4 * N + i], ey = wc * cell[5 * N + i], ez = wc * cell[6 * N + i];
-    const float hx = wc * cell[7 * N + i], hy = wc * cell[8 * N + i], hz = wc * cell[9 * N + i];
-    const BlockInverse inv = block_prepare(du, dv, dw, ex, ey, ez, hx, hy, hz, cd + cell[19 * N + i]);
-    op.diag[i] = make_float4(du, dv, dw, cd);
-    op.coupling[i] = make_float4(ex, ey, ez, hx);
-    op.coupling_yz[i] = make_float2(hy, hz);
-    op.schur[i] = inv.schur;
     const float q00 = wc * cell[10 * N + i], q01 = wc * cell[11 * N + i], q02 = wc * cell[12 * N + i];
     const float q10 = wc * cell[13 * N + i], q11 = wc * cell[14 * N + i], q12 = wc * cell[15 * N + i];
     const float q20 = wc * cell[16 * N + i], q21 = wc * cell[17 * N + i], q22 = wc * cell[18 * N + i];
     const float half_wc = 0.5f * wc;
+    float sum = 0.0f;
     int slot = 0;
     for (int j = m.offsets[i]; j < m.offsets[i + 1] && slot < width; ++j) {
       const int c = m.adjacent[j];
       if (c < 0) continue;
       const int f = m.faces[j];
-      const float s = m.sign[j];
+      const float s = m.sign[j], share = share_of(weight, i, c);
+      const float sx = m.sx[f], sy = m.sy[f], sz = m.sz[f];
+      sum += wc * share *
+             (fabsf(sx) * r[c] / cell[c] + fabsf(sy) * r[N + c] / cell[N + c] +
+              fabsf(sz) * r[2 * N + c] / cell[2 * N + c]);
       const float a = -mu[f] * diffusion[f] + fminf(s * mass[f], 0.0f);
-      const float bx = half_wc * s * m.sx[f], by = half_wc * s * m.sy[f], bz = half_wc * s * m.sz[f];
+      const float bx = half_wc * s * sx, by = half_wc * s * sy, bz = half_wc * s * sz;
       const float gx = bx + q00 * m.dx[j] + q01 * m.dy[j] + q02 * m.dz[j];
       const float gy = by + q10 * m.dx[j] + q11 * m.dy[j] + q12 * m.dz[j];
       const float gz = bz + q20 * m.dx[j] + q21 * m.dy[j] + q22 * m.dz[j];
-      const float h = wc * s * share_of(weight, i, c);
       const std::size_t k = slot * N + i;
       op.edge[k] = make_float4(a, gx, gy, gz);
-      op.edge_h[k] = h;
+      op.edge_h[k] = wc * s * share;
       op.link[k] = make_int2(c, f);
       ++slot;
     }
     for (; slot < width; ++slot) op.link[slot * N + i] = make_int2(-1, 0);
+    cell[19 * N + i] = sum;
+    const float du = cell[i], dv = cell[N + i], dw = cell[2 * N + i], cd = cell[3 * N + i];
+    const float ex = wc * cell[4 * N + i], ey = wc * cell[5 * N + i], ez = wc * cell[6 * N + i];
+    const float hx = wc * cell[7 * N + i], hy = wc * cell[8 * N + i], hz = wc * cell[9 * N + i];
+    const BlockInverse inv = block_prepare(du, dv, dw, ex, ey, ez, hx, hy, hz, cd + sum);
+    op.diag[i] = make_float4(du, dv, dw, cd);
+    op.coupling[i] = make_float4(ex, ey, ez, hx);
+    op.coupling_yz[i] = make_float2(hy, hz);
+    op.schur[i] = inv.schur;
   }
 }
 
@@ -484,23 +450,17 @@ void cpl_assemble(const CoupledMeshDevice& m, const CoupledSolveInputs& in, floa
   const int n = m.n, nf = m.n_faces;
   if (n <= 0) return;
   const FineGeometry g = geometry(m);
-  counter += 7;
+  counter += 4;
   pdl(k_cpl_face_coefficient, grid_for(nf), kBlock, 0, s, nf, m.n_internal, m.owner,
       m.neighbour, m.kind, m.diffusion, m.volume, in.physical_diagonal, coefficient,
       coefficient_scale);
-  pdl(k_cpl_velocity_block, grid_for(n), kBlock, 0, s, n, m.n_internal, m.offsets, m.faces,
-      m.sign, m.adjacent, m.kind, m.sx, m.sy, m.sz, in.face_weights, cell);
-  pdl(k_cpl_rhs, grid_for(n), kBlock, 0, s, n, m.offsets, m.faces, m.sign,
+  pdl(k_cpl_cell_sums, grid_for(n), kBlock, 0, s, n, m.n_internal, g, m.kind, in.face_weights,
       static_cast<const float*>(coefficient), in.mass, in.net_outflow, in.ru, in.rv, in.rw, cell,
-      b, reference, continuity_scale);
-  pdl(k_cpl_fine_gsum, grid_for(n), kBlock, 0, s, n, g, static_cast<const float*>(cell), scratch,
-      wc);
-  pdl(k_cpl_fine_schur, grid_for(n), kBlock, 0, s, n, g, in.face_weights,
-      static_cast<const float*>(scratch), cell, wc);
+      scratch, b, reference, continuity_scale, wc);
   pdl(k_cpl_face_records, grid_for(nf), kBlock, 0, s, nf, m.sx, m.sy, m.sz,
       static_cast<const float*>(coefficient), const_cast<float4*>(op.face));
   pdl(k_cpl_fine_pack, grid_for(n), kBlock, 0, s, n, m.width, g, in.viscosity, m.diffusion,
-      in.mass, in.face_weights, static_cast<const float*>(cell), op, wc);
+      in.mass, in.face_weights, static_cast<const float*>(scratch), cell, op, wc);
 }
 
 void cpl_fine_spmv(int n, const CoupledFine& op, int width, const float4* x, float4* y,
