@@ -62,21 +62,24 @@ enum class Rows { Residual, Smooth, SmoothProlonged };
 
 // out = b - A x, or the sweep x + (2/3) inv (b - A x); SmoothProlonged reads
 // x + coarse[aggregate] in the place of x (the prolongation, which adds it
-// once per row, folded into the first post-sweep).
-template <int kRows, int kPer, int kAhead, Rows kMode>
+// once per row, folded into the first post-sweep). kSorted: the block's rows go to
+// its threads in the given order, longest first, so that a warp of short rows
+// does not wait for a hub row in it.
+template <int kRows, int kPer, int kAhead, Rows kMode, bool kSorted>
 __global__ void __launch_bounds__(kBlock) k_staged_rows(
     int n, const int* __restrict__ rows, const int* __restrict__ cols,
     const float* __restrict__ vals, const float* __restrict__ inv, const float* __restrict__ x,
     const float* __restrict__ b, float* __restrict__ out, const int* __restrict__ status,
-    const int* __restrict__ aggregate, const float* __restrict__ coarse) {
+    const int* __restrict__ aggregate, const float* __restrict__ coarse,
+    const int* __restrict__ order) {
   constexpr int kStage = kPer * kBlock;
   constexpr bool kProlong = kMode == Rows::SmoothProlonged;
   __shared__ float2 staged[kStage];
   const int tid = threadIdx.x;
   const int row0 = blockIdx.x * kRows, row1 = min(n, row0 + kRows);
   const int first = rows[row0], last = rows[row1];
-  const int i = row0 + tid;
-  const bool owner = tid < kRows && i < n;
+  const bool owner = tid < kRows && row0 + tid < n;
+  const int i = kSorted && owner ? order[row0 + tid] : row0 + tid;
   const int begin = owner ? rows[i] : 0, end = owner ? rows[i + 1] : 0;
   const float scale = kMode != Rows::Residual && owner ? inv[i] : 0.0f;
   const int own_group = kProlong && owner ? aggregate[i] : -1;
@@ -398,19 +401,24 @@ int row_blocks(int n, int rows) { return (n + rows - 1) / rows; }
 template <Rows kMode>
 void staged(int n, const int* rows, const int* cols, const float* vals, const float* inv,
             const float* x, const float* b, float* out, const int* status, const int* aggregate,
-            const float* coarse, cudaStream_t s) {
+            const float* coarse, const int* order, cudaStream_t s) {
   ++launch::counter;
   // Few rows: 64 to a block, each thread one to four entries, with the adding
   // looked ahead (12,571 rows, longest 165: 3.8 us a sweep against 4.0 with the
   // larger form; 4,096 rows of up to 7: 2.0 against 2.1). More rows: 128 to a
   // block and plain adding, which leaves registers for more blocks (39,033 rows:
   // 3.6 us against 3.7; 48,848: 5.2 against 5.7; 159,785: 5.6 against 7.9).
+  // An order comes with levels whose longest row has kStagedHub entries or more
+  // (48,848 rows, longest 123: 4.4 us against 5.2; at 46 entries it gives nothing).
   if (n <= launch::kStagedSmall)
-    pdl(k_staged_rows<64, 4, 4, kMode>, row_blocks(n, 64), kBlock, 0, s, n, rows, cols, vals, inv,
-        x, b, out, status, aggregate, coarse);
+    pdl(k_staged_rows<64, 4, 4, kMode, false>, row_blocks(n, 64), kBlock, 0, s, n, rows, cols,
+        vals, inv, x, b, out, status, aggregate, coarse, order);
+  else if (order != nullptr)
+    pdl(k_staged_rows<128, 8, 0, kMode, true>, row_blocks(n, 128), kBlock, 0, s, n, rows, cols,
+        vals, inv, x, b, out, status, aggregate, coarse, order);
   else
-    pdl(k_staged_rows<128, 8, 0, kMode>, row_blocks(n, 128), kBlock, 0, s, n, rows, cols, vals,
-        inv, x, b, out, status, aggregate, coarse);
+    pdl(k_staged_rows<128, 8, 0, kMode, false>, row_blocks(n, 128), kBlock, 0, s, n, rows, cols,
+        vals, inv, x, b, out, status, aggregate, coarse, order);
 }
 
 }  // namespace
@@ -418,20 +426,22 @@ void staged(int n, const int* rows, const int* cols, const float* vals, const fl
 namespace launch {
 
 void staged_residual(int n, const int* rows, const int* cols, const float* vals, const float* x,
-                     const float* b, float* r, const int* status, cudaStream_t s) {
+                     const float* b, float* r, const int* status, const int* order,
+                     cudaStream_t s) {
   if (n <= 0) return;
-  staged<Rows::Residual>(n, rows, cols, vals, nullptr, x, b, r, status, nullptr, nullptr, s);
+  staged<Rows::Residual>(n, rows, cols, vals, nullptr, x, b, r, status, nullptr, nullptr, order,
+                         s);
 }
 
 void staged_smooth(int n, const int* rows, const int* cols, const float* vals, const float* x,
                    const float* b, const float* inv, float* next, const int* status,
-                   const int* aggregate, const float* coarse, cudaStream_t s) {
+                   const int* aggregate, const float* coarse, const int* order, cudaStream_t s) {
   if (n <= 0) return;
   if (aggregate != nullptr)
     staged<Rows::SmoothProlonged>(n, rows, cols, vals, inv, x, b, next, status, aggregate, coarse,
-                                  s);
+                                  order, s);
   else
-    staged<Rows::Smooth>(n, rows, cols, vals, inv, x, b, next, status, nullptr, nullptr, s);
+    staged<Rows::Smooth>(n, rows, cols, vals, inv, x, b, next, status, nullptr, nullptr, order, s);
 }
 
 void restrict_rows(int nc, const int* offsets, const int* members, const float* fine,

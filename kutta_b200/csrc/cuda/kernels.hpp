@@ -133,14 +133,16 @@ void level_rows(int n, const int* rows, const int* diag, float* vals, const Leve
 // one thread per row adds them. They load the operator before they wait for
 // the previous kernel, so that kernel must not be its writer. At most
 // kStagedSmall rows take blocks of 64 rows, more take 128 (see staged()).
-constexpr int kStagedSmall = 16384;
+// With order, rows [128 k, 128 k + 128) are taken in that order (longest first).
+constexpr int kStagedSmall = 16384, kStagedHub = 64;
 void staged_residual(int n, const int* rows, const int* cols, const float* vals, const float* x,
-                     const float* b, float* r, const int* status, cudaStream_t s);
+                     const float* b, float* r, const int* status, const int* order,
+                     cudaStream_t s);
 // With aggregate != null the sweep starts from x + coarse[aggregate] (the
 // prolongation folded in; x itself is left as it is).
 void staged_smooth(int n, const int* rows, const int* cols, const float* vals, const float* x,
                    const float* b, const float* inv, float* next, const int* status,
-                   const int* aggregate, const float* coarse, cudaStream_t s);
+                   const int* aggregate, const float* coarse, const int* order, cudaStream_t s);
 // b_c = the Kahan sum of each aggregate's members of `fine`; with next != null the coarse level's zero-start sweep too.
 void restrict_rows(int nc, const int* offsets, const int* members, const float* fine,
                    float* coarse, const int* rows, const float* vals, const float* inv,

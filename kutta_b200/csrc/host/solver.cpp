@@ -184,9 +184,19 @@ void Solver::plan_plain(cudaStream_t s) {
   for (std::size_t i = 0; i < levels_.size(); ++i) {
     auto& l = levels_[i];
     l.staged = l.n <= kDirectRows;
-    if (i == 0 || l.staged) continue;
+    if (i == 0 || l.n <= launch::kStagedSmall) continue;
     const std::vector<int> rows = row_pointers(l, s);
-    for (int k = 0; k < l.n && !l.staged; ++k) l.staged = rows[k + 1] - rows[k] > kDirectLongest;
+    int longest = 0;
+    for (int k = 0; k < l.n; ++k) longest = std::max(longest, rows[k + 1] - rows[k]);
+    l.staged = l.staged || longest > kDirectLongest;
+    if (longest < launch::kStagedHub) continue;
+    std::vector<int> order(static_cast<std::size_t>(l.n));
+    std::iota(order.begin(), order.end(), 0);
+    for (int k = 0; k < l.n; k += 128)
+      std::stable_sort(order.begin() + k, order.begin() + std::min(l.n, k + 128),
+                       [&](int p, int q) { return rows[p + 1] - rows[p] > rows[q + 1] - rows[q]; });
+    l.order.upload(order, s);
+    wait(s);  // the host array is released here
   }
   if (nullspace_ || options_.cycle != Cycle::V) return;
   launch::PlainTail t{};
@@ -544,7 +554,8 @@ void Solver::smooth(DevLevel& l, const int* rows, const int* cols, const float* 
                           scalars_.get(), 4, status_.get(), Epilogue::PcgBetaFlexible, stream_);
     else if (l.staged && !zero)
       launch::staged_smooth(l.n, rows, cols, vals, x, b, l.l1.get(), l.r, status,
-                            sweep == 0 && coarse ? l.aggregate.get() : nullptr, coarse, stream_);
+                            sweep == 0 && coarse ? l.aggregate.get() : nullptr, coarse,
+                            l.order.get(), stream_);
     else
       launch::smooth(l.n, rows, cols, vals, x, b, l.l1.get(), l.r, status, zero, stream_);
     if (timed) cuda_check(cudaEventRecord(events_[events_used_++], stream_), "cudaEventRecord");
@@ -594,7 +605,7 @@ void Solver::cycle(std::size_t index, const float* b, float*& x, const int* stat
     else if (index == 0 && packed_.width > 0)
       launch::packed_residual(l.n, packed(), x, b, l.r, status, stream_);
     else if (l.staged)
-      launch::staged_residual(l.n, rows, cols, vals, x, b, l.r, status, stream_);
+      launch::staged_residual(l.n, rows, cols, vals, x, b, l.r, status, l.order.get(), stream_);
     else
       launch::residual(l.n, rows, cols, vals, x, b, l.r, status, stream_);
     auto& c = levels_[index + 1];

@@ -85,6 +85,7 @@ struct DevLevel {
   // The plain solve's row kernels form the row's products with all threads of a
   // block (launch::staged_smooth) instead of a thread per row.
   bool staged = false;
+  DArray<int> order;            // rows by length in blocks of 128 (levels with hub rows)
   // Levels of the one-block tail (launch::PlainTail::Level).
   DArray<int> tail_order, tail_start, tail_source;
   // transfer to level + 1
