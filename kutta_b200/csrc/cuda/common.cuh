@@ -225,12 +225,18 @@ __device__ __forceinline__ void neumaier_term(float& sum, float& error, float te
   sum = next;
 }
 
+// The next float above a finite v: a float's bits order as integers within each
+// sign, so one up or, below zero, one down; the smallest subnormal above a zero.
+__device__ __forceinline__ float next_up(float v) {
+  const int bits = __float_as_int(v);
+  return v == 0.0f ? __int_as_float(1) : __int_as_float(bits + (bits >> 31 | 1));
+}
 // Upward-rounded sums, src/kutta/kernels/prelude.h:82-100.
 __device__ __forceinline__ float add_up(float a, float b) {
   const float sum = a + b;
   const float part = sum - a;
   const float error = (a - (sum - part)) + (b - part);
-  return error > 0.0f ? nextafterf(sum, __int_as_float(0x7f800000)) : sum;
+  return error > 0.0f ? next_up(sum) : sum;
 }
 struct UpperSum {
   float sum, error;
@@ -268,34 +274,72 @@ __device__ __forceinline__ double block_sum(double v, double* shared /* >= 32 */
 }
 __device__ __forceinline__ double nan_max(double a, double b) { return (b > a || isnan(b)) ? b : a; }
 
+// The end of krylov_diagonal's row: the inverse (L1) diagonal from the diagonal,
+// the off-diagonal magnitudes' sum and whether a value is not finite; returns
+// the invalid flag.
+__device__ __forceinline__ float diagonal_value(float d, float off, float bad, int use_l1,
+                                                float& inverse) {
+  const float inv = d != 0.0f ? 1.0f / d : 0.0f;
+  const float l1 = fmaxf(fabsf(d), 0.5f * (fabsf(d) + off));
+  inverse = use_l1 != 0 ? (l1 != 0.0f ? 1.0f / l1 : 0.0f) : inv;
+  return (bad != 0.0f || inv - inv != 0.0f || l1 - l1 != 0.0f)
+             ? 2.0f
+             : (use_l1 != 0 && d < 0.0f ? 3.0f : (d == 0.0f ? 1.0f : 0.0f));
+}
+
+// f(j, vals[j]) for the entries of a row in order, eight loads in flight: the
+// rows' chains are short next to a load each.
+template <class F>
+__device__ __forceinline__ void row_values(const float* vals, int begin, int end, F f) {
+  constexpr int kBatch = 8;
+  for (int j = begin; j < end; j += kBatch) {
+    float v[kBatch];
+#pragma unroll
+    for (int k = 0; k < kBatch; ++k) v[k] = j + k < end ? vals[j + k] : 0.0f;
+#pragma unroll
+    for (int k = 0; k < kBatch; ++k)
+      if (j + k < end) f(j + k, v[k]);
+  }
+}
+
 // krylov_diagonal's row (src/kutta/kernels/linalg.kern.h:52-70): the inverse
 // (L1) diagonal of row i into inverse[i]; returns its invalid flag (0 valid,
 // 1 zero diagonal, 2 nonfinite, 3 negative diagonal under L1).
 __device__ __forceinline__ float diagonal_row(int i, const int* __restrict__ rows,
                                               const int* __restrict__ diag,
                                               const float* vals, float* inverse, int use_l1) {
-  const float d = vals[diag[i]];
+  const int at = diag[i];
+  const float d = vals[at];
   float off = 0.0f, bad = 0.0f;
-  for (int j = rows[i]; j < rows[i + 1]; ++j) {
-    const float v = vals[j];
+  row_values(vals, rows[i], rows[i + 1], [&](int j, float v) {
     if (v - v != 0.0f) bad = 1.0f;
-    if (j != diag[i]) off += fabsf(v);
-  }
-  const float inv = d != 0.0f ? 1.0f / d : 0.0f;
-  const float l1 = fmaxf(fabsf(d), 0.5f * (fabsf(d) + off));
-  inverse[i] = use_l1 != 0 ? (l1 != 0.0f ? 1.0f / l1 : 0.0f) : inv;
-  return (bad != 0.0f || inv - inv != 0.0f || l1 - l1 != 0.0f)
-             ? 2.0f
-             : (use_l1 != 0 && d < 0.0f ? 3.0f : (d == 0.0f ? 1.0f : 0.0f));
+    if (j != at) off += fabsf(v);
+  });
+  return diagonal_value(d, off, bad, use_l1, inverse[i]);
 }
 // amg_m_matrix_diagonal's share of fine row i (src/kutta/kernels/amg.kern.h:44-58):
 // its diagonal plus its off-diagonals, upward rounded.
 __device__ __forceinline__ float row_surplus(int i, const int* __restrict__ rows,
                                              const int* __restrict__ diag, const float* vals) {
-  UpperSum sum{vals[diag[i]], 0.0f};
-  for (int j = rows[i]; j < rows[i + 1]; ++j)
-    if (j != diag[i]) sum = upper_add(sum, vals[j]);
+  const int at = diag[i];
+  UpperSum sum{vals[at], 0.0f};
+  row_values(vals, rows[i], rows[i + 1], [&](int j, float v) {
+    if (j != at) sum = upper_add(sum, v);
+  });
   return upper_value(sum);
+}
+// Row i's values as the packed rows hold them: the off-diagonals in column
+// order, then zeros; the diagonal apart.
+__device__ __forceinline__ void pack_row(int i, int width, const int* __restrict__ rows,
+                                         const int* __restrict__ diag, const float* vals,
+                                         float* packed, float* packed_diag) {
+  float* out = packed + static_cast<std::size_t>(i) * width;
+  const int d = diag[i];
+  int k = 0;
+  for (int j = rows[i]; j < rows[i + 1]; ++j)
+    if (j != d) out[k++] = vals[j];
+  for (; k < width; ++k) out[k] = 0.0f;
+  packed_diag[i] = vals[d];
 }
 __device__ __forceinline__ double warp_max(double v) {
 #pragma unroll

@@ -117,6 +117,19 @@ __device__ __forceinline__ void finish(const Reducer& red, double a, double b, b
   }
 }
 
+// The maximum over the grid into check[slot] (NaN wins).
+__device__ __forceinline__ void finish_max(const Reducer& red, double worst, double* check,
+                                           int slot) {
+  __shared__ double shared[32];
+  worst = block_max(worst, shared);
+  if (!publish(red, worst, 0, false)) return;
+  const double total = gather_max(red, shared);
+  if (threadIdx.x == 0) {
+    check[slot] = total;
+    *red.ticket = 0;
+  }
+}
+
 // BiCGStab's r.r and, for the next update, rhat.r: solver_check, then
 // solver_bicg_beta unless the check stopped the iteration (solver.cpp:314-361
 // runs the second at the start of the next update, on the same r).

@@ -306,15 +306,7 @@ __global__ void k_pack_rows(int n, int width, const int* __restrict__ rows,
                             const int* __restrict__ diag_index, const float* __restrict__ vals,
                             float* __restrict__ packed, float* __restrict__ packed_diag) {
   pdl_entry();
-  ROWS(i, n) {
-    float* out = packed + static_cast<std::size_t>(i) * width;
-    int k = 0;
-    const int d = diag_index[i];
-    for (int j = rows[i]; j < rows[i + 1]; ++j)
-      if (j != d) out[k++] = vals[j];
-    for (; k < width; ++k) out[k] = 0.0f;
-    packed_diag[i] = vals[d];
-  }
+  ROWS(i, n) pack_row(i, width, rows, diag_index, vals, packed, packed_diag);
 }
 
 // amg_coarse_solve, linalg.kern.h:126-147: the whole <=24-row system in one
@@ -364,15 +356,7 @@ __global__ void k_diagonal(int n, const int* __restrict__ rows, const int* __res
   pdl_entry();
   double worst = 0;
   ROWS(i, n) worst = nan_max(worst, diagonal_row(i, rows, diag, vals, inverse, use_l1));
-  __shared__ double shared[32];
-  worst = block_max(worst, shared);
-  const Reducer r = as_reducer(red);
-  if (!publish(r, worst, 0, false)) return;
-  const double total = gather_max(r, shared);
-  if (threadIdx.x == 0) {
-    check[slot] = total;
-    *r.ticket = 0;
-  }
+  finish_max(as_reducer(red), worst, check, slot);
 }
 
 // ---- AMG transfer and Galerkin, src/kutta/kernels/amg.kern.h ------------------
@@ -388,16 +372,39 @@ __global__ void k_prolong(int nf, const int* __restrict__ aggregate,
   }
 }
 
-// amg_galerkin :27-38: Neumaier sum over the coarse entry's fine entries.
-__global__ void k_galerkin(int nnz_c, const int* __restrict__ offsets,
-                           const int* __restrict__ entries, const float* __restrict__ fine,
-                           float* __restrict__ coarse) {
+// amg_galerkin :27-38: Neumaier sum over the coarse entry's fine entries. An
+// off-diagonal entry has one to a few of them, a diagonal some thirty, and a
+// warp walks as far as its longest list; so the diagonals, marked in `diagonal`
+// (a bit per entry), are summed by blocks of their own, a thread per row, or not
+// at all where the M-matrix diagonal replaces them (kDiagonals false).
+template <bool kDiagonals>
+__global__ void k_galerkin(int n_c, int nnz_c, const int* __restrict__ offsets,
+                           const int* __restrict__ entries, const unsigned* __restrict__ diagonal,
+                           const int* __restrict__ diag, const float* __restrict__ fine,
+                           float* __restrict__ coarse, int diagonal_blocks) {
   pdl_entry();
-  ROWS(e, nnz_c) {
+  const auto sum_list = [&](int e) {
     float sum = 0.0f, error = 0.0f;
-    for (int j = offsets[e]; j < offsets[e + 1]; ++j) neumaier_term(sum, error, fine[entries[j]]);
+    const int end = offsets[e + 1];
+    for (int j = offsets[e]; j < end; ++j) neumaier_term(sum, error, fine[entries[j]]);
     coarse[e] = sum + error;
+  };
+  const int block = static_cast<int>(blockIdx.x) - diagonal_blocks;
+  if (kDiagonals && block < 0) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n_c) sum_list(diag[i]);
+    return;
   }
+  const int stride = (gridDim.x - diagonal_blocks) * blockDim.x;
+  for (int e = block * blockDim.x + threadIdx.x; e < nnz_c; e += stride)
+    if (!(diagonal[e >> 5] >> (e & 31) & 1u)) sum_list(e);
+}
+
+// The bits of the diagonal entries (words zeroed before).
+__global__ void k_mark_diagonals(int n, const int* __restrict__ diag,
+                                 unsigned* __restrict__ words) {
+  pdl_entry();
+  ROWS(i, n) atomicOr(words + (diag[i] >> 5), 1u << (diag[i] & 31));
 }
 
 // amg_m_matrix_diagonal :44-58 in two passes with the same roundings in the
@@ -432,9 +439,9 @@ __global__ void k_m_matrix_combine(int nc, const int* __restrict__ offsets,
 // inverse L1 diagonal and its invalid flag (k_diagonal), and where wanted the
 // row's surplus for the level below (k_row_surplus) and its BF16 copy
 // (k_bf16_pack). A thread's row stays in L1 between the parts, and every part
-// is the same operations in the same order. Assembly, refresh and corrections on
-// the 1.57M-row tet hierarchy take 15 launches instead of 30, 440 us instead of
-// 462.
+// is the same operations in the same order. (Staging a block's rows in shared
+// memory was slower: the upward-rounded chains bound it, not the loads; eight
+// loads in flight took the levels of a 1.57M-row tet hierarchy from 101 to 96 us.)
 template <bool kCombine>
 __global__ void k_level_rows(int n, const int* __restrict__ rows, const int* __restrict__ diag,
                              float* vals, const int* __restrict__ offsets,
@@ -447,12 +454,22 @@ __global__ void k_level_rows(int n, const int* __restrict__ rows, const int* __r
   double worst = 0;
   ROWS(i, n) {
     if constexpr (kCombine) {
+      constexpr int kBatch = 8;
       UpperSum diagonal{0.0f, 0.0f};
-      for (int m = offsets[i]; m < offsets[i + 1]; ++m)
-        diagonal = upper_add(diagonal, fine_surplus[members[m]]);
-      for (int j = rows[i]; j < rows[i + 1]; ++j)
-        if (j != diag[i]) diagonal = upper_add(diagonal, -vals[j]);
-      vals[diag[i]] = upper_value(diagonal);
+      const int end = offsets[i + 1];
+      for (int m = offsets[i]; m < end; m += kBatch) {
+        float v[kBatch];
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k) v[k] = m + k < end ? fine_surplus[members[m + k]] : 0.0f;
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k)
+          if (m + k < end) diagonal = upper_add(diagonal, v[k]);
+      }
+      const int at = diag[i];
+      row_values(vals, rows[i], rows[i + 1], [&](int j, float v) {
+        if (j != at) diagonal = upper_add(diagonal, -v);
+      });
+      vals[at] = upper_value(diagonal);
     }
     worst = nan_max(worst, diagonal_row(i, rows, diag, vals, inverse, 1));
     if (surplus != nullptr) surplus[i] = row_surplus(i, rows, diag, vals);
@@ -466,15 +483,7 @@ __global__ void k_level_rows(int n, const int* __restrict__ rows, const int* __r
         v16[j] = __bfloat16_as_ushort(__float2bfloat16_rn(vals[j] * inv));
     }
   }
-  __shared__ double shared[32];
-  worst = block_max(worst, shared);
-  const Reducer r = as_reducer(red);
-  if (!publish(r, worst, 0, false)) return;
-  const double total = gather_max(r, shared);
-  if (threadIdx.x == 0) {
-    check[slot] = total;
-    *r.ticket = 0;
-  }
+  finish_max(as_reducer(red), worst, check, slot);
 }
 
 // ---- Krylov vector updates, scalars.kern.h:122-152 ---------------------------
@@ -823,11 +832,22 @@ void prolong(int nf, const int* aggregate, const float* coarse, float* fine, con
   ++counter;
   pdl(k_prolong, blocks(nf), kBlock, 0, s, nf, aggregate, coarse, fine, status);
 }
-void galerkin(int nnz_c, const int* offsets, const int* entries, const float* fine, float* coarse,
-              cudaStream_t s) {
+void galerkin(int n_c, int nnz_c, const int* offsets, const int* entries, const unsigned* diagonal,
+              const int* diag, bool diagonals, const float* fine, float* coarse, cudaStream_t s) {
   if (nnz_c <= 0) return;
   ++counter;
-  pdl(k_galerkin, blocks(nnz_c), kBlock, 0, s, nnz_c, offsets, entries, fine, coarse);
+  const int own = diagonals ? (n_c + kBlock - 1) / kBlock : 0;
+  if (diagonals)
+    pdl(k_galerkin<true>, own + blocks(nnz_c), kBlock, 0, s, n_c, nnz_c, offsets, entries, diagonal,
+        diag, fine, coarse, own);
+  else
+    pdl(k_galerkin<false>, blocks(nnz_c), kBlock, 0, s, n_c, nnz_c, offsets, entries, diagonal, diag,
+        fine, coarse, own);
+}
+void mark_diagonals(int n, const int* diag, unsigned* words, cudaStream_t s) {
+  if (n <= 0) return;
+  ++counter;
+  pdl(k_mark_diagonals, blocks(n), kBlock, 0, s, n, diag, words);
 }
 void m_matrix_diagonal(int nf, int nc, const int* offsets, const int* members, const int* fine_rows,
                        const int* fine_diag, const float* fine, const int* rows, const int* diag,

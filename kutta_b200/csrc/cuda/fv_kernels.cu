@@ -6,8 +6,10 @@
 //                         and its right-hand side from the face coefficients
 //                         and mass fluxes (:164-183); with `fused`, the row's
 //                         inverse L1 diagonal (the refresh's first step,
-//                         linalg.kern.h:52-70) and its validity flag follow in
-//                         the same pass, from the values the thread just wrote;
+//                         linalg.kern.h:52-70) and its validity flag, the row's
+//                         surplus for the level below and its packed copy follow
+//                         in the same pass, from the values the thread just wrote
+//                         (gathering the row in shared memory first was slower);
 //   fv_correct_flux       face flux correction (:185-190);
 //   fv_correct_velocity   cell velocity and pressure correction (:192-201).
 //
@@ -16,6 +18,7 @@
 #include <cuda_runtime.h>
 
 #include "common.cuh"
+#include "epilogues.cuh"
 #include "kernels.hpp"
 
 namespace kb2 {
@@ -65,30 +68,21 @@ __global__ void k_fv_pressure_assemble(int n, const int* __restrict__ offsets,
                                        const float* __restrict__ coefficient,
                                        const float* __restrict__ flux, float* __restrict__ values,
                                        float* __restrict__ rhs, int reference,
-                                       float* __restrict__ inverse,
-                                       float* __restrict__ surplus, DeviceReducer red,
-                                       double* check, int slot) {
+                                       launch::FvFused fused, DeviceReducer red, double* check,
+                                       int slot) {
   pdl_entry();
   double worst = 0;
   ROWS(i, n) {
     rhs[i] = assemble_row(i, offsets, faces, sign, adjacent, entry, rows, diag, coefficient, flux,
                           values, reference);
     if constexpr (kFused) {
-      worst = nan_max(worst, diagonal_row(i, rows, diag, values, inverse, 1));
-      if (surplus != nullptr) surplus[i] = row_surplus(i, rows, diag, values);
+      worst = nan_max(worst, diagonal_row(i, rows, diag, values, fused.inverse, 1));
+      if (fused.surplus != nullptr) fused.surplus[i] = row_surplus(i, rows, diag, values);
+      if (fused.width > 0)
+        pack_row(i, fused.width, rows, diag, values, fused.packed, fused.packed_diag);
     }
   }
-  if constexpr (kFused) {
-    __shared__ double shared[32];
-    worst = block_max(worst, shared);
-    const Reducer r{red.partials, red.ticket};
-    if (!publish(r, worst, 0, false)) return;
-    const double total = gather_max(r, shared);
-    if (threadIdx.x == 0) {
-      check[slot] = total;
-      *r.ticket = 0;
-    }
-  }
+  if constexpr (kFused) finish_max(as_reducer(red), worst, check, slot);
 }
 
 __global__ void k_fv_correct_flux(int n, const int* __restrict__ owner,
@@ -136,21 +130,19 @@ void fv_pressure_assemble(int n, const int* offsets, const int* faces, const flo
   if (n <= 0) return;
   ++counter;
   pdl(k_fv_pressure_assemble<false>, grid_for(n), kBlock, 0, s, n, offsets, faces, sign, adjacent,
-      entry, rows, diag, coefficient, flux, values, rhs, reference, static_cast<float*>(nullptr),
-      static_cast<float*>(nullptr), DeviceReducer{nullptr, nullptr}, static_cast<double*>(nullptr),
-      0);
+      entry, rows, diag, coefficient, flux, values, rhs, reference, FvFused{},
+      DeviceReducer{nullptr, nullptr}, static_cast<double*>(nullptr), 0);
 }
 
 void fv_pressure_assemble_l1(int n, const int* offsets, const int* faces, const float* sign,
                              const int* adjacent, const int* entry, const int* rows,
                              const int* diag, const float* coefficient, const float* flux,
-                             float* values, float* rhs, int reference, float* inverse,
-                             float* surplus, DeviceReducer red, double* check, int slot, cudaStream_t s) {
+                             float* values, float* rhs, int reference, const FvFused& fused,
+                             DeviceReducer red, double* check, int slot, cudaStream_t s) {
   if (n <= 0) return;
   ++counter;
   pdl(k_fv_pressure_assemble<true>, grid_for(n), kBlock, 0, s, n, offsets, faces, sign, adjacent,
-      entry, rows, diag, coefficient, flux, values, rhs, reference, inverse, surplus, red, check,
-      slot);
+      entry, rows, diag, coefficient, flux, values, rhs, reference, fused, red, check, slot);
 }
 
 void fv_correct_flux(int n, const int* owner, const int* neighbour, const float* correction,

@@ -104,8 +104,11 @@ void diagonal(int n, const int* rows, const int* diag, const float* vals, float*
 // ---- AMG transfer and Galerkin --------------------------------------------
 void prolong(int nf, const int* aggregate, const float* coarse, float* fine, const int* status,
              cudaStream_t s);
-void galerkin(int nnz_c, const int* offsets, const int* entries, const float* fine, float* coarse,
-              cudaStream_t s);
+// Coarse values from the fine ones over the entry map; `diagonal` has a bit per
+// entry (mark_diagonals), and without `diagonals` those are left alone.
+void galerkin(int n_c, int nnz_c, const int* offsets, const int* entries, const unsigned* diagonal,
+              const int* diag, bool diagonals, const float* fine, float* coarse, cudaStream_t s);
+void mark_diagonals(int n, const int* diag, unsigned* words, cudaStream_t s);
 // amg_m_matrix_diagonal: surplus holds nf floats of scratch.
 void m_matrix_diagonal(int nf, int nc, const int* offsets, const int* members, const int* fine_rows,
                        const int* fine_diag, const float* fine, const int* rows, const int* diag,
@@ -386,12 +389,20 @@ void fv_pressure_assemble(int n, const int* offsets, const int* faces, const flo
                           const int* adjacent, const int* entry, const int* rows, const int* diag,
                           const float* coefficient, const float* flux, float* values, float* rhs,
                           int reference, cudaStream_t s);
+// What the assembly fused with the refresh also writes: the inverse L1 diagonal
+// and, where not null (width > 0), the row surpluses (the packed rows).
+struct FvFused {
+  float* inverse;
+  float* surplus;
+  int width;
+  float* packed;
+  float* packed_diag;
+};
 void fv_pressure_assemble_l1(int n, const int* offsets, const int* faces, const float* sign,
                              const int* adjacent, const int* entry, const int* rows,
                              const int* diag, const float* coefficient, const float* flux,
-                             float* values, float* rhs, int reference, float* inverse,
-                             float* surplus, DeviceReducer red, double* check, int slot,
-                             cudaStream_t s);
+                             float* values, float* rhs, int reference, const FvFused& fused,
+                             DeviceReducer red, double* check, int slot, cudaStream_t s);
 void fv_correct_flux(int n, const int* owner, const int* neighbour, const float* correction,
                      const float* coefficient, float* flux, int internal, cudaStream_t s);
 void fv_correct_velocity(int n, const float* volume, const float* inverse, const float* diagonal,

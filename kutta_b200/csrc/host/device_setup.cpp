@@ -186,7 +186,13 @@ class Builder {
                                cudaMemcpyHostToDevice, s_),
                "upload");
     c.val.reset(nnz);
-    launch::galerkin(c.nnz, c.entry_offsets.get(), c.entries.get(), fine.vals, c.val.get(), s_);
+    SArray<unsigned> diagonal((nnz + 31) / 32, s_);
+    if (nnz)
+      cuda_check(cudaMemsetAsync(diagonal.get(), 0, (nnz + 31) / 32 * sizeof(unsigned), s_),
+                 "memset");
+    launch::mark_diagonals(nc, c.diag.get(), diagonal.get(), s_);
+    launch::galerkin(nc, c.nnz, c.entry_offsets.get(), c.entries.get(), diagonal.get(),
+                     c.diag.get(), !o_.m_matrix, fine.vals, c.val.get(), s_);
     if (o_.m_matrix) {
       SArray<float> surplus(static_cast<std::size_t>(fine.n), s_);
       launch::m_matrix_diagonal(fine.n, nc, c.member_offsets.get(), c.members.get(), fine.rows,

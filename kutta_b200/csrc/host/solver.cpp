@@ -158,6 +158,15 @@ Solver::Solver(Kind kind, const CsrView& a, const Options& options,
   } else if (amg()) {
     plan_plain(s);
   }
+  for (std::size_t i = 0; amg() && i < levels_.size(); ++i) {
+    surplus(i);  // allocated here rather than in the first refresh
+    if (i == 0) continue;
+    auto& l = levels_[i];
+    const std::size_t words = (static_cast<std::size_t>(l.nnz) + 31) / 32;
+    l.diagonal.reset(words);
+    cuda_check(cudaMemsetAsync(l.diagonal.get(), 0, words * sizeof(unsigned), s), "memset");
+    launch::mark_diagonals(l.n, l.diag.get(), l.diagonal.get(), s);
+  }
   wait(s);
 }
 
@@ -917,10 +926,11 @@ void Solver::assemble_refresh(const FvPressure& fv, float* values, float* rhs, c
   stream_ = s;
   val_ = values;
   auto& l = levels_[0];
+  const launch::FvFused fused{l.l1.get(), surplus(0), packed_.width, packed_.vals.get(),
+                              packed_.diag.get()};
   launch::fv_pressure_assemble_l1(n_, fv.offsets, fv.faces, fv.sign, fv.adjacent, fv.entry,
                                   l.row_ptr.get(), l.diag.get(), fv.coefficient, fv.flux, values,
-                                  rhs, fv.reference, l.l1.get(), surplus(0), reducer(),
-                                  values_.get(), 0, s);
+                                  rhs, fv.reference, fused, reducer(), values_.get(), 0, s);
   refresh_levels(values, true, s);
 }
 
@@ -944,8 +954,8 @@ void Solver::refresh_levels(const float* val, bool fine_done, cudaStream_t s) {
     p.surplus = i + 1 < levels_.size() ? surplus(i) : nullptr;
     if (i > 0) {
       auto& above = levels_[i - 1];
-      launch::galerkin(l.nnz, above.entry_offsets.get(), above.entries.get(), matrix, l.val.get(),
-                       s);
+      launch::galerkin(l.n, l.nnz, above.entry_offsets.get(), above.entries.get(),
+                       l.diagonal.get(), l.diag.get(), !options_.m_matrix, matrix, l.val.get(), s);
       if (options_.m_matrix) {
         p.offsets = above.member_offsets.get();
         p.members = above.members.get();
@@ -961,7 +971,7 @@ void Solver::refresh_levels(const float* val, bool fine_done, cudaStream_t s) {
                          reducer(), values_.get(), static_cast<int>(i), s);
   }
   const int slots = static_cast<int>(levels_.size());
-  if (packed_.width > 0)
+  if (packed_.width > 0 && !fine_done)
     launch::pack_rows(n_, packed_.width, rows0(), cols0(), levels_[0].diag.get(), val,
                       packed_.vals.get(), packed_.diag.get(), s);
   if (plain_tail_start_ != 0) launch::plain_tail_entries(plain_tail_, s);

@@ -90,6 +90,7 @@ struct DevLevel {
   DArray<int> tail_order, tail_start, tail_source;
   // transfer to level + 1
   DArray<int> aggregate, member_offsets, members, entry_offsets, entries;
+  DArray<unsigned> diagonal;    // a bit per entry: whether it is a diagonal one
 };
 
 // Solve-time measurement: device time of every fine-level smoother sweep (CUDA
