@@ -6,8 +6,7 @@
 // fixed tree; they are fused into the kernel that produces their operand and the
 // last block runs the reference's single-thread scalar update as an epilogue,
 // so a PCG iteration is a handful of launches instead of a dozen.
-#include <cuda_bf16.h>
-
+#include "bf16_rows.cuh"
 #include "common.cuh"
 #include "epilogues.cuh"
 #include "kernels.hpp"
@@ -447,9 +446,8 @@ __global__ void k_level_rows(int n, const int* __restrict__ rows, const int* __r
                              float* vals, const int* __restrict__ offsets,
                              const int* __restrict__ members,
                              const float* __restrict__ fine_surplus, float* __restrict__ inverse,
-                             float* __restrict__ surplus, unsigned short* __restrict__ v16,
-                             float* __restrict__ scale, DeviceReducer red, double* check,
-                             int slot) {
+                             float* __restrict__ surplus, Bf16Store store, DeviceReducer red,
+                             double* check, int slot) {
   pdl_entry();
   double worst = 0;
   ROWS(i, n) {
@@ -473,15 +471,7 @@ __global__ void k_level_rows(int n, const int* __restrict__ rows, const int* __r
     }
     worst = nan_max(worst, diagonal_row(i, rows, diag, vals, inverse, 1));
     if (surplus != nullptr) surplus[i] = row_surplus(i, rows, diag, vals);
-    if (v16 != nullptr) {
-      float most = 0.0f;
-      for (int j = rows[i]; j < rows[i + 1]; ++j) most = fmaxf(most, fabsf(vals[j]));
-      const float s = most > 0.0f ? most : 1.0f;
-      scale[i] = s;
-      const float inv = 1.0f / s;
-      for (int j = rows[i]; j < rows[i + 1]; ++j)
-        v16[j] = __bfloat16_as_ushort(__float2bfloat16_rn(vals[j] * inv));
-    }
+    if (store.scale != nullptr) bf16_store_row(i, vals, store);
   }
   finish_max(as_reducer(red), worst, check, slot);
 }
@@ -864,10 +854,10 @@ void level_rows(int n, const int* rows, const int* diag, float* vals, const Leve
   ++counter;
   if (p.members != nullptr)
     pdl(k_level_rows<true>, blocks(n), kBlock, 0, s, n, rows, diag, vals, p.offsets, p.members,
-        p.fine_surplus, p.inverse, p.surplus, p.v16, p.scale, red, check, slot);
+        p.fine_surplus, p.inverse, p.surplus, p.store, red, check, slot);
   else
     pdl(k_level_rows<false>, blocks(n), kBlock, 0, s, n, rows, diag, vals, p.offsets, p.members,
-        p.fine_surplus, p.inverse, p.surplus, p.v16, p.scale, red, check, slot);
+        p.fine_surplus, p.inverse, p.surplus, p.store, red, check, slot);
 }
 void pcg_step_dot(int n, float* x, float* r, const float* p, const float* q, const int* rows,
                   const float* vals, const float* inv, float* next, DeviceReducer red,

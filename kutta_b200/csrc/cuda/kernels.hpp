@@ -114,18 +114,36 @@ void m_matrix_diagonal(int nf, int nc, const int* offsets, const int* members, c
                        const int* fine_diag, const float* fine, const int* rows, const int* diag,
                        float* coarse, float* surplus, cudaStream_t s);
 
+// A BF16 operator: per entry the value v16 and the column, or, where every column
+// lies within 16 bits of its row, both in one word of `packed` (value in the high
+// half, column - row in the low). Row i's values are scale[i] times these.
+struct Bf16Rows {
+  const int* rows;
+  const int* cols;
+  const unsigned short* v16;
+  const unsigned* packed;
+  const float* scale;
+};
+// The same to be written from FP32 values (v16 or packed).
+struct Bf16Store {
+  const int* rows;
+  const int* cols;
+  unsigned short* v16;
+  unsigned* packed;
+  float* scale;
+};
+
 // A level's row data in one refresh pass: with members the M-matrix diagonal
 // into vals (from the level above's fine_surplus), the inverse L1 diagonal with
 // its invalid flags' maximum in check[slot], and where not null the rows'
-// surplus and BF16 copy (v16, scale).
+// surplus and BF16 copy (store.scale).
 struct LevelRows {
   const int* offsets;
   const int* members;
   const float* fine_surplus;
   float* inverse;
   float* surplus;
-  unsigned short* v16;
-  float* scale;
+  Bf16Store store;
 };
 void level_rows(int n, const int* rows, const int* diag, float* vals, const LevelRows& p,
                 DeviceReducer red, double* check, int slot, cudaStream_t s);
@@ -214,27 +232,24 @@ void reduce_value(ReduceMode mode, int n, const float* x, const float* y, Device
 
 // ---- mixed precision (no reference counterpart) ---------------------------
 // Coarse operator as BF16 times a per-row FP32 scale (max |a_ij|).
-void bf16_pack(int n, const int* rows, const float* vals, unsigned short* v16, float* scale,
-               cudaStream_t s);
-void bf16_smooth(int n, const int* rows, const int* cols, const unsigned short* v16,
-                 const float* scale, const float* x, const float* b, const float* inv, float* next,
-                 const int* status, bool zero_start, cudaStream_t s);
-void bf16_residual(int n, const int* rows, const int* cols, const unsigned short* v16,
-                   const float* scale, const float* x, const float* b, float* r, const int* status,
-                   cudaStream_t s);
+void bf16_pack(int n, const float* vals, const Bf16Store& out, cudaStream_t s);
+// *wide = 1 if a column lies further than 32,767 from its row (*wide is not cleared).
+void bf16_wide(int n, const int* rows, const int* cols, int* wide, cudaStream_t s);
+void bf16_smooth(int n, const Bf16Rows& m, const float* x, const float* b, const float* inv,
+                 float* next, const int* status, bool zero_start, cudaStream_t s);
+void bf16_residual(int n, const Bf16Rows& m, const float* x, const float* b, float* r,
+                   const int* status, cudaStream_t s);
 // Restriction for the mixed V-cycle: plain FP32 sums, four lanes per aggregate.
 void restrict_lanes(int nc, const int* offsets, const int* members, const float* fine,
                     float* coarse, const int* status, cudaStream_t s);
 // K-cycle inner step on a BF16 level: q = A p, p.q and w.p -> scalars[0..3],
 // then alpha (inner_alpha). With copy != null the first step of a cycle: p is
 // copied there, the guard is the parent's status and the level's own starts.
-void bf16_spmv_dot2(int n, const int* rows, const int* cols, const unsigned short* v16,
-                    const float* scale, const float* p, const float* w, float* q, float* copy,
+void bf16_spmv_dot2(int n, const Bf16Rows& m, const float* p, const float* w, float* q, float* copy,
                     DeviceReducer red, float* scalars, const int* parent, int* status,
                     cudaStream_t s);
 // bf16_smooth from x with next.q -> scalars[4..5] and beta (inner_beta).
-void bf16_smooth_dot(int n, const int* rows, const int* cols, const unsigned short* v16,
-                     const float* scale, const float* x, const float* b, const float* inv,
+void bf16_smooth_dot(int n, const Bf16Rows& m, const float* x, const float* b, const float* inv,
                      float* next, const float* q, DeviceReducer red, float* scalars, int* status,
                      cudaStream_t s);
 // inner_first, t.t and b.b -> scalars[4..7] and the exit check (inner_check).

@@ -7,6 +7,7 @@
 #include <algorithm>
 #include <atomic>
 
+#include "bf16_rows.cuh"
 #include "common.cuh"
 #include "kernels.hpp"
 
@@ -27,18 +28,20 @@ __device__ __forceinline__ float bf(unsigned short v) {
 }
 
 // Row scale = max |a_ij| (FP32); stored value = bf16(a_ij / scale).
-__global__ void k_bf16_pack(int n, const int* __restrict__ rows, const float* __restrict__ vals,
-                            unsigned short* __restrict__ v16, float* __restrict__ scale) {
+__global__ void k_bf16_pack(int n, const float* __restrict__ vals, Bf16Store out) {
   pdl_entry();
+  ROWS(i, n) bf16_store_row(i, vals, out);
+}
+
+// Whether a column lies further from its row than a 16-bit offset says.
+__global__ void k_bf16_wide(int n, const int* __restrict__ rows, const int* __restrict__ cols,
+                            int* __restrict__ wide) {
+  pdl_entry();
+  bool found = false;
   ROWS(i, n) {
-    float m = 0.0f;
-    for (int j = rows[i]; j < rows[i + 1]; ++j) m = fmaxf(m, fabsf(vals[j]));
-    const float s = m > 0.0f ? m : 1.0f;
-    scale[i] = s;
-    const float inv = 1.0f / s;
-    for (int j = rows[i]; j < rows[i + 1]; ++j)
-      v16[j] = __bfloat16_as_ushort(__float2bfloat16_rn(vals[j] * inv));
+    for (int j = rows[i]; j < rows[i + 1]; ++j) found = found || abs(cols[j] - i) > 32767;
   }
+  if (found) *wide = 1;
 }
 
 // Coarse rows hold about a dozen entries: four lanes share a row, each taking
@@ -47,31 +50,59 @@ __global__ void k_bf16_pack(int n, const int* __restrict__ rows, const float* __
 constexpr int kLanes = 4;
 constexpr int kRowsPerWarp = 32 / kLanes;
 
-// This lane's share of sum_j a_ij x_j (BF16 values, FP32 accumulation). The
-// row is taken in chunks of kLanes * kPerLane entries; a lane issues all its
-// column and value loads of a chunk before any gather, so each warp keeps
-// several independent loads in flight (these levels are latency-bound).
+// This lane's share of sum_j a_ij x_j (BF16 values, FP32 accumulation) of kR
+// rows (-1: none). A row is taken in chunks of kLanes * kPerLane entries; a lane
+// issues all its loads of a chunk, of kR rows, before any gather. These levels
+// are bound by latency: a wave of warps waits for the row pointers, the entries
+// and the gathered x in turn, so two rows per lane halve the number of waves
+// where there are several (446,000 rows: a residual 11.7 us against 14.5, a
+// sweep 11.1 against 13.7, the restriction to them 14.0 against 16.9); a level
+// that fits in one wave is no faster for it, and the kernels with reductions,
+// whose grid is fixed, slower (16.9 us against 15.9).
+// kPacked: value and column offset in one word (launch::Bf16Rows), which is one
+// load per entry instead of two and 4 bytes instead of 6.
 constexpr int kPerLane = 3;
-__device__ __forceinline__ float bf16_row_part(int i, int lane, const int* __restrict__ rows,
-                                               const int* __restrict__ cols,
-                                               const unsigned short* __restrict__ v16,
-                                               const float* __restrict__ x) {
-  float acc = 0.0f;
-  const int end = rows[i + 1];
-  for (int j0 = rows[i] + lane; j0 < end; j0 += kLanes * kPerLane) {
-    int c[kPerLane];
-    float a[kPerLane];
+template <bool kPacked, int kR>
+__device__ __forceinline__ void bf16_row_parts(const int (&row)[kR], int lane,
+                                               const launch::Bf16Rows& m,
+                                               const float* __restrict__ x, float (&acc)[kR]) {
+  int at[kR], end[kR];
 #pragma unroll
-    for (int u = 0; u < kPerLane; ++u) {
-      const int j = j0 + u * kLanes;
-      c[u] = j < end ? cols[j] : -1;
-      a[u] = j < end ? bf(v16[j]) : 0.0f;
-    }
-#pragma unroll
-    for (int u = 0; u < kPerLane; ++u)
-      if (c[u] >= 0) acc = fmaf(a[u], x[c[u]], acc);
+  for (int r = 0; r < kR; ++r) {
+    at[r] = row[r] >= 0 ? m.rows[row[r]] + lane : 0;
+    end[r] = row[r] >= 0 ? m.rows[row[r] + 1] : 0;
+    acc[r] = 0.0f;
   }
-  return acc;
+  while (at[0] < end[0] || at[kR - 1] < end[kR - 1]) {
+    int c[kR][kPerLane];
+    float a[kR][kPerLane], v[kR][kPerLane];
+#pragma unroll
+    for (int r = 0; r < kR; ++r)
+#pragma unroll
+      for (int u = 0; u < kPerLane; ++u) {
+        const int j = at[r] + u * kLanes;
+        const bool in = j < end[r];
+        if constexpr (kPacked) {
+          const unsigned e = in ? __ldg(m.packed + j) : 0;
+          c[r][u] = in ? row[r] + static_cast<short>(e & 0xffffu) : -1;
+          a[r][u] = __uint_as_float(e & 0xffff0000u);
+        } else {
+          c[r][u] = in ? __ldg(m.cols + j) : -1;
+          a[r][u] = in ? bf(__ldg(m.v16 + j)) : 0.0f;
+        }
+      }
+#pragma unroll
+    for (int r = 0; r < kR; ++r)
+#pragma unroll
+      for (int u = 0; u < kPerLane; ++u) v[r][u] = c[r][u] >= 0 ? x[c[r][u]] : 0.0f;
+#pragma unroll
+    for (int r = 0; r < kR; ++r) {
+#pragma unroll
+      for (int u = 0; u < kPerLane; ++u)
+        if (c[r][u] >= 0) acc[r] = fmaf(a[r][u], v[r][u], acc[r]);
+      at[r] += kLanes * kPerLane;
+    }
+  }
 }
 // Sum over the row's four lanes, in lane 0 (every lane of the warp calls it).
 __device__ __forceinline__ float row_total(float v) {
@@ -80,31 +111,62 @@ __device__ __forceinline__ float row_total(float v) {
   return v;
 }
 
-// Visits rows kLanes lanes at a time; the loop bound is uniform across a warp,
-// so every lane reaches the shuffles. body(i, lane, valid).
-template <class Body>
+// Visits rows kLanes lanes at a time, kR rows (1 or 2) per group of lanes; the
+// loop bound is uniform across a warp, so every lane reaches the shuffles.
+// body(rows, lane), a row of -1 for none.
+template <int kR, class Body>
 __device__ __forceinline__ void for_rows(int n, Body body) {
   const int lane = threadIdx.x & (kLanes - 1);
   const int warp = static_cast<int>((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   const int warps = static_cast<int>((gridDim.x * blockDim.x) >> 5);
-  for (int row0 = warp * kRowsPerWarp; row0 < n; row0 += warps * kRowsPerWarp) {
-    const int i = row0 + static_cast<int>((threadIdx.x & 31) / kLanes);
-    body(i, lane, i < n);
+  for (int row0 = warp * kR * kRowsPerWarp; row0 < n; row0 += warps * kR * kRowsPerWarp) {
+    int rows[kR];
+#pragma unroll
+    for (int r = 0; r < kR; ++r) {
+      const int i = row0 + r * kRowsPerWarp + static_cast<int>((threadIdx.x & 31) / kLanes);
+      rows[r] = i < n ? i : -1;
+    }
+    body(rows, lane);
   }
 }
+// Rows above which the row kernels without a reduction take two per group: one
+// wave of single rows (148 SMs x 2,048 threads / kLanes).
+constexpr int kPairRows = 148 * 2048 / kLanes;
 
 // A reduction's grid stays within the partials buffer (kMaxBlocks blocks).
 inline int lanes_grid(int n, bool reduction) {
-  const long long blocks = (static_cast<long long>(n) * kLanes + kBlock - 1) / kBlock;
+  const long long rows = reduction || n <= kPairRows ? n : (n + 1LL) / 2;
+  const long long blocks = (rows * kLanes + kBlock - 1) / kBlock;
   const long long cap = reduction ? static_cast<long long>(kMaxBlocks) : (1LL << 30);
   return static_cast<int>(std::max(1LL, std::min(blocks, cap)));
 }
 
+// What a group's first lane needs besides the row's sum, loaded before it rather
+// than a memory latency after it.
+template <int kR>
+struct RowData {
+  float scale[kR], b[kR], inv[kR], x[kR];
+  __device__ __forceinline__ RowData(const int (&rows)[kR], int lane, const launch::Bf16Rows& m,
+                                     const float* __restrict__ right,
+                                     const float* __restrict__ inverse,
+                                     const float* __restrict__ iterate) {
+#pragma unroll
+    for (int r = 0; r < kR; ++r) {
+      const bool mine = rows[r] >= 0 && lane == 0;
+      scale[r] = mine ? m.scale[rows[r]] : 0.0f;
+      b[r] = mine ? right[rows[r]] : 0.0f;
+      inv[r] = mine && inverse ? inverse[rows[r]] : 0.0f;
+      x[r] = mine && iterate ? iterate[rows[r]] : 0.0f;
+    }
+  }
+  __device__ __forceinline__ float sweep(int r, float total) const {
+    return x[r] + (2.0f / 3.0f) * inv[r] * (b[r] - scale[r] * total);
+  }
+};
+
 // Damped L1-Jacobi sweep with the BF16 operator (FP32 accumulation).
-template <bool kZero>
-__global__ void k_bf16_smooth(int n, const int* __restrict__ rows, const int* __restrict__ cols,
-                              const unsigned short* __restrict__ v16,
-                              const float* __restrict__ scale, const float* __restrict__ x,
+template <bool kZero, bool kPacked, int kR>
+__global__ void k_bf16_smooth(int n, launch::Bf16Rows m, const float* __restrict__ x,
                               const float* __restrict__ b, const float* __restrict__ inv,
                               float* __restrict__ next, const int* __restrict__ status) {
   pdl_entry();
@@ -113,50 +175,80 @@ __global__ void k_bf16_smooth(int n, const int* __restrict__ rows, const int* __
     ROWS(i, n) next[i] = (2.0f / 3.0f) * inv[i] * b[i];
     return;
   }
-  for_rows(n, [&](int i, int lane, bool valid) {
-    const float acc = row_total(valid ? bf16_row_part(i, lane, rows, cols, v16, x) : 0.0f);
-    if (valid && lane == 0) next[i] = x[i] + (2.0f / 3.0f) * inv[i] * (b[i] - scale[i] * acc);
+  for_rows<kR>(n, [&](const int (&rows)[kR], int lane) {
+    const RowData<kR> d(rows, lane, m, b, inv, x);
+    float acc[kR];
+    bf16_row_parts<kPacked, kR>(rows, lane, m, x, acc);
+#pragma unroll
+    for (int r = 0; r < kR; ++r) {
+      const float total = row_total(acc[r]);
+      if (rows[r] >= 0 && lane == 0) next[rows[r]] = d.sweep(r, total);
+    }
   });
 }
 
-__global__ void k_bf16_residual(int n, const int* __restrict__ rows, const int* __restrict__ cols,
-                                const unsigned short* __restrict__ v16,
-                                const float* __restrict__ scale, const float* __restrict__ x,
+template <bool kPacked, int kR>
+__global__ void k_bf16_residual(int n, launch::Bf16Rows m, const float* __restrict__ x,
                                 const float* __restrict__ b, float* __restrict__ r,
                                 const int* __restrict__ status) {
   pdl_entry();
   if (status[0] != 0) return;
-  for_rows(n, [&](int i, int lane, bool valid) {
-    const float acc = row_total(valid ? bf16_row_part(i, lane, rows, cols, v16, x) : 0.0f);
-    if (valid && lane == 0) r[i] = b[i] - scale[i] * acc;
+  for_rows<kR>(n, [&](const int (&rows)[kR], int lane) {
+    const RowData<kR> d(rows, lane, m, b, nullptr, nullptr);
+    float acc[kR];
+    bf16_row_parts<kPacked, kR>(rows, lane, m, x, acc);
+#pragma unroll
+    for (int q = 0; q < kR; ++q) {
+      const float total = row_total(acc[q]);
+      if (rows[q] >= 0 && lane == 0) r[rows[q]] = d.b[q] - d.scale[q] * total;
+    }
   });
 }
 
 // Coarse b = sum of the fine residual over each aggregate's members, four
 // lanes per aggregate with their member loads batched like the row kernels.
+template <int kR>
 __global__ void k_restrict_lanes(int nc, const int* __restrict__ offsets,
                                  const int* __restrict__ members, const float* __restrict__ fine,
                                  float* __restrict__ coarse, const int* __restrict__ status) {
   pdl_entry();
   if (status[0] != 0) return;
-  for_rows(nc, [&](int g, int lane, bool valid) {
-    float acc = 0.0f;
-    if (valid) {
-      const int end = offsets[g + 1];
-      for (int j0 = offsets[g] + lane; j0 < end; j0 += kLanes * kPerLane) {
-        int m[kPerLane];
+  for_rows<kR>(nc, [&](const int (&groups)[kR], int lane) {
+    int at[kR], end[kR];
+    float acc[kR];
+#pragma unroll
+    for (int r = 0; r < kR; ++r) {
+      at[r] = groups[r] >= 0 ? offsets[groups[r]] + lane : 0;
+      end[r] = groups[r] >= 0 ? offsets[groups[r] + 1] : 0;
+      acc[r] = 0.0f;
+    }
+    while (at[0] < end[0] || at[kR - 1] < end[kR - 1]) {
+      int m[kR][kPerLane];
+      float v[kR][kPerLane];
+#pragma unroll
+      for (int r = 0; r < kR; ++r)
 #pragma unroll
         for (int u = 0; u < kPerLane; ++u) {
-          const int j = j0 + u * kLanes;
-          m[u] = j < end ? members[j] : -1;
+          const int j = at[r] + u * kLanes;
+          m[r][u] = j < end[r] ? members[j] : -1;
         }
 #pragma unroll
+      for (int r = 0; r < kR; ++r)
+#pragma unroll
+        for (int u = 0; u < kPerLane; ++u) v[r][u] = m[r][u] >= 0 ? fine[m[r][u]] : 0.0f;
+#pragma unroll
+      for (int r = 0; r < kR; ++r) {
+#pragma unroll
         for (int u = 0; u < kPerLane; ++u)
-          if (m[u] >= 0) acc += fine[m[u]];
+          if (m[r][u] >= 0) acc[r] += v[r][u];
+        at[r] += kLanes * kPerLane;
       }
     }
-    acc = row_total(acc);
-    if (valid && lane == 0) coarse[g] = acc;
+#pragma unroll
+    for (int r = 0; r < kR; ++r) {
+      const float total = row_total(acc[r]);
+      if (groups[r] >= 0 && lane == 0) coarse[groups[r]] = total;
+    }
   });
 }
 
@@ -208,10 +300,8 @@ __device__ __forceinline__ void inner_beta(float* scalars, int* status) {
 // kFirst: p is the level's z, copied to `copy` on the way, `status` is the
 // parent's, and the level's own status starts here (2, the plain cycle, while
 // the parent has stopped); otherwise status is the level's own.
-template <bool kFirst>
-__global__ void k_bf16_spmv_dot2(int n, const int* __restrict__ rows, const int* __restrict__ cols,
-                                 const unsigned short* __restrict__ v16,
-                                 const float* __restrict__ scale, const float* __restrict__ p,
+template <bool kFirst, bool kPacked>
+__global__ void k_bf16_spmv_dot2(int n, launch::Bf16Rows m, const float* __restrict__ p,
                                  const float* __restrict__ w, float* __restrict__ q,
                                  float* __restrict__ copy, DeviceReducer red, float* scalars,
                                  const int* status, int* own) {
@@ -221,14 +311,19 @@ __global__ void k_bf16_spmv_dot2(int n, const int* __restrict__ rows, const int*
     return;
   }
   double a = 0.0, b = 0.0;
-  for_rows(n, [&](int i, int lane, bool valid) {
-    const float acc = row_total(valid ? bf16_row_part(i, lane, rows, cols, v16, p) : 0.0f);
-    if (valid && lane == 0) {
-      const float qi = scale[i] * acc, pi = p[i];
-      q[i] = qi;
-      if (kFirst) copy[i] = pi;
+  for_rows<1>(n, [&](const int (&rows)[1], int lane) {
+    const RowData<1> d(rows, lane, m, w, nullptr, p);
+    float acc[1];
+    bf16_row_parts<kPacked, 1>(rows, lane, m, p, acc);
+#pragma unroll
+    for (int r = 0; r < 1; ++r) {
+      const float total = row_total(acc[r]);
+      if (rows[r] < 0 || lane != 0) continue;
+      const float qi = d.scale[r] * total, pi = d.x[r];
+      q[rows[r]] = qi;
+      if (kFirst) copy[rows[r]] = pi;
       a += static_cast<double>(pi) * static_cast<double>(qi);
-      b += static_cast<double>(w[i]) * static_cast<double>(pi);
+      b += static_cast<double>(d.b[r]) * static_cast<double>(pi);
     }
   });
   if (!finish_dot2(red, a, b, scalars, 0)) return;
@@ -238,22 +333,25 @@ __global__ void k_bf16_spmv_dot2(int n, const int* __restrict__ rows, const int*
 
 // The last sweep of the second inner cycle with z.q -> scalars[4..5] (q = A p of
 // the first) and beta.
-__global__ void k_bf16_smooth_dot(int n, const int* __restrict__ rows,
-                                  const int* __restrict__ cols,
-                                  const unsigned short* __restrict__ v16,
-                                  const float* __restrict__ scale, const float* __restrict__ x,
+template <bool kPacked>
+__global__ void k_bf16_smooth_dot(int n, launch::Bf16Rows m, const float* __restrict__ x,
                                   const float* __restrict__ b, const float* __restrict__ inv,
                                   float* __restrict__ next, const float* __restrict__ q,
                                   DeviceReducer red, float* scalars, int* status) {
   pdl_entry();
   if (status[0] != 0) return;
   double a = 0.0;
-  for_rows(n, [&](int i, int lane, bool valid) {
-    const float acc = row_total(valid ? bf16_row_part(i, lane, rows, cols, v16, x) : 0.0f);
-    if (valid && lane == 0) {
-      const float z = x[i] + (2.0f / 3.0f) * inv[i] * (b[i] - scale[i] * acc);
-      next[i] = z;
-      a += static_cast<double>(z) * static_cast<double>(q[i]);
+  for_rows<1>(n, [&](const int (&rows)[1], int lane) {
+    const RowData<1> d(rows, lane, m, b, inv, x);
+    float acc[1];
+    bf16_row_parts<kPacked, 1>(rows, lane, m, x, acc);
+#pragma unroll
+    for (int r = 0; r < 1; ++r) {
+      const float total = row_total(acc[r]);
+      if (rows[r] < 0 || lane != 0) continue;
+      const float z = d.sweep(r, total);
+      next[rows[r]] = z;
+      a += static_cast<double>(z) * static_cast<double>(q[rows[r]]);
     }
   });
   __shared__ double shared[32];
@@ -776,50 +874,56 @@ __global__ void k_narrow(int n, const double* __restrict__ y, float* __restrict_
 
 namespace launch {
 
-void bf16_pack(int n, const int* rows, const float* vals, unsigned short* v16, float* scale,
-               cudaStream_t s) {
+void bf16_pack(int n, const float* vals, const Bf16Store& out, cudaStream_t s) {
   if (n <= 0) return;
   ++counter;
-  pdl(k_bf16_pack, rows_grid(n), kBlock, 0, s, n, rows, vals, v16, scale);
+  pdl(k_bf16_pack, rows_grid(n), kBlock, 0, s, n, vals, out);
 }
-void bf16_smooth(int n, const int* rows, const int* cols, const unsigned short* v16,
-                 const float* scale, const float* x, const float* b, const float* inv, float* next,
-                 const int* status, bool zero_start, cudaStream_t s) {
+void bf16_wide(int n, const int* rows, const int* cols, int* wide, cudaStream_t s) {
+  if (n <= 0) return;
+  ++counter;
+  pdl(k_bf16_wide, rows_grid(n), kBlock, 0, s, n, rows, cols, wide);
+}
+void bf16_smooth(int n, const Bf16Rows& m, const float* x, const float* b, const float* inv,
+                 float* next, const int* status, bool zero_start, cudaStream_t s) {
   if (n <= 0) return;
   ++counter;
   if (zero_start)
-    pdl(k_bf16_smooth<true>, rows_grid(n), kBlock, 0, s, n, rows, cols, v16, scale, x, b, inv, next, status);
+    pdl(k_bf16_smooth<true, false, 1>, rows_grid(n), kBlock, 0, s, n, m, x, b, inv, next, status);
   else
-    pdl(k_bf16_smooth<false>, lanes_grid(n, false), kBlock, 0, s, n, rows, cols, v16, scale, x, b, inv, next, status);
+    pdl(m.packed != nullptr
+            ? (n > kPairRows ? k_bf16_smooth<false, true, 2> : k_bf16_smooth<false, true, 1>)
+            : (n > kPairRows ? k_bf16_smooth<false, false, 2> : k_bf16_smooth<false, false, 1>),
+        lanes_grid(n, false), kBlock, 0, s, n, m, x, b, inv, next, status);
 }
 void restrict_lanes(int nc, const int* offsets, const int* members, const float* fine,
                     float* coarse, const int* status, cudaStream_t s) {
   if (nc <= 0) return;
   ++counter;
-  pdl(k_restrict_lanes, lanes_grid(nc, false), kBlock, 0, s, nc, offsets, members, fine, coarse,
-                                                            status);
+  pdl(nc > kPairRows ? k_restrict_lanes<2> : k_restrict_lanes<1>, lanes_grid(nc, false), kBlock, 0,
+      s, nc, offsets, members, fine, coarse, status);
 }
-void bf16_spmv_dot2(int n, const int* rows, const int* cols, const unsigned short* v16,
-                    const float* scale, const float* p, const float* w, float* q, float* copy,
+void bf16_spmv_dot2(int n, const Bf16Rows& m, const float* p, const float* w, float* q, float* copy,
                     DeviceReducer red, float* scalars, const int* parent, int* status,
                     cudaStream_t s) {
   if (n <= 0) return;
   ++counter;
+  const auto go = [&](auto kernel, const int* guard) {
+    pdl(kernel, lanes_grid(n, true), kBlock, 0, s, n, m, p, w, q, copy, red, scalars, guard, status);
+  };
+  const bool packed = m.packed != nullptr;
   if (copy != nullptr)
-    pdl(k_bf16_spmv_dot2<true>, lanes_grid(n, true), kBlock, 0, s, n, rows, cols, v16, scale, p, w,
-        q, copy, red, scalars, parent, status);
+    go(packed ? k_bf16_spmv_dot2<true, true> : k_bf16_spmv_dot2<true, false>, parent);
   else
-    pdl(k_bf16_spmv_dot2<false>, lanes_grid(n, true), kBlock, 0, s, n, rows, cols, v16, scale, p, w,
-        q, copy, red, scalars, static_cast<const int*>(status), status);
+    go(packed ? k_bf16_spmv_dot2<false, true> : k_bf16_spmv_dot2<false, false>, status);
 }
-void bf16_smooth_dot(int n, const int* rows, const int* cols, const unsigned short* v16,
-                     const float* scale, const float* x, const float* b, const float* inv,
+void bf16_smooth_dot(int n, const Bf16Rows& m, const float* x, const float* b, const float* inv,
                      float* next, const float* q, DeviceReducer red, float* scalars, int* status,
                      cudaStream_t s) {
   if (n <= 0) return;
   ++counter;
-  pdl(k_bf16_smooth_dot, lanes_grid(n, true), kBlock, 0, s, n, rows, cols, v16, scale, x, b, inv,
-      next, q, red, scalars, status);
+  pdl(m.packed != nullptr ? k_bf16_smooth_dot<true> : k_bf16_smooth_dot<false>, lanes_grid(n, true),
+      kBlock, 0, s, n, m, x, b, inv, next, q, red, scalars, status);
 }
 void inner_first_dot(int n, const float* b, const float* p, const float* q, float* x, float* t,
                      float* scalars, int* status, DeviceReducer red, cudaStream_t s) {
@@ -827,13 +931,13 @@ void inner_first_dot(int n, const float* b, const float* p, const float* q, floa
   ++counter;
   pdl(k_inner_first_dot, grid_for(n), kBlock, 0, s, n, b, p, q, x, t, scalars, status, red);
 }
-void bf16_residual(int n, const int* rows, const int* cols, const unsigned short* v16,
-                   const float* scale, const float* x, const float* b, float* r, const int* status,
-                   cudaStream_t s) {
+void bf16_residual(int n, const Bf16Rows& m, const float* x, const float* b, float* r,
+                   const int* status, cudaStream_t s) {
   if (n <= 0) return;
   ++counter;
-  pdl(k_bf16_residual, lanes_grid(n, false), kBlock, 0, s, n, rows, cols, v16, scale, x, b, r,
-                                                          status);
+  pdl(m.packed != nullptr ? (n > kPairRows ? k_bf16_residual<true, 2> : k_bf16_residual<true, 1>)
+                          : (n > kPairRows ? k_bf16_residual<false, 2> : k_bf16_residual<false, 1>),
+      lanes_grid(n, false), kBlock, 0, s, n, m, x, b, r, status);
 }
 void dense_inverse(int n, const int* rows, const int* cols, const float* vals, double* lower,
                    double* inverse, double* error, cudaStream_t s, double* ratio) {

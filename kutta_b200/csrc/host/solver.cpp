@@ -136,7 +136,11 @@ Solver::Solver(Kind kind, const CsrView& a, const Options& options,
     for (std::size_t i = 1; i < levels_.size(); ++i) {
       auto& l = levels_[i];
       if (options_.coarse_bf16) {
-        l.v16.reset(static_cast<std::size_t>(l.nnz));
+        // The cluster tail reads columns and values apart.
+        if (!options_.fused_tail && near_columns(l, s))
+          l.packed16.reset(static_cast<std::size_t>(l.nnz));
+        else
+          l.v16.reset(static_cast<std::size_t>(l.nnz));
         l.scale.reset(static_cast<std::size_t>(l.n));
       }
     }
@@ -275,6 +279,18 @@ void Solver::plan_plain(cudaStream_t s) {
   plain_tail_start_ = start;
 }
 
+// Whether every column of the level lies within 16 bits of its row.
+bool Solver::near_columns(const DevLevel& l, cudaStream_t s) {
+  DArray<int> wide(1);
+  int found = 0;
+  cuda_check(cudaMemsetAsync(wide.get(), 0, sizeof(int), s), "memset");
+  launch::bf16_wide(l.n, l.row_ptr.get(), l.col.get(), wide.get(), s);
+  cuda_check(cudaMemcpyAsync(&found, wide.get(), sizeof(int), cudaMemcpyDeviceToHost, s),
+             "readback");
+  wait(s);
+  return found == 0;
+}
+
 // The packed rows' pattern: each row's off-diagonal column offsets in column
 // order, padded with 0 to the width (4 or 8). Left empty (the CSR kernels
 // serve) when a row has more than 8 off-diagonal entries or an offset does
@@ -398,8 +414,7 @@ void Solver::prepare_mixed(cudaStream_t s, int slot, bool packed) {
   cuda_check(cudaMemsetAsync(error, 0, 2 * sizeof(double), s), "memset");
   for (std::size_t i = 1; i < levels_.size(); ++i) {
     auto& l = levels_[i];
-    if (l.v16.allocated() && !packed)
-      launch::bf16_pack(l.n, l.row_ptr.get(), l.val.get(), l.v16.get(), l.scale.get(), s);
+    if (l.bf16() && !packed) launch::bf16_pack(l.n, l.val.get(), l.bf16_store(), s);
     if (dense(l))
       launch::dense_inverse(l.n, l.row_ptr.get(), l.col.get(), l.val.get(), l.dense_lower.get(),
                             l.dense_inverse.get(), error, s, error + 1);
@@ -549,11 +564,10 @@ void Solver::smooth(DevLevel& l, const int* rows, const int* cols, const float* 
                    (with_dots ? 20.0 : 16.0) * l.n;
     if (timed) event_bytes_.push_back(bytes);
     if (inner_dot_ == &l && !zero_start && sweep + 1 == sweeps)
-      launch::bf16_smooth_dot(l.n, rows, cols, l.v16.get(), l.scale.get(), x, b, l.l1.get(), l.r,
-                              l.q.get(), reducer(), l.scalars.get(), l.status.get(), stream_);
-    else if (l.v16.allocated())
-      launch::bf16_smooth(l.n, rows, cols, l.v16.get(), l.scale.get(), x, b, l.l1.get(), l.r,
-                          status, zero, stream_);
+      launch::bf16_smooth_dot(l.n, l.bf16_rows(), x, b, l.l1.get(), l.r, l.q.get(), reducer(),
+                              l.scalars.get(), l.status.get(), stream_);
+    else if (l.bf16())
+      launch::bf16_smooth(l.n, l.bf16_rows(), x, b, l.l1.get(), l.r, status, zero, stream_);
     else if (packed_rows)
       launch::packed_smooth_dot2(l.n, packed(), x, b, l.l1.get(), l.r, q_, reducer(),
                                  scalars_.get(), 4, status_.get(), Epilogue::PcgBetaFlexible,
@@ -608,9 +622,8 @@ void Solver::cycle(std::size_t index, const float* b, float*& x, const int* stat
     }
   } else {
     smooth(l, rows, cols, vals, b, x, options_.pre_sweeps, true, status, swept);
-    if (l.v16.allocated())
-      launch::bf16_residual(l.n, rows, cols, l.v16.get(), l.scale.get(), x, b, l.r, status,
-                            stream_);
+    if (l.bf16())
+      launch::bf16_residual(l.n, l.bf16_rows(), x, b, l.r, status, stream_);
     else if (index == 0 && packed_.width > 0)
       launch::packed_residual(l.n, packed(), x, b, l.r, status, stream_);
     else if (l.staged)
@@ -679,14 +692,14 @@ void Solver::inner(std::size_t index, const int* parent) {
 
   // A BF16 level (mixed precision, SPD) uses its BF16 operator, with the
   // reductions fused into the kernels that produce their operands.
-  const bool bf16 = l.v16.allocated() && spd;
+  const bool bf16 = l.bf16() && spd;
   const double bf16_bytes = 6.0 * l.nnz + 4.0 * (n + 1) + 16.0 * n;
 
   cycle(index, l.b.get(), l.z, parent);
   if (bf16) {
     // The scalar steps ride on the reductions that produce their operands.
-    launch::bf16_spmv_dot2(n, rows, cols, l.v16.get(), l.scale.get(), l.z, l.b.get(), q, p,
-                           reducer(), sc, parent, st, stream_);
+    launch::bf16_spmv_dot2(n, l.bf16_rows(), l.z, l.b.get(), q, p, reducer(), sc, parent, st,
+                           stream_);
     tally(bf16_bytes + 4.0 * n);
     launch::inner_first_dot(n, l.b.get(), p, q, l.x, t, sc, st, reducer(), stream_);
     tally(24.0 * n);
@@ -715,8 +728,7 @@ void Solver::inner(std::size_t index, const int* parent) {
   launch::direction(n, l.z, p, sc, st, stream_);
   tally(12.0 * n);
   if (bf16) {
-    launch::bf16_spmv_dot2(n, rows, cols, l.v16.get(), l.scale.get(), p, t, q, nullptr, reducer(),
-                           sc, st, st, stream_);
+    launch::bf16_spmv_dot2(n, l.bf16_rows(), p, t, q, nullptr, reducer(), sc, st, st, stream_);
     tally(bf16_bytes);
   } else {
     launch::spmv(n, rows, cols, vals, p, q, st, stream_);
@@ -961,8 +973,7 @@ void Solver::refresh_levels(const float* val, bool fine_done, cudaStream_t s) {
         p.members = above.members.get();
         p.fine_surplus = surplus(i - 1);
       }
-      p.v16 = l.v16.get();
-      p.scale = l.scale.get();
+      if (l.bf16()) p.store = l.bf16_store();
       matrix = l.val.get();
     }
     // Without members the pass writes no values, so the caller's stay untouched.

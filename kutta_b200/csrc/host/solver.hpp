@@ -80,7 +80,15 @@ struct DevLevel {
   float* z = nullptr;
   // Mixed precision: BF16 operator with row scales; dense FP64 inverse.
   DArray<unsigned short> v16;
+  DArray<unsigned> packed16;   // or value and column offset in one word
   DArray<float> scale;
+  bool bf16() const { return scale.allocated(); }
+  launch::Bf16Rows bf16_rows() const {
+    return {row_ptr.get(), col.get(), v16.get(), packed16.get(), scale.get()};
+  }
+  launch::Bf16Store bf16_store() const {
+    return {row_ptr.get(), col.get(), v16.get(), packed16.get(), scale.get()};
+  }
   DArray<double> dense_lower, dense_inverse;
   // The plain solve's row kernels form the row's products with all threads of a
   // block (launch::staged_smooth) instead of a thread per row.
@@ -159,6 +167,7 @@ class Solver {
   launch::TailPlan tail_{};
   // The plain V-cycle's choice of row kernels per level, and its smallest
   // levels (>= plain_tail_start_, 0: none) in one block.
+  static bool near_columns(const DevLevel& l, cudaStream_t s);
   void plan_plain(cudaStream_t s);
   static std::vector<int> row_pointers(const DevLevel& l, cudaStream_t s);
   std::size_t plain_tail_start_ = 0;
@@ -207,7 +216,7 @@ class Solver {
   // request flag set around apply() when they do.
   bool can_fuse_dots() const {
     return amg() && variable() && !nullspace_ && levels_.size() > 1 && options_.post_sweeps >= 1 &&
-           !levels_[0].v16.allocated() &&
+           !levels_[0].bf16() &&
            !(learned_ != nullptr && (learned_mode_ & kLearnedCycle));
   }
   bool fuse_dots_ = false;
