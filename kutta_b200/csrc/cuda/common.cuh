@@ -225,18 +225,14 @@ __device__ __forceinline__ void neumaier_term(float& sum, float& error, float te
   sum = next;
 }
 
-// The next float above a finite v: a float's bits order as integers within each
-// sign, so one up or, below zero, one down; the smallest subnormal above a zero.
-__device__ __forceinline__ float next_up(float v) {
-  const int bits = __float_as_int(v);
-  return v == 0.0f ? __int_as_float(1) : __int_as_float(bits + (bits >> 31 | 1));
-}
-// Upward-rounded sums, src/kutta/kernels/prelude.h:82-100.
+// Upward-rounded sums, src/kutta/kernels/prelude.h:82-100: the float above the
+// nearest one where the TwoSum error is positive, which is the sum rounded up; a
+// sum that rounds to -infinity has no error (NaN) and stays. One rounding
+// instruction instead of the error, 4 instead of 13: the rows' chains of these
+// bound the refresh's row passes.
 __device__ __forceinline__ float add_up(float a, float b) {
-  const float sum = a + b;
-  const float part = sum - a;
-  const float error = (a - (sum - part)) + (b - part);
-  return error > 0.0f ? next_up(sum) : sum;
+  const float up = __fadd_ru(a, b);
+  return up == -3.402823466e38f ? a + b : up;
 }
 struct UpperSum {
   float sum, error;

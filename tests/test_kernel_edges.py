@@ -1,0 +1,167 @@
+"""Kernels at the sizes where they change over: assembly rows at and above what
+a thread holds in registers, the dense inverse around its warps' and slices'
+edges, mixed coarse rows with and without columns in 16-bit reach and above the
+two-rows rule, and the learned stage's backward at ragged row counts."""
+import numpy as np
+import pytest
+
+from kutta_b200 import harness
+from kutta_b200 import linalg as L
+from oracle import fv
+
+pytestmark = pytest.mark.gpu
+M = L.OperatorStructure.SymmetricMMatrix
+
+
+def _bits(a):
+    return np.ascontiguousarray(a).view(np.uint32)
+
+
+def _random_rows(n, degree, seed):
+    """A symmetric M-matrix whose rows have up to `degree` off-diagonals."""
+    rng = np.random.default_rng(seed)
+    load = np.zeros(n, int)
+    pairs = set()
+    for i in range(n - 1):
+        for j in {i + 1, *rng.integers(0, n, degree)}:
+            p = (min(i, j), max(i, j))
+            if i != j and p not in pairs and load[i] < degree and load[j] < degree:
+                pairs.add(p)
+                load[[i, j]] += 1
+    i, j = np.array(sorted(pairs)).T
+    w = np.exp(rng.uniform(-3, 0, len(i))).astype(np.float32).astype(np.float64)
+    row = np.concatenate([i, j, np.arange(n)])
+    col = np.concatenate([j, i, np.arange(n)])
+    total = np.bincount(np.concatenate([i, j]), np.concatenate([w, w]), n) * 1.01 + 1e-3
+    val = np.concatenate([-w, -w, np.nextafter(total.astype(np.float32), np.float32(np.inf))])
+    return _system(row, col, val, n, rng)
+
+
+def _system(row, col, val, n, rng):
+    order = np.lexsort((col, row))
+    row, col, val = row[order], col[order].astype(np.int32), val[order]
+    row_ptr = np.concatenate([[0], np.cumsum(np.bincount(row, minlength=n))]).astype(np.int32)
+    diag = np.nonzero(row == col)[0].astype(np.int32)
+    return harness.HostSystem(row_ptr, col, diag, val.astype(np.float64),
+                              rng.standard_normal(n).astype(np.float32))
+
+
+def _device_fv(c):
+    import torch
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()  # noqa: E731
+    return L.FvPressure(t(c.offsets), t(c.faces), t(c.sign), t(c.adjacent), t(c.entry),
+                        t(c.coefficient), t(c.flux), int(c.reference))
+
+
+@pytest.mark.parametrize("reference", [-1, 100])
+@pytest.mark.parametrize("degree, duplicate", [(3, 0.0), (4, 0.3), (5, 0.1), (6, 0.2), (8, 0.0)])
+def test_assembly_rows_match_oracle_and_refresh(cuda, degree, duplicate, reference):
+    """Faces below, at and above six per row, some sharing an entry, some
+    entries without a face (they keep their value): bit for bit the oracle's
+    values, and with the refresh fused the separate refresh's levels."""
+    import torch
+    s = _random_rows(3000, degree, degree)
+    c = harness.fv_faces(s.row_ptr, s.col, s.diag, seed=3, duplicate=duplicate, boundary=1.0,
+                         reference=reference)
+    # Every 50th internal face becomes a wall face of both its cells, so that
+    # their entries may be left without one.
+    slots = np.isin(c.faces, np.arange(0, c.internal, 50))
+    c.adjacent[slots] = -1
+    start = s.val.astype(np.float32)
+    v, r = start.copy(), np.zeros(s.n, np.float32)
+    fv.oracle_assemble(c, v, r)
+    a = L.upload(s)
+    rhs = torch.zeros(s.n, device="cuda")
+    L.fv_pressure_assemble(a, _device_fv(c), rhs)
+    assert np.array_equal(_bits(a.val.cpu().numpy()), _bits(v))
+    assert np.array_equal(_bits(rhs.cpu().numpy()), _bits(r))
+    levels = []
+    for fused in (False, True):
+        a = L.upload(s)
+        solver = L.make_amg_solver(L.SolverKind.AmgPcg, s, L.AmgOptions(structure=M))
+        rhs = torch.zeros(s.n, device="cuda")
+        if fused:
+            solver.assemble_refresh(a, _device_fv(c), rhs)
+        else:
+            L.fv_pressure_assemble(a, _device_fv(c), rhs)
+            solver.refresh(a)
+        levels.append([a.val.cpu().numpy(), rhs.cpu().numpy(),
+                       *(x for lv in solver.levels() for x in lv[3:5])])
+        x = torch.zeros(s.n, device="cuda")
+        solver.solve(a, x, rhs, L.SolveControl(1e-5, 1e-30, 300))
+        levels[-1].append(x.cpu().numpy())  # reads the packed rows
+    for one, two in zip(*levels):
+        assert np.array_equal(_bits(one), _bits(two))
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 63, 64, 65, 95, 96, 97, 111, 112])
+def test_dense_inverse_edges(cuda, n):
+    """Against numpy in FP64: |error| <= n eps cond |inverse| to first order for
+    an elimination without pivoting on an SPD matrix; 8 n eps cond allows for the
+    products' own rounding."""
+    import torch
+    rng = np.random.default_rng(n)
+    q = rng.standard_normal((n, n))
+    dense = (q @ q.T / n + np.diag(rng.uniform(0.5, 2.0, n))).astype(np.float32).astype(np.float64)
+    dense = np.tril(dense) + np.tril(dense, -1).T
+    i, j = np.indices((n, n)).reshape(2, -1)
+    a = L.upload(_system(i, j, dense.ravel(), n, rng))
+    inv = torch.empty(n * n, dtype=torch.float64, device="cuda")
+    flag = torch.full((1,), 7.0, dtype=torch.float64, device="cuda")
+    L.dense_inverse(a, inv, flag)
+    got, want = inv.cpu().numpy().reshape(n, n), np.linalg.inv(dense)
+    assert flag.item() == 0.0
+    bound = 8 * n * np.finfo(float).eps * np.linalg.cond(dense)
+    assert np.max(np.abs(got - want)) <= bound * np.max(np.abs(want))
+
+
+@pytest.mark.parametrize("sides", [(40, 33, 27), (96, 96, 72)])
+@pytest.mark.parametrize("shuffled", [False, True], ids=["near", "far"])
+def test_mixed_coarse_rows(cuda, sides, shuffled):
+    """Coarse levels whose columns lie near their rows (value and column in one
+    word) or, with shuffled cells and more than 32,767 coarse rows, far from
+    them, on either side of 75,776 rows: the FP64 residual formed here meets the
+    tolerance, in as many refinements either way (a wrong entry would stall)."""
+    import scipy.sparse as sp
+    import torch
+    s = harness.box_system(*sides, tet=False, seed=6)
+    A = sp.csr_matrix((s.val, s.col, s.row_ptr), shape=(s.n, s.n))
+    rng = np.random.default_rng(1)
+    if shuffled:
+        order = rng.permutation(s.n)
+        A = A[order][:, order].tocsr()
+    A.sort_indices()
+    row = np.repeat(np.arange(s.n), np.diff(A.indptr))
+    t = harness.HostSystem(A.indptr.astype(np.int32), A.indices.astype(np.int32),
+                           np.nonzero(row == A.indices)[0].astype(np.int32), A.data,
+                           rng.standard_normal(s.n).astype(np.float32))
+    a = L.upload(t)
+    solver = L.make_mixed_solver(t)
+    solver.refresh(a)
+    x = torch.zeros(s.n, dtype=torch.float64, device="cuda")
+    st = solver.solve(a, x, torch.from_numpy(t.b).cuda(), L.SolveControl(1e-9, 1e-30, 1000))
+    b = t.b.astype(np.float64)
+    assert st.converged and st.refinements <= 5
+    assert np.linalg.norm(b - A @ x.cpu().numpy()) <= 1.0001e-9 * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("n", [2, 7, 9, 31, 33, 127, 129, 1001, 4097])
+def test_learned_gradient_at_ragged_sizes(cuda, n):
+    """Row counts that leave a part of a thread's eight rows, a warp's or a
+    128-row tile: the FP32 backward against the tensor-core one, whose BF16
+    operands carry 8 bits (3e-2 of each block, as at full sizes), and its loss."""
+    import scipy.sparse as sp
+    import torch
+    s = harness.poisson(n, 1)
+    a = L.upload(s)
+    g = L.LearnedStage(seed=5)
+    g.bind(a)
+    A = sp.csr_matrix((s.val, s.col, s.row_ptr), shape=(n, n))
+    e = np.random.default_rng(n).standard_normal(n)
+    t = torch.from_numpy((A @ e).astype(np.float32)).cuda()
+    e = torch.from_numpy(e.astype(np.float32)).cuda()
+    tc, loss_tc = g.gradient(t, e, tensor_cores=True)
+    fp, loss_fp = g.gradient(t, e, tensor_cores=False)
+    assert np.all(np.isfinite(fp)) and np.linalg.norm(fp) > 0
+    assert loss_tc == pytest.approx(loss_fp, rel=1e-5, abs=1e-6)
+    assert np.linalg.norm(tc - fp) <= 3e-2 * np.linalg.norm(fp)
