@@ -41,6 +41,7 @@ PRODUCT_CU = {
     "exact_kernels.cu": EXACT,
     "coarse_rows.cu": EXACT,
     "mixed_kernels.cu": [],
+    "mixed_tail.cu": [],
     "tail_cycle.cu": [],
     "learned.cu": [],
     "learned_tc.cu": [],

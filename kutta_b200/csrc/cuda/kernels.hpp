@@ -252,6 +252,35 @@ void bf16_spmv_dot2(int n, const Bf16Rows& m, const float* p, const float* w, fl
 void bf16_smooth_dot(int n, const Bf16Rows& m, const float* x, const float* b, const float* inv,
                      float* next, const float* q, DeviceReducer red, float* scalars, int* status,
                      cudaStream_t s);
+// The smallest levels and the dense coarsest in one block (mixed_tail.cu): the
+// V-cycle, or with `inner` the two Krylov steps on the first of them. Offsets (at)
+// count 32-bit words of its shared memory, of which the image's are loaded.
+struct MixedTail {
+  static constexpr int kMaxLevels = 8, kMaxRows = 1024, kMaxBytes = 224 * 1024;
+  struct Level {
+    int n;
+    int slices_at, entries_at;       // per 32 rows (first slot, slots per row); slots
+    int scale_at, inv_at;
+    int aggregate_at;                // the next level's row or -1
+    int groups_at, members_at;       // the next level's rows' slices of byte offsets
+    int x_at, r_at, b_at;
+  };
+  // The last is the dense one: n, entries_at (FP64 inverse), x_at, b_at (FP64).
+  Level level[kMaxLevels];
+  int levels, pre, post, bytes;
+  bool inner;
+  int order_at, p_at, inverse_at, image_words;
+  const unsigned* image;
+  struct Values {
+    int slots, entries_at, n, scale_at, inv_at;
+    const int *source, *order;
+    const unsigned* packed;
+    const float *scale, *inv;
+  };
+};
+void mixed_tail_values(const MixedTail::Values& v, unsigned* image, cudaStream_t s);
+void mixed_tail(const MixedTail& t, const float* right, float* out, const int* status,
+                cudaStream_t s);
 // inner_first, t.t and b.b -> scalars[4..7] and the exit check (inner_check).
 void inner_first_dot(int n, const float* b, const float* p, const float* q, float* x, float* t,
                      float* scalars, int* status, DeviceReducer red, cudaStream_t s);

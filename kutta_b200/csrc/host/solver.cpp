@@ -148,7 +148,9 @@ Solver::Solver(Kind kind, const CsrView& a, const Options& options,
     if (options_.dense_coarsest && levels_.size() > 1 && c.n <= 1024) {
       c.dense_lower.reset(static_cast<std::size_t>(c.n) * c.n);
       c.dense_inverse.reset(static_cast<std::size_t>(c.n) * c.n);
+      c.inverse = c.dense_inverse.get();
     }
+    plan_mixed_tail(s);
     // Usable before the first refresh, from the setup values.
     prepare_mixed(s, 0);
     cuda_check(cudaMemcpyAsync(host_values_.get(), values_.get(), 2 * sizeof(double),
@@ -352,7 +354,7 @@ void Solver::plan_tail() {
     p.post = options_.post_sweeps;
     p.coarse_sweeps = options_.coarse_sweeps;
     p.cluster = cluster;
-    p.dense = dense(coarsest) ? coarsest.dense_inverse.get() : nullptr;
+    p.dense = dense(coarsest) ? coarsest.inverse : nullptr;
     double bytes = 0;
     int shared_floats = 0;
     for (int k = 0; k < p.levels; ++k) {
@@ -406,6 +408,164 @@ void Solver::plan_tail() {
   }
 }
 
+// The largest run of levels, at most kMaxRows rows each and with the dense
+// coarsest below, that fits one block's shared memory (mixed_tail.cu). Only the
+// first of them may carry inner Krylov steps.
+void Solver::plan_mixed_tail(cudaStream_t s) {
+  using launch::MixedTail;
+  const std::size_t count = levels_.size();
+  if (kind_ != Kind::AmgPcg || nullspace_ || !options_.coarse_bf16 || options_.fused_tail ||
+      count < 3 || !dense(levels_.back()) || options_.pre_sweeps < 1 || options_.post_sweeps < 1)
+    return;
+  const auto host = [&](const DArray<int>& from) {
+    std::vector<int> to(from.size());
+    if (!to.empty())
+      cuda_check(cudaMemcpyAsync(to.data(), from.get(), to.size() * sizeof(int),
+                                 cudaMemcpyDeviceToHost, s),
+                 "readback");
+    wait(s);
+    return to;
+  };
+  for (std::size_t start = 1; start + 1 < count; ++start) {
+    if (levels_[start].n > MixedTail::kMaxRows || count - start > MixedTail::kMaxLevels) continue;
+    if (options_.cycle == Cycle::K && start + 2 < count && inner_level(start + 1)) continue;
+    MixedTail t{};
+    std::vector<unsigned> image;
+    const auto put = [&](const auto& words) {
+      const int at = static_cast<int>(image.size());
+      image.insert(image.end(), words.begin(), words.end());
+      image.resize((image.size() + 3) & ~std::size_t{3});
+      return at;
+    };
+    // Rows of lists (length, word k) as slices of 32 rows, each as long as its
+    // longest row and a multiple of four; shorter rows are filled with `empty`.
+    const auto slices = [&](int n, auto length, auto word, unsigned empty, int& slices_at,
+                            int& slots_at) {
+      std::vector<unsigned> bounds, slots;
+      for (int i0 = 0; i0 < n; i0 += 32) {
+        int longest = 0;
+        for (int i = i0; i < std::min(n, i0 + 32); ++i) longest = std::max(longest, length(i));
+        longest = (longest + 3) & ~3;
+        bounds.push_back(static_cast<unsigned>(slots.size()));
+        bounds.push_back(static_cast<unsigned>(longest));
+        for (int k = 0; k < longest; ++k)
+          for (int i = i0; i < i0 + 32; ++i)
+            slots.push_back(i < n && k < length(i) ? word(i, k) : empty);
+      }
+      slices_at = put(bounds);
+      slots_at = put(slots);
+      return static_cast<int>(slots.size());
+    };
+    std::vector<std::vector<int>> order(count - start), rank(count - start);
+    std::vector<std::vector<int>> rows(count - start);
+    bool fits = true;
+    for (std::size_t i = start; i < count; ++i) {
+      const DevLevel& l = levels_[i];
+      auto& o = order[i - start];
+      o.resize(static_cast<std::size_t>(l.n));
+      std::iota(o.begin(), o.end(), 0);
+      if (i + 1 < count) {
+        fits = fits && l.packed16.allocated();
+        auto& p = rows[i - start] = row_pointers(l, s);
+        std::stable_sort(o.begin(), o.end(),
+                         [&](int a, int b) { return p[a + 1] - p[a] > p[b + 1] - p[b]; });
+      }
+      rank[i - start].resize(o.size());
+      for (int k = 0; k < l.n; ++k) rank[i - start][static_cast<std::size_t>(o[k])] = k;
+    }
+    std::vector<std::vector<int>> sources;
+    std::vector<MixedTail::Values> values;
+    for (std::size_t i = start; fits && i + 1 < count; ++i) {
+      const DevLevel& l = levels_[i];
+      MixedTail::Level& d = t.level[i - start];
+      const auto& o = order[i - start];
+      const auto& p = rows[i - start];
+      const auto& next = order[i - start + 1];
+      const std::vector<int> cols = host(l.col), members = host(l.members),
+                             offsets = host(l.member_offsets), aggregate = host(l.aggregate);
+      std::vector<int> source;
+      d.n = l.n;
+      const unsigned zero = 4u * static_cast<unsigned>(l.n);
+      const int slots = slices(
+          l.n, [&](int r) { return p[o[r] + 1] - p[o[r]]; },
+          [&](int r, int k) {
+            return 4u * static_cast<unsigned>(rank[i - start][cols[p[o[r]] + k]]);
+          },
+          zero, d.slices_at, d.entries_at);
+      // The CSR entry of each slot, in the same walk.
+      source.assign(static_cast<std::size_t>(slots), -1);
+      for (int r = 0; r < l.n; ++r) {
+        const int slot = static_cast<int>(image[d.slices_at + 2 * (r / 32)]) + r % 32;
+        for (int k = 0; k < p[o[r] + 1] - p[o[r]]; ++k) source[slot + 32 * k] = p[o[r]] + k;
+      }
+      const int nc = levels_[i + 1].n;
+      slices(
+          nc, [&](int g) { return offsets[next[g] + 1] - offsets[next[g]]; },
+          [&](int g, int k) {
+            return 4u * static_cast<unsigned>(rank[i - start][members[offsets[next[g]] + k]]);
+          },
+          zero, d.groups_at, d.members_at);
+      std::vector<unsigned> words(static_cast<std::size_t>(l.n));
+      for (int r = 0; r < l.n; ++r) {
+        const int g = aggregate[o[r]];
+        words[r] = static_cast<unsigned>(g >= 0 ? rank[i - start + 1][g] : -1);
+      }
+      d.aggregate_at = put(words);
+      d.scale_at = put(words);  // set by the values
+      d.inv_at = put(words);
+      sources.push_back(std::move(source));
+      values.push_back({slots, d.entries_at, l.n, d.scale_at, d.inv_at, nullptr, nullptr,
+                        l.packed16.get(), l.scale.get(), l.l1.get()});
+      fits = 4 * image.size() <= MixedTail::kMaxBytes;
+    }
+    if (!fits) continue;
+    t.order_at = put(order[0]);
+    const int nd = levels_.back().n;
+    MixedTail::Level& dense_level = t.level[count - 1 - start];
+    dense_level.n = nd;
+    t.inverse_at = dense_level.entries_at = static_cast<int>(image.size());
+    const std::size_t inverse_words = 2 * static_cast<std::size_t>(nd) * nd;
+    t.image_words = t.inverse_at + static_cast<int>((inverse_words + 3) & ~std::size_t{3});
+    long long words = t.image_words;
+    const auto take = [&](long long size) {
+      const long long at = words;
+      words += (size + 3) & ~3LL;
+      return static_cast<int>(at);
+    };
+    for (std::size_t i = start; i < count; ++i) {
+      MixedTail::Level& d = t.level[i - start];
+      d.x_at = take(d.n + 1LL);
+      d.r_at = take(d.n + 1LL);
+      d.b_at = take(2LL * d.n);
+    }
+    t.p_at = take(t.level[0].n + 1LL);
+    if (4 * words > MixedTail::kMaxBytes) continue;
+    t.bytes = static_cast<int>(4 * words);
+    t.levels = static_cast<int>(count - start);
+    t.pre = options_.pre_sweeps;
+    t.post = options_.post_sweeps;
+    t.inner = options_.cycle == Cycle::K && inner_level(start);
+    image.resize(static_cast<std::size_t>(t.image_words));
+    mixed_tail_image_.upload(image, s);
+    t.image = mixed_tail_image_.get();
+    levels_.back().inverse = reinterpret_cast<double*>(mixed_tail_image_.get() + t.inverse_at);
+    levels_.back().dense_inverse = DArray<double>();
+    for (std::size_t i = start; i + 1 < count; ++i) {
+      DevLevel& l = levels_[i];
+      l.tail_source.upload(sources[i - start], s);
+      l.tail_order.upload(order[i - start], s);
+      values[i - start].source = l.tail_source.get();
+      values[i - start].order = l.tail_order.get();
+    }
+    wait(s);  // the host arrays are released here
+    mixed_tail_ = t;
+    mixed_tail_values_ = std::move(values);
+    mixed_tail_start_ = start;
+    mixed_tail_bytes_ = 4.0 * t.image_words + 8.0 * t.level[0].n;
+    return;
+  }
+}
+
 // BF16 copies of the coarse operators (unless the refresh's row pass has made
 // them) and the dense inverse of the coarsest, from the current FP32 coarse
 // values; the dense SPD check lands in values_[slot].
@@ -417,8 +577,10 @@ void Solver::prepare_mixed(cudaStream_t s, int slot, bool packed) {
     if (l.bf16() && !packed) launch::bf16_pack(l.n, l.val.get(), l.bf16_store(), s);
     if (dense(l))
       launch::dense_inverse(l.n, l.row_ptr.get(), l.col.get(), l.val.get(), l.dense_lower.get(),
-                            l.dense_inverse.get(), error, s, error + 1);
+                            l.inverse, error, s, error + 1);
   }
+  for (const auto& v : mixed_tail_values_)
+    launch::mixed_tail_values(v, mixed_tail_image_.get(), s);
 }
 
 // The coarsest level is solved with its dense inverse only when that is
@@ -612,7 +774,7 @@ void Solver::cycle(std::size_t index, const float* b, float*& x, const int* stat
   }
   if (index + 1 == levels_.size()) {
     if (dense(l) && dense_ok_) {
-      launch::dense_solve(l.n, l.dense_inverse.get(), b, x, status, stream_);
+      launch::dense_solve(l.n, l.inverse, b, x, status, stream_);
       tally(8.0 * l.n * l.n + 8.0 * l.n);
     } else if (l.n <= 24) {
       launch::coarse_solve(l.n, rows, cols, vals, x, b, l.l1.get(), status,
@@ -651,7 +813,10 @@ void Solver::cycle(std::size_t index, const float* b, float*& x, const int* stat
                              stream_);
     tally(8.0 * l.nnz + 4.0 * (l.n + 1) + 12.0 * l.n + 4.0 * (c.n + 1) + 8.0 * l.n + 4.0 * c.n);
     if (nullspace_) project(c.b.get(), c.n, c.projection.get());
-    if (inner_next)
+    if (mixed_tail_start_ == index + 1 && dense_ok_) {
+      launch::mixed_tail(mixed_tail_, c.b.get(), c.x, status, stream_);
+      tally(mixed_tail_bytes_);
+    } else if (inner_next)
       inner(index + 1, status);
     else if (!tail_next)
       cycle(index + 1, c.b.get(), c.x, status, sweep_next);
@@ -1289,6 +1454,8 @@ std::string Solver::describe() const {
                                : ", nearly singular coarsest smoothed instead of its dense inverse")
                   : "");
     if (packed_.width > 0) out << ", packed fine rows";
+    if (mixed_tail_start_ != 0 && dense_ok_)
+      out << ", levels " << mixed_tail_start_ << "-" << levels_.size() - 1 << " in one block";
     if (tail_on_)
       out << ", levels " << tail_start_ << "-" << levels_.size() - 1 << " in one "
           << tail_.cluster << "-CTA cluster launch";

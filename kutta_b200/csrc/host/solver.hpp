@@ -90,11 +90,12 @@ struct DevLevel {
     return {row_ptr.get(), col.get(), v16.get(), packed16.get(), scale.get()};
   }
   DArray<double> dense_lower, dense_inverse;
+  double* inverse = nullptr;    // dense_inverse, or its place in the one-block tail's image
   // The plain solve's row kernels form the row's products with all threads of a
   // block (launch::staged_smooth) instead of a thread per row.
   bool staged = false;
   DArray<int> order;            // rows by length in blocks of 128 (levels with hub rows)
-  // Levels of the one-block tail (launch::PlainTail::Level).
+  // Levels of the one-block tails (launch::PlainTail::Level, MixedTail::Values).
   DArray<int> tail_order, tail_start, tail_source;
   // transfer to level + 1
   DArray<int> aggregate, member_offsets, members, entry_offsets, entries;
@@ -141,7 +142,7 @@ class Solver {
   // A variable preconditioner needs the flexible beta (solver.cpp:296-298): the
   // K-cycle, and the mixed V-cycle (BF16 rounding breaks exact symmetry).
   bool variable() const { return amg() && (options_.cycle == Cycle::K || options_.coarse_bf16); }
-  bool dense(const DevLevel& l) const { return l.dense_inverse.allocated(); }
+  bool dense(const DevLevel& l) const { return l.inverse != nullptr; }
   // Whether coarse level `index` takes the K-cycle's inner Krylov step (given
   // a K-cycle and a level above the coarsest two).
   bool inner_level(std::size_t index) const {
@@ -167,6 +168,13 @@ class Solver {
   launch::TailPlan tail_{};
   // The plain V-cycle's choice of row kernels per level, and its smallest
   // levels (>= plain_tail_start_, 0: none) in one block.
+  // The mixed solve's: levels >= mixed_tail_start_ (0: none) in one block.
+  void plan_mixed_tail(cudaStream_t s);
+  launch::MixedTail mixed_tail_{};
+  std::vector<launch::MixedTail::Values> mixed_tail_values_;
+  DArray<unsigned> mixed_tail_image_;
+  std::size_t mixed_tail_start_ = 0;
+  double mixed_tail_bytes_ = 0;
   static bool near_columns(const DevLevel& l, cudaStream_t s);
   void plan_plain(cudaStream_t s);
   static std::vector<int> row_pointers(const DevLevel& l, cudaStream_t s);

@@ -145,6 +145,42 @@ def test_mixed_coarse_rows(cuda, sides, shuffled):
     assert np.linalg.norm(b - A @ x.cpu().numpy()) <= 1.0001e-9 * np.linalg.norm(b)
 
 
+@pytest.mark.parametrize("cycle, sweeps", [(L.AmgCycle.V, 1), (L.AmgCycle.V, 2), (L.AmgCycle.K, 1),
+                                           (L.AmgCycle.K, 3)], ids=["v1", "v2", "k1", "k3"])
+@pytest.mark.parametrize("make, one_block", [
+    # 62 rows below (no level in between); 125 + 15; 500 + 62; 1,024 and 1,025 rows,
+    # of which the first fill the block; 1,125, 140 and 18.
+    (lambda: harness.poisson(500, 1), False),
+    *((lambda n=n: harness.poisson(n, 1), True) for n in (1000, 4000, 8192, 8200, 9000)),
+    (lambda: harness.box_system(10, 10, 10, tet=True, seed=2), True),
+    (lambda: harness.box_system(24, 22, 20, tet=False, seed=3), True),
+    # Rows of up to 76 entries; more entries than shared memory holds.
+    (lambda: _random_rows(3000, 6, 8), True),
+    (lambda: _random_rows(7000, 9, 8), False),
+], ids=["500", "1000", "4000", "8192", "8200", "9000", "tet", "hex", "hubs", "large"])
+def test_small_levels_in_one_block(cuda, make, one_block, cycle, sweeps):
+    """One application of the preconditioner with its smallest levels in one
+    block against the same with the cluster launch and separate kernels
+    (fused_coarse): the same steps in FP32, whose sums of a few tens of terms may
+    run in another order, each rounding within 32 eps of its row's terms, and a
+    cycle that contracts: 1e-5 relative."""
+    import torch
+    s = make()
+    a = L.upload(s)
+    b = torch.from_numpy(s.b).cuda()
+    z = []
+    for fused in (False, True):
+        amg = L.AmgOptions(cycle=cycle, pre_sweeps=sweeps, post_sweeps=sweeps, structure=M)
+        solver = L.make_mixed_solver(s, L.MixedOptions(amg=amg, fused_coarse=fused))
+        solver.refresh(a)
+        out = torch.zeros(s.n, device="cuda")
+        solver.precondition(a, b, out)
+        z.append(out.double().cpu().numpy())
+        if not fused:
+            assert ("in one block" in solver.describe()) == one_block, solver.describe()
+    assert np.linalg.norm(z[0] - z[1]) <= 1e-5 * np.linalg.norm(z[1])
+
+
 @pytest.mark.parametrize("n", [2, 7, 9, 31, 33, 127, 129, 1001, 4097])
 def test_learned_gradient_at_ragged_sizes(cuda, n):
     """Row counts that leave a part of a thread's eight rows, a warp's or a
