@@ -329,7 +329,8 @@ int b2_csr_residual(int n, int nnz, const int32_t* d_row_ptr, const int32_t* d_c
     KB2_REQUIRE(d_row_ptr && d_x && d_b && d_r && (nnz == 0 || (d_col && d_val)),
                 "CSR: null argument");
     KB2_REQUIRE(d_x != d_r && d_b != d_r, "CSR: residual RHS size or alias mismatch");
-    kb2::launch::residual(n, d_row_ptr, d_col, d_val, d_x, d_b, d_r, nullptr, as_stream(stream));
+    kb2::launch::residual(n, d_row_ptr, d_col, nullptr, d_val, d_x, d_b, d_r, nullptr,
+                          as_stream(stream));
     kb2::cuda_check(cudaGetLastError(), "csr_residual");
   });
 }
@@ -368,7 +369,7 @@ int b2_amg_smooth(int n, const int32_t* d_row_ptr, const int32_t* d_col, const f
                     (zero_start || d_x),
                 "smooth: null argument");
     KB2_REQUIRE(d_next != d_x && d_next != d_b, "smooth: output aliases an input");
-    kb2::launch::smooth(n, d_row_ptr, d_col, d_val, d_x, d_b, d_inverse, d_next, nullptr,
+    kb2::launch::smooth(n, d_row_ptr, d_col, nullptr, d_val, d_x, d_b, d_inverse, d_next, nullptr,
                         zero_start != 0, as_stream(stream));
     kb2::cuda_check(cudaGetLastError(), "amg_smooth");
   });

@@ -33,8 +33,27 @@ using namespace dev;
 
 // ---- CSR row kernels --------------------------------------------------------
 // One row per thread: on the 5-entry fine rows this direct form measured
-// fastest (74% of the copy peak); staging tiles in shared memory or
+// fastest; staging tiles in shared memory or
 // register-chunking the row both measured slower there.
+
+// The column of entry j of row i: from the CSR columns, or with kNear from 16-bit
+// offsets from the row (a level whose columns all lie that near). These kernels
+// are bound by HBM, and an entry is then 6 bytes instead of 8: a sweep over
+// 2,097,152 rows of seven entries 26.3 us instead of 28.3, over 1,572,864 rows of
+// five 15.3 instead of 18.5.
+template <bool kNear>
+struct Columns {
+  const void* data;
+  __device__ __forceinline__ int operator()(int i, int j) const {
+    if constexpr (kNear) return i + __ldg(static_cast<const short*>(data) + j);
+    return __ldg(static_cast<const int*>(data) + j);
+  }
+};
+__global__ void k_near_offsets(int n, const int* __restrict__ rows, const int* __restrict__ cols,
+                               short* __restrict__ near) {
+  pdl_entry();
+  ROWS(i, n) for (int j = rows[i]; j < rows[i + 1]; ++j) near[j] = static_cast<short>(cols[j] - i);
+}
 
 // csr_spmv / csr_spmv_guarded, linalg.kern.h:5-16,111-114.
 __global__ void k_spmv(int n, const int* __restrict__ rows, const int* __restrict__ cols,
@@ -52,7 +71,8 @@ __global__ void k_spmv(int n, const int* __restrict__ rows, const int* __restric
 
 // csr_spmv_guarded + dot_into(w, q) + a scalar kernel: PCG's p.q and alpha
 // (solver.cpp:288-290, w = p) or BiCGStab's rhat.q and alpha (:335-337, w = rhat).
-__global__ void k_spmv_dot(int n, const int* __restrict__ rows, const int* __restrict__ cols,
+template <bool kNear>
+__global__ void k_spmv_dot(int n, const int* __restrict__ rows, Columns<kNear> cols,
                            const float* __restrict__ vals, const float* __restrict__ p,
                            const float* __restrict__ w, float* __restrict__ q, DeviceReducer red,
                            float* scalars, int offset, int* status, Epilogue epi) {
@@ -62,7 +82,7 @@ __global__ void k_spmv_dot(int n, const int* __restrict__ rows, const int* __res
   ROWS(i, n) {
     float sum = 0.0f, error = 0.0f;
     const int end = rows[i + 1];
-    for (int j = rows[i]; j < end; ++j) kahan_term(sum, error, vals[j], p[cols[j]]);
+    for (int j = rows[i]; j < end; ++j) kahan_term(sum, error, vals[j], p[cols(i, j)]);
     q[i] = sum;
     acc += static_cast<double>(w[i]) * static_cast<double>(sum);
   }
@@ -70,7 +90,8 @@ __global__ void k_spmv_dot(int n, const int* __restrict__ rows, const int* __res
 }
 
 // csr_spmv_guarded + dot2_into(t, t; t, s) + solver_bicg_omega (solver.cpp:343-347).
-__global__ void k_spmv_dot2(int n, const int* __restrict__ rows, const int* __restrict__ cols,
+template <bool kNear>
+__global__ void k_spmv_dot2(int n, const int* __restrict__ rows, Columns<kNear> cols,
                             const float* __restrict__ vals, const float* __restrict__ x,
                             const float* __restrict__ sv, float* __restrict__ t, DeviceReducer red,
                             float* scalars, int* status) {
@@ -80,7 +101,7 @@ __global__ void k_spmv_dot2(int n, const int* __restrict__ rows, const int* __re
   ROWS(i, n) {
     float sum = 0.0f, error = 0.0f;
     const int end = rows[i + 1];
-    for (int j = rows[i]; j < end; ++j) kahan_term(sum, error, vals[j], x[cols[j]]);
+    for (int j = rows[i]; j < end; ++j) kahan_term(sum, error, vals[j], x[cols(i, j)]);
     t[i] = sum;
     tt += static_cast<double>(sum) * static_cast<double>(sum);
     ts += static_cast<double>(sum) * static_cast<double>(sv[i]);
@@ -89,7 +110,8 @@ __global__ void k_spmv_dot2(int n, const int* __restrict__ rows, const int* __re
 }
 
 // csr_residual / csr_residual_guarded, linalg.kern.h:32-50,115-118.
-__global__ void k_residual(int n, const int* __restrict__ rows, const int* __restrict__ cols,
+template <bool kNear>
+__global__ void k_residual(int n, const int* __restrict__ rows, Columns<kNear> cols,
                            const float* __restrict__ vals, const float* __restrict__ x,
                            const float* __restrict__ b, float* __restrict__ r,
                            const int* __restrict__ status) {
@@ -98,14 +120,14 @@ __global__ void k_residual(int n, const int* __restrict__ rows, const int* __res
   ROWS(i, n) {
     float sum = b[i], error = 0.0f;
     const int end = rows[i + 1];
-    for (int j = rows[i]; j < end; ++j) residual_term(sum, error, vals[j], x[cols[j]]);
+    for (int j = rows[i]; j < end; ++j) residual_term(sum, error, vals[j], x[cols(i, j)]);
     r[i] = sum + error;
   }
 }
 
 // amg_smooth (linalg.kern.h:150-156) and amg_smooth_zero (:162-170).
-template <bool kZero>
-__global__ void k_smooth(int n, const int* __restrict__ rows, const int* __restrict__ cols,
+template <bool kZero, bool kNear>
+__global__ void k_smooth(int n, const int* __restrict__ rows, Columns<kNear> cols,
                          const float* __restrict__ vals, const float* __restrict__ x,
                          const float* __restrict__ b, const float* __restrict__ inv,
                          float* __restrict__ next, const int* __restrict__ status) {
@@ -118,7 +140,7 @@ __global__ void k_smooth(int n, const int* __restrict__ rows, const int* __restr
     }
     float sum = b[i], error = 0.0f;
     const int end = rows[i + 1];
-    for (int j = rows[i]; j < end; ++j) residual_term(sum, error, vals[j], x[cols[j]]);
+    for (int j = rows[i]; j < end; ++j) residual_term(sum, error, vals[j], x[cols(i, j)]);
     next[i] = x[i] + (2.0f / 3.0f) * inv[i] * (sum + error);
   }
 }
@@ -727,34 +749,58 @@ void spmv(int n, const int* rows, const int* cols, const float* vals, const floa
   ++counter;
   pdl(k_spmv, full_grid(n), kBlock, 0, s, n, rows, cols, vals, x, y, status);
 }
-void spmv_dot(int n, const int* rows, const int* cols, const float* vals, const float* p,
-              const float* w, float* q, DeviceReducer red, float* scalars, int offset,
-              int* status, Epilogue epi, cudaStream_t s) {
+void spmv_dot(int n, const int* rows, const int* cols, const short* near, const float* vals,
+              const float* p, const float* w, float* q, DeviceReducer red, float* scalars,
+              int offset, int* status, Epilogue epi, cudaStream_t s) {
   ++counter;
-  pdl(k_spmv_dot, blocks(n), kBlock, 0, s, n, rows, cols, vals, p, w, q, red, scalars, offset,
-                                          status, epi);
+  if (near)
+    pdl(k_spmv_dot<true>, blocks(n), kBlock, 0, s, n, rows, Columns<true>{near}, vals, p, w, q, red,
+        scalars, offset, status, epi);
+  else
+    pdl(k_spmv_dot<false>, blocks(n), kBlock, 0, s, n, rows, Columns<false>{cols}, vals, p, w, q,
+        red, scalars, offset, status, epi);
 }
-void spmv_dot2(int n, const int* rows, const int* cols, const float* vals, const float* x,
-               const float* sv, float* t, DeviceReducer red, float* scalars, int* status,
-               cudaStream_t s) {
+void spmv_dot2(int n, const int* rows, const int* cols, const short* near, const float* vals,
+               const float* x, const float* sv, float* t, DeviceReducer red, float* scalars,
+               int* status, cudaStream_t s) {
   ++counter;
-  pdl(k_spmv_dot2, blocks(n), kBlock, 0, s, n, rows, cols, vals, x, sv, t, red, scalars, status);
+  if (near)
+    pdl(k_spmv_dot2<true>, blocks(n), kBlock, 0, s, n, rows, Columns<true>{near}, vals, x, sv, t,
+        red, scalars, status);
+  else
+    pdl(k_spmv_dot2<false>, blocks(n), kBlock, 0, s, n, rows, Columns<false>{cols}, vals, x, sv, t,
+        red, scalars, status);
 }
-void residual(int n, const int* rows, const int* cols, const float* vals, const float* x,
-              const float* b, float* r, const int* status, cudaStream_t s) {
+void residual(int n, const int* rows, const int* cols, const short* near, const float* vals,
+              const float* x, const float* b, float* r, const int* status, cudaStream_t s) {
   if (n <= 0) return;
   ++counter;
-  pdl(k_residual, full_grid(n), kBlock, 0, s, n, rows, cols, vals, x, b, r, status);
+  if (near)
+    pdl(k_residual<true>, full_grid(n), kBlock, 0, s, n, rows, Columns<true>{near}, vals, x, b, r,
+        status);
+  else
+    pdl(k_residual<false>, full_grid(n), kBlock, 0, s, n, rows, Columns<false>{cols}, vals, x, b, r,
+        status);
 }
-void smooth(int n, const int* rows, const int* cols, const float* vals, const float* x,
-            const float* b, const float* inv, float* next, const int* status, bool zero_start,
-            cudaStream_t s) {
+void smooth(int n, const int* rows, const int* cols, const short* near, const float* vals,
+            const float* x, const float* b, const float* inv, float* next, const int* status,
+            bool zero_start, cudaStream_t s) {
   if (n <= 0) return;
   ++counter;
   if (zero_start)
-    pdl(k_smooth<true>, full_grid(n), kBlock, 0, s, n, rows, cols, vals, x, b, inv, next, status);
+    pdl(k_smooth<true, false>, full_grid(n), kBlock, 0, s, n, rows, Columns<false>{cols}, vals, x, b,
+        inv, next, status);
+  else if (near)
+    pdl(k_smooth<false, true>, full_grid(n), kBlock, 0, s, n, rows, Columns<true>{near}, vals, x, b,
+        inv, next, status);
   else
-    pdl(k_smooth<false>, full_grid(n), kBlock, 0, s, n, rows, cols, vals, x, b, inv, next, status);
+    pdl(k_smooth<false, false>, full_grid(n), kBlock, 0, s, n, rows, Columns<false>{cols}, vals, x,
+        b, inv, next, status);
+}
+void near_offsets(int n, const int* rows, const int* cols, short* near, cudaStream_t s) {
+  if (n <= 0) return;
+  ++counter;
+  pdl(k_near_offsets, full_grid(n), kBlock, 0, s, n, rows, cols, near);
 }
 void smooth_dot2(int n, const int* rows, const int* cols, const float* vals, const float* x,
                  const float* b, const float* inv, float* next, const float* q, DeviceReducer red,

@@ -46,13 +46,16 @@ extern std::atomic<long long> counter;
 void spmv(int n, const int* rows, const int* cols, const float* vals, const float* x, float* y,
           const int* status, cudaStream_t s);
 // q = A p and w.q -> scalars[offset] as a pair, then `epi` (guarded by status).
-void spmv_dot(int n, const int* rows, const int* cols, const float* vals, const float* p,
-              const float* w, float* q, DeviceReducer red, float* scalars, int offset,
-              int* status, Epilogue epi, cudaStream_t s);
+void spmv_dot(int n, const int* rows, const int* cols, const short* near, const float* vals,
+              const float* p, const float* w, float* q, DeviceReducer red, float* scalars,
+              int offset, int* status, Epilogue epi, cudaStream_t s);
 // t = A x, t.t and t.sv -> scalars[2], scalars[4] and solver_bicg_omega.
-void spmv_dot2(int n, const int* rows, const int* cols, const float* vals, const float* x,
-               const float* sv, float* t, DeviceReducer red, float* scalars, int* status,
-               cudaStream_t s);
+void spmv_dot2(int n, const int* rows, const int* cols, const short* near, const float* vals,
+               const float* x, const float* sv, float* t, DeviceReducer red, float* scalars,
+               int* status, cudaStream_t s);
+// near[j] = column of entry j - its row, for rows with all columns within 16 bits;
+// the row kernels that take `near` read it in the place of cols where not null.
+void near_offsets(int n, const int* rows, const int* cols, short* near, cudaStream_t s);
 // The mixed solve's packed copy of the fine operator ("packed rows"): per
 // row i the diagonal value diag[i] and `width` (4 or 8) off-diagonal slots,
 // values vals[width i + k] and int16 column offsets offsets[width i + k] =
@@ -80,13 +83,13 @@ void packed_smooth_dot2(int n, PackedRows a, const float* x, const float* b, con
                         float* next, const float* q, DeviceReducer red, float* scalars,
                         int offset, int* status, Epilogue epi, cudaStream_t s);
 // r = b - A x, Neumaier + Dekker compensated (csr_residual). status may be null.
-void residual(int n, const int* rows, const int* cols, const float* vals, const float* x,
-              const float* b, float* r, const int* status, cudaStream_t s);
+void residual(int n, const int* rows, const int* cols, const short* near, const float* vals,
+              const float* x, const float* b, float* r, const int* status, cudaStream_t s);
 // next = x + (2/3) inv (b - A x)  (amg_smooth); zero_start: x treated as the
 // zero vector without reading it (amg_smooth_zero).
-void smooth(int n, const int* rows, const int* cols, const float* vals, const float* x,
-            const float* b, const float* inv, float* next, const int* status, bool zero_start,
-            cudaStream_t s);
+void smooth(int n, const int* rows, const int* cols, const short* near, const float* vals,
+            const float* x, const float* b, const float* inv, float* next, const int* status,
+            bool zero_start, cudaStream_t s);
 // The fine post-sweep with the flexible PCG's r.z and z.q (b = r, next = z)
 // reduced into scalars[offset..] and the epilogue run, as reduce_into(Dot2).
 void smooth_dot2(int n, const int* rows, const int* cols, const float* vals, const float* x,

@@ -213,6 +213,12 @@ void Solver::plan_plain(cudaStream_t s) {
     l.order.upload(order, s);
     wait(s);  // the host array is released here
   }
+  // Rows read by a thread each take 16-bit offsets for columns where they can.
+  for (auto& l : levels_)
+    if (!l.staged && near_columns(l, s)) {
+      l.near.reset(static_cast<std::size_t>(l.nnz));
+      launch::near_offsets(l.n, l.row_ptr.get(), l.col.get(), l.near.get(), s);
+    }
   if (nullspace_ || options_.cycle != Cycle::V) return;
   launch::PlainTail t{};
   std::size_t start = levels_.size();
@@ -605,7 +611,7 @@ void Solver::residual(const float* x, const float* b, float* r) {
   if (packed_.width > 0)
     launch::packed_residual(n_, packed(), x, b, r, nullptr, stream_);
   else
-    launch::residual(n_, rows0(), cols0(), val_, x, b, r, nullptr, stream_);
+    launch::residual(n_, rows0(), cols0(), near0(), val_, x, b, r, nullptr, stream_);
   tally(fine_operator_bytes() + 12.0 * n_);
 }
 
@@ -624,7 +630,7 @@ void Solver::check_device() const {
 void Solver::set_profile(bool on) {
   profiling_ = on;
   prof_ = Profile{};
-  prof_.fine_sweep_bytes = 8.0 * nnz_ + 4.0 * (n_ + 1) + 16.0 * n_;
+  prof_.fine_sweep_bytes = csr_bytes(levels_[0]) + 16.0 * n_;
   launch_mark_ = launch::counter.load();
   events_used_ = 0;
   event_bytes_.clear();
@@ -722,7 +728,7 @@ void Solver::smooth(DevLevel& l, const int* rows, const int* cols, const float* 
     const bool packed_rows = with_dots && packed_.width > 0;
     const double bytes =
         zero ? 12.0 * l.n
-             : (packed_rows ? fine_operator_bytes() : 8.0 * l.nnz + 4.0 * (l.n + 1)) +
+             : (packed_rows ? fine_operator_bytes() : csr_bytes(l)) +
                    (with_dots ? 20.0 : 16.0) * l.n;
     if (timed) event_bytes_.push_back(bytes);
     if (inner_dot_ == &l && !zero_start && sweep + 1 == sweeps)
@@ -742,7 +748,8 @@ void Solver::smooth(DevLevel& l, const int* rows, const int* cols, const float* 
                             sweep == 0 && coarse ? l.aggregate.get() : nullptr, coarse,
                             l.order.get(), stream_);
     else
-      launch::smooth(l.n, rows, cols, vals, x, b, l.l1.get(), l.r, status, zero, stream_);
+      launch::smooth(l.n, rows, cols, l.near.get(), vals, x, b, l.l1.get(), l.r, status, zero,
+                     stream_);
     if (timed) cuda_check(cudaEventRecord(events_[events_used_++], stream_), "cudaEventRecord");
     tally(bytes);
     std::swap(x, l.r);  // ping-pong: the two buffers exchange roles (amg.cpp:280)
@@ -791,7 +798,7 @@ void Solver::cycle(std::size_t index, const float* b, float*& x, const int* stat
     else if (l.staged)
       launch::staged_residual(l.n, rows, cols, vals, x, b, l.r, status, l.order.get(), stream_);
     else
-      launch::residual(l.n, rows, cols, vals, x, b, l.r, status, stream_);
+      launch::residual(l.n, rows, cols, l.near.get(), vals, x, b, l.r, status, stream_);
     auto& c = levels_[index + 1];
     const bool inner_next =
         options_.cycle == Cycle::K && index + 2 < levels_.size() && inner_level(index + 1);
@@ -811,7 +818,7 @@ void Solver::cycle(std::size_t index, const float* b, float*& x, const int* stat
     } else
       launch::restrict_lanes(c.n, l.member_offsets.get(), l.members.get(), l.r, c.b.get(), status,
                              stream_);
-    tally(8.0 * l.nnz + 4.0 * (l.n + 1) + 12.0 * l.n + 4.0 * (c.n + 1) + 8.0 * l.n + 4.0 * c.n);
+    tally(csr_bytes(l) + 12.0 * l.n + 4.0 * (c.n + 1) + 8.0 * l.n + 4.0 * c.n);
     if (nullspace_) project(c.b.get(), c.n, c.projection.get());
     if (mixed_tail_start_ == index + 1 && dense_ok_) {
       launch::mixed_tail(mixed_tail_, c.b.get(), c.x, status, stream_);
@@ -930,7 +937,7 @@ void Solver::precondition(const float* r, float*& z) {
   cycle(0, r, z, status_.get(), swept_);
   if (learned_ != nullptr && (learned_mode_ & kLearnedCycle)) {
     float* t = learned_residual_.get();
-    launch::residual(n_, rows0(), cols0(), val_, z, r, t, status_.get(), stream_);
+    launch::residual(n_, rows0(), cols0(), near0(), val_, z, r, t, status_.get(), stream_);
     learned_direction(t);
     launch::gnn_step(n_, z, learned_correction_.get(), learned_dots_.get(), stream_);
     tally(8.0 * nnz_ + 4.0 * (n_ + 1) + 12.0 * n_ + 12.0 * n_);
@@ -1245,8 +1252,8 @@ void Solver::pcg(float* x, const float* b, const Control& c, double target, Stat
         launch::packed_spmv_dot(n_, packed(), p_, p_, q_, reducer(), scalars_.get(), 2,
                                 status_.get(), Epilogue::PcgAlpha, stream_);
       else
-        launch::spmv_dot(n_, rows0(), cols0(), val_, p_, p_, q_, reducer(), scalars_.get(), 2,
-                         status_.get(), Epilogue::PcgAlpha, stream_);
+        launch::spmv_dot(n_, rows0(), cols0(), near0(), val_, p_, p_, q_, reducer(),
+                         scalars_.get(), 2, status_.get(), Epilogue::PcgAlpha, stream_);
       const bool last = stats.iterations + j + 1 == c.max_iter;
       const bool sweep = amg() && levels_.size() > 1 && !last;
       auto& fine = levels_[0];
@@ -1317,15 +1324,15 @@ void Solver::bicgstab(float* x, const float* b, const Control& c, double target,
       (void)j;
       launch::bicg_direction(n_, r_, q_, p_, sc, status_.get(), stream_);
       apply(p_, z_);
-      launch::spmv_dot(n_, rows0(), cols0(), val_, z_, shadow_, q_, reducer(), sc, 2,
+      launch::spmv_dot(n_, rows0(), cols0(), near0(), val_, z_, shadow_, q_, reducer(), sc, 2,
                        status_.get(), Epilogue::BicgAlpha, stream_);
       launch::bicg_difference(n_, r_, q_, s_, reducer(), sc, status_.get(), stream_);
       apply(s_, zs_);
-      launch::spmv_dot2(n_, rows0(), cols0(), val_, zs_, s_, t_, reducer(), sc, status_.get(),
-                        stream_);
+      launch::spmv_dot2(n_, rows0(), cols0(), near0(), val_, zs_, s_, t_, reducer(), sc,
+                        status_.get(), stream_);
       launch::bicg_step(n_, x, r_, z_, zs_, s_, t_, shadow_, reducer(), sc, status_.get(),
                         stream_);
-      tally(2.0 * (8.0 * nnz_ + 4.0 * (n_ + 1)) + 80.0 * n_);
+      tally(2.0 * csr_bytes(levels_[0]) + 80.0 * n_);
     }
     const auto state = poll(x, b);
     stats.iterations = state[1];

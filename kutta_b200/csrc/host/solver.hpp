@@ -94,6 +94,7 @@ struct DevLevel {
   // The plain solve's row kernels form the row's products with all threads of a
   // block (launch::staged_smooth) instead of a thread per row.
   bool staged = false;
+  DArray<short> near;           // column - row of each entry (launch::near_offsets)
   DArray<int> order;            // rows by length in blocks of 128 (levels with hub rows)
   // Levels of the one-block tails (launch::PlainTail::Level, MixedTail::Values).
   DArray<int> tail_order, tail_start, tail_source;
@@ -196,11 +197,15 @@ class Solver {
   }
   // Algorithmic bytes of one pass over the fine operator: CSR, or the packed
   // rows' stored entries (padding slots are not counted).
+  static double csr_bytes(const DevLevel& l) {
+    return (l.near.allocated() ? 6.0 : 8.0) * l.nnz + 4.0 * (l.n + 1);
+  }
   double fine_operator_bytes() const {
-    return packed_.width > 0 ? 6.0 * (nnz_ - n_) + 4.0 * n_ : 8.0 * nnz_ + 4.0 * (n_ + 1);
+    return packed_.width > 0 ? 6.0 * (nnz_ - n_) + 4.0 * n_ : csr_bytes(levels_[0]);
   }
   const int* rows0() const { return levels_[0].row_ptr.get(); }
   const int* cols0() const { return levels_[0].col.get(); }
+  const short* near0() const { return levels_[0].near.get(); }
 
   // Device primitives on stream_.
   void residual(const float* x, const float* b, float* r);

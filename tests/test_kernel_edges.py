@@ -115,6 +115,42 @@ def test_dense_inverse_edges(cuda, n):
     assert np.max(np.abs(got - want)) <= bound * np.max(np.abs(want))
 
 
+def _shuffled(s, seed):
+    import scipy.sparse as sp
+    rng = np.random.default_rng(seed)
+    order = rng.permutation(s.n)
+    A = sp.csr_matrix((s.val, s.col, s.row_ptr), shape=(s.n, s.n))[order][:, order].tocoo()
+    return _system(A.row, A.col, A.data, s.n, rng)
+
+
+@pytest.mark.parametrize("kind", ["pcg", "bicg"])
+@pytest.mark.parametrize("name, make", [
+    ("offset32767", lambda: harness.poisson(32767, 3)),
+    ("offset32768", lambda: harness.poisson(32768, 3)),
+    ("shuffled", lambda: _shuffled(harness.poisson(290, 230), 2)),
+])
+def test_plain_rows_with_near_and_far_columns(cuda, name, make, kind):
+    """Levels read by a thread per row (more than 65,536 rows), with all columns
+    within 16 bits of their row and without: whole solves against the oracle, x
+    within relative 1e-5 and equal iterations, as the solver parity tests require."""
+    import torch
+    from oracle import kutta_oracle as O
+    s = make()
+    ours, theirs = ((L.SolverKind.AmgPcg, O.AMG_PCG) if kind == "pcg" else
+                    (L.SolverKind.AmgBicgstab, O.AMG_BICGSTAB))
+    a = L.upload(s)
+    solver = L.make_amg_solver(ours, s, L.AmgOptions(pre_sweeps=2, post_sweeps=2))
+    solver.refresh(a)
+    b = np.random.default_rng(4).standard_normal(s.n).astype(np.float32)
+    x = torch.zeros(s.n, device="cuda")
+    st = solver.solve(a, x, torch.from_numpy(b).cuda(), L.SolveControl(1e-3, 1e-38, 60))
+    o = O.solve(s, theirs, b=b, rel_tol=1e-3, abs_tol=1e-38, max_iter=60,
+                opts=O.options(theirs, pre_sweeps=2, post_sweeps=2))
+    got = x.cpu().numpy().astype(np.float64)
+    assert (st.iterations, st.converged) == (o.iterations, o.converged)
+    assert np.linalg.norm(got - o.x) <= 1e-5 * np.linalg.norm(o.x.astype(np.float64))
+
+
 @pytest.mark.parametrize("sides", [(40, 33, 27), (96, 96, 72)])
 @pytest.mark.parametrize("shuffled", [False, True], ids=["near", "far"])
 def test_mixed_coarse_rows(cuda, sides, shuffled):
