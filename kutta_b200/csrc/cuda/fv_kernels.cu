@@ -106,7 +106,8 @@ __device__ __forceinline__ float register_row(int i, int begin, int count, int a
       if (face[u] < 0) continue;
       b -= sign[u] * flux[u];
       if (nb[u] < 0 || nb[u] == a.reference) ap = upper_add(ap, d[u]);
-      if (nb[u] < 0) continue;
+      // (A face between a cell and itself names the diagonal, which is set last.)
+      if (nb[u] < 0 || entry[u] == at) continue;
       const int slot = entry[u] - begin - (entry[u] > at);
       found |= 1u << slot;
       const int into = nb[u] != a.reference && i != a.reference ? slot : -1;

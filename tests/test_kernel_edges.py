@@ -57,7 +57,8 @@ def _device_fv(c):
 @pytest.mark.parametrize("degree, duplicate", [(3, 0.0), (4, 0.3), (5, 0.1), (6, 0.2), (8, 0.0)])
 def test_assembly_rows_match_oracle_and_refresh(cuda, degree, duplicate, reference):
     """Faces below, at and above six per row, some sharing an entry, some
-    entries without a face (they keep their value): bit for bit the oracle's
+    entries without a face (they keep their value), some faces naming the
+    diagonal: bit for bit the oracle's
     values, and with the refresh fused the separate refresh's levels."""
     import torch
     s = _random_rows(3000, degree, degree)
@@ -67,6 +68,11 @@ def test_assembly_rows_match_oracle_and_refresh(cuda, degree, duplicate, referen
     # their entries may be left without one.
     slots = np.isin(c.faces, np.arange(0, c.internal, 50))
     c.adjacent[slots] = -1
+    # A few others lie between a cell and itself (one layer of a periodic mesh).
+    own = np.isin(c.faces, np.arange(7, c.internal, 90))
+    cell = np.repeat(np.arange(s.n), np.diff(c.offsets))[own]
+    c.adjacent[own] = cell
+    c.entry[own] = s.diag[cell]
     start = s.val.astype(np.float32)
     v, r = start.copy(), np.zeros(s.n, np.float32)
     fv.oracle_assemble(c, v, r)
