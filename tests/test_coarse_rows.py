@@ -106,3 +106,24 @@ def test_solve_matches_oracle(cuda, name, point):
     got = x.cpu().numpy().astype(np.float64)
     assert (st.iterations, st.converged) == (o.iterations, o.converged)
     assert np.linalg.norm(got - o.x) <= 1e-5 * np.linalg.norm(o.x.astype(np.float64))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("scale", [1e-32, 1e32])
+def test_solve_beyond_the_split_guard(cuda, scale):
+    """Entries or iterates above 1e30, where the reference's product error is
+    zero: the same iterations as the oracle and x as above."""
+    import torch
+    s = harness.poisson(47, 43)
+    s.val = (s.val * scale).astype(f32).astype(np.float64)
+    b = np.random.default_rng(1).standard_normal(s.n).astype(f32)
+    a = L.upload(s)
+    solver = L.make_amg_solver(L.SolverKind.AmgPcg, s, L.AmgOptions(pre_sweeps=2, post_sweeps=2))
+    solver.refresh(a)
+    x = torch.zeros(s.n, device="cuda")
+    st = solver.solve(a, x, torch.from_numpy(b).cuda(), L.SolveControl(1e-4, 1e-38, 200))
+    o = O.solve(s, O.AMG_PCG, b=b, rel_tol=1e-4, abs_tol=1e-38, max_iter=200,
+                opts=O.options(O.AMG_PCG, pre_sweeps=2, post_sweeps=2))
+    got = x.cpu().numpy().astype(np.float64)
+    assert (st.iterations, st.converged) == (o.iterations, o.converged)
+    assert np.linalg.norm(got - o.x) <= 1e-5 * np.linalg.norm(o.x.astype(np.float64))
