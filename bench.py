@@ -899,11 +899,11 @@ def run_coupled(args):
     launches = (L.kernel_launches() - launches0) // args.steps
     st = results[-1]
     # The fine sweep alone: per cell x, b, next (float4 each) and the five
-    # per-cell records (88 bytes); per internal cell-face slot the edge
+    # per-cell records (44 bytes); per internal cell-face slot the edge
     # (a, gx, gy, gz), h and (neighbour, face) (28 bytes); per face its
     # (sx, sy, sz, rc) record (16 bytes).
     width_slots = int(np.sum(mesh["adjacent"] >= 0))
-    sweep_bytes = n * (48 + 88) + width_slots * 28 + nf * 16
+    sweep_bytes = n * (48 + 44) + width_slots * 28 + nf * 16
     x4 = torch.randn(4 * n, device="cuda")
     b4 = torch.randn(4 * n, device="cuda")
     y4 = torch.empty(4 * n, device="cuda")
