@@ -726,6 +726,9 @@ void Solver::smooth(DevLevel& l, const int* rows, const int* cols, const float* 
     // starts from zero) carries the fused reductions.
     const bool with_dots = fine && fuse_dots_ && !zero_start && sweep + 1 == sweeps;
     const bool packed_rows = with_dots && packed_.width > 0;
+    // Only the staged sweep adds a correction.
+    KB2_REQUIRE(sweep != 0 || coarse == nullptr || (l.staged && !with_dots),
+                "smooth: the coarse correction would be lost");
     const double bytes =
         zero ? 12.0 * l.n
              : (packed_rows ? fine_operator_bytes() : csr_bytes(l)) +
@@ -827,8 +830,10 @@ void Solver::cycle(std::size_t index, const float* b, float*& x, const int* stat
       inner(index + 1, status);
     else if (!tail_next)
       cycle(index + 1, c.b.get(), c.x, status, sweep_next);
-    // On staged levels the first post-sweep adds the correction as it reads x.
-    const bool fold = l.staged && options_.post_sweeps > 0;
+    // On staged levels the first post-sweep adds the correction as it reads x,
+    // unless it is the last one of the fine level and carries the fused dots.
+    const bool with_dots = index == 0 && fuse_dots_ && options_.post_sweeps == 1;
+    const bool fold = l.staged && options_.post_sweeps > 0 && !with_dots;
     if (!fold) launch::prolong(l.n, l.aggregate.get(), c.x, x, status, stream_);
     tally(12.0 * l.n + 4.0 * c.n);
     smooth(l, rows, cols, vals, b, x, options_.post_sweeps, false, status, false,
