@@ -880,10 +880,15 @@ void Solver::inner(std::size_t index, const int* parent) {
     tally(bf16_bytes + 4.0 * n);
     launch::inner_first_dot(n, l.b.get(), p, q, l.x, t, sc, st, reducer(), stream_);
     tally(24.0 * n);
+    // z.q rides on the cycle's last sweep, unless a projection comes after it.
     const DevLevel* outer = inner_dot_;
-    inner_dot_ = &l;
+    inner_dot_ = nullspace_ ? nullptr : &l;
     cycle(index, t, l.z, st);
     inner_dot_ = outer;
+    if (nullspace_) {
+      reduce_into(ReduceMode::Dot, n, l.z, q, nullptr, nullptr, sc, 4, st);
+      launch::inner_beta(sc, st, stream_);
+    }
   } else {
     copy(p, l.z, n);
     launch::spmv(n, rows, cols, vals, p, q, parent, stream_);

@@ -11,16 +11,35 @@ from kutta_b200 import linalg as L
 pytestmark = pytest.mark.gpu
 
 
-class Model:
-    """The cycle and its flexible PCG in FP64 on the solver's own levels."""
+def _bf16_rows(v, row_ptr):
+    """The values that the mixed solve's coarse rows hold: max |a_ij| times the
+    BF16 rounding of a_ij over it (float operations)."""
+    import torch
+    row = np.repeat(np.arange(len(row_ptr) - 1), np.diff(row_ptr))
+    scale = np.zeros(len(row_ptr) - 1, np.float32)
+    np.maximum.at(scale, row, np.abs(v))
+    scale[scale == 0] = 1
+    share = v * (np.float32(1) / scale)[row]
+    return scale[row].astype(np.float64) * torch.from_numpy(share).bfloat16().double().numpy()
 
-    def __init__(self, solver, a, sweeps, coarse_sweeps=32):
+
+class Model:
+    """The cycle and its flexible PCG in FP64 on the solver's own levels; with
+    `constant`, corrections and coarse right-hand sides are projected."""
+
+    def __init__(self, solver, a, sweeps, k_levels=0, bf16=False, constant=False,
+                 coarse_sweeps=32):
         self.sweeps, self.coarse_sweeps = sweeps, coarse_sweeps
+        self.k_levels, self.constant = k_levels, constant
+        self.second_steps = 0
         self.levels = []
         for k, (n, rp, cl, vl, l1, ag) in enumerate(solver.levels()):
-            v = a.val.cpu().numpy() if k == 0 else vl
+            v = a.val.cpu().numpy() if k == 0 else _bf16_rows(vl, rp) if bf16 else vl
             A = sp.csr_matrix((v.astype(np.float64), cl, rp), shape=(n, n))
             self.levels.append((A, l1.astype(np.float64), ag))
+
+    def project(self, v):
+        return v - v.mean() if self.constant else v
 
     def smooth(self, k, b, x, sweeps):
         A, l1, _ = self.levels[k]
@@ -32,14 +51,15 @@ class Model:
         A, _, ag = self.levels[k]
         x = np.zeros(A.shape[0])
         if k + 1 == len(self.levels):
-            return self.smooth(k, b, x, self.coarse_sweeps)
+            return self.project(self.smooth(k, b, x, self.coarse_sweeps))
         x = self.smooth(k, b, x, self.sweeps)
         nc = self.levels[k + 1][0].shape[0]
         at = ag >= 0
-        rc = np.bincount(ag[at], (b - A @ x)[at], nc)
-        xc = self.inner(k + 1, rc) if k + 2 < len(self.levels) else self.cycle(k + 1, rc)
+        rc = self.project(np.bincount(ag[at], (b - A @ x)[at], nc))
+        inner = k + 2 < len(self.levels) and (self.k_levels == 0 or k < self.k_levels)
+        xc = self.inner(k + 1, rc) if inner else self.cycle(k + 1, rc)
         x[at] += xc[ag[at]]
-        return self.smooth(k, b, x, self.sweeps)
+        return self.project(self.smooth(k, b, x, self.sweeps))
 
     def inner(self, k, b):
         A = self.levels[k][0]
@@ -50,6 +70,7 @@ class Model:
         x, t = alpha * p, b - alpha * q
         if t @ t <= b @ b / 16:
             return x
+        self.second_steps += 1
         z = self.cycle(k, t)
         p = z - (z @ q) / pq * p
         q = A @ p
@@ -97,3 +118,32 @@ def test_plain_k_cycle_follows_fp64(cuda, make, max_levels, sweeps):
     got = x.cpu().numpy().astype(np.float64)
     assert st.converged and st.iterations == iterations
     assert np.linalg.norm(got - want) <= 1e-5 * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("k_levels", [1, 0], ids=["k_level1", "k_all"])
+@pytest.mark.parametrize("sweeps", [1, 2])
+@pytest.mark.parametrize("sides", [(17, 17, 17), (31, 30, 24)])
+def test_mixed_k_cycle_with_constant_nullspace(cuda, sides, sweeps, k_levels):
+    """One application of the preconditioner on a Neumann problem, whose inner
+    steps' products take the projected corrections: FP32 against FP64 on the same
+    BF16 rows, each of some twenty passes rounding to 6e-8."""
+    import torch
+    s = harness.poisson(*sides, 1, False, True)
+    a = L.upload(s)
+    options = dict(cycle=L.AmgCycle.K, pre_sweeps=sweeps, post_sweeps=sweeps,
+                   nullspace=L.NullSpace.Constant)
+    solver = L.make_mixed_solver(s, L.MixedOptions(
+        amg=L.AmgOptions(**options), k_cycle_levels=k_levels, absorb_singletons=False))
+    solver.refresh(a)
+    assert "smoothed instead of its dense inverse" in solver.describe()
+    b = np.random.default_rng(3).standard_normal(s.n).astype(np.float32)
+    z = torch.zeros(s.n, device="cuda")
+    solver.precondition(a, torch.from_numpy(b).cuda(), z)
+    # The same hierarchy, whose levels can be read back.
+    plain = L.make_amg_solver(L.SolverKind.AmgPcg, s, L.AmgOptions(coarse_rows=112, **options))
+    plain.refresh(a)
+    model = Model(plain, a, sweeps, k_levels, bf16=True, constant=True)
+    want = model.cycle(0, b.astype(np.float64))
+    err = np.linalg.norm(z.cpu().numpy() - want) / np.linalg.norm(want)
+    assert (model.second_steps == 1) == (k_levels == 1 or sides[0] == 17)
+    assert err <= 1e-6
