@@ -609,6 +609,58 @@ __device__ __forceinline__ void triangle_pair(int p, int& i, int& j) {
   j = p - i * (i + 1) / 2;
 }
 
+// The lower triangle of the operator into `dense` (n x n) and its diagonal into
+// diag0; all threads of the block, which the caller synchronises before and after.
+__device__ __forceinline__ void dense_lower(int n, const int* __restrict__ rows,
+                                            const int* __restrict__ cols,
+                                            const float* __restrict__ vals, double* dense,
+                                            double* diag0) {
+  for (int k = threadIdx.x; k < n * n; k += kDenseThreads) dense[k] = 0.0;
+  __syncthreads();
+  for (int i = threadIdx.x; i < n; i += kDenseThreads)
+    for (int j = rows[i]; j < rows[i + 1]; ++j) {
+      if (cols[j] <= i) dense[i * n + cols[j]] = vals[j];
+      if (cols[j] == i) diag0[i] = vals[j];
+    }
+}
+
+// The pivots of the Cholesky factor of `dense`, each element updated in the order
+// of the steps k: thread 0's `failed` (a pivot is not positive) and `smallest` (the
+// least share of its diagonal). Below this share the root-free elimination's
+// rounding may give a vanishing pivot another sign than the factor's, on which the
+// caller's refusal of an operator that is not SPD rests: a 4 x 5 Neumann Laplacian
+// has a positive last pivot in the factor and a negative one in the elimination.
+// The inverse of such an operator is not used for solves (Solver::choose_coarsest
+// asks for the same share).
+constexpr double kConditionedPivot = 1e-6;
+__device__ void cholesky_pivots(int n, double* dense, const double* diag0, double* column,
+                                bool& failed, double& smallest) {
+  __shared__ double pivot;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  failed = false;
+  smallest = 1.0;
+  for (int k = 0; k < n; ++k) {
+    if (threadIdx.x == 0) {
+      double d = dense[k * n + k];
+      if (!(d > 0.0)) {
+        failed = true;
+        d = 1.0;
+      } else {
+        smallest = fmin(smallest, d / diag0[k]);
+      }
+      pivot = sqrt(d);
+    }
+    __syncthreads();
+    for (int i = k + 1 + static_cast<int>(threadIdx.x); i < n; i += kDenseThreads)
+      column[i] = dense[i * n + k] / pivot;
+    __syncthreads();
+    for (int i = k + 1 + warp; i < n; i += kDenseThreads / 32)
+      for (int j = k + 1 + lane; j <= i; j += 32)
+        dense[i * n + j] = fma(-column[i], column[j], dense[i * n + j]);
+    __syncthreads();
+  }
+}
+
 __global__ void __launch_bounds__(kDenseThreads)
     k_dense_inverse_shared(int n, const int* __restrict__ rows, const int* __restrict__ cols,
                            const float* __restrict__ vals, double* __restrict__ W, double* error,
@@ -620,13 +672,7 @@ __global__ void __launch_bounds__(kDenseThreads)
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
   bool failed = false;
   double smallest = 1.0;  // thread 0's
-  for (int k = t; k < n * n; k += kDenseThreads) dense[k] = 0.0;
-  __syncthreads();
-  for (int i = t; i < n; i += kDenseThreads)
-    for (int j = rows[i]; j < rows[i + 1]; ++j) {
-      if (cols[j] <= i) dense[i * n + cols[j]] = vals[j];
-      if (cols[j] == i) diag0[i] = vals[j];
-    }
+  dense_lower(n, rows, cols, vals, dense, diag0);
   __syncthreads();
   double m[kDenseTile][kDenseTile];
 #pragma unroll
@@ -695,6 +741,11 @@ __global__ void __launch_bounds__(kDenseThreads)
       W[static_cast<std::size_t>(i) * n + j] = acc[c];
       W[static_cast<std::size_t>(j) * n + i] = acc[c];
     }
+  }
+  if (__syncthreads_or(t == 0 && (failed || smallest < kConditionedPivot))) {
+    dense_lower(n, rows, cols, vals, dense, diag0);
+    __syncthreads();
+    cholesky_pivots(n, dense, diag0, inverse, failed, smallest);
   }
   if (t == 0) {
     *error = failed ? 1.0 : 0.0;

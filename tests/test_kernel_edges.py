@@ -121,6 +121,43 @@ def test_dense_inverse_edges(cuda, n):
     assert np.max(np.abs(got - want)) <= bound * np.max(np.abs(want))
 
 
+def _cholesky_fails(dense):
+    """Whether a pivot of the FP64 Cholesky factor is not positive, each element
+    updated by one FMA per step (the exact rational value rounded once)."""
+    import math
+    from fractions import Fraction
+    n, fails = len(dense), False
+    lower = dense.tolist()
+    for k in range(n):
+        d = lower[k][k]
+        fails = fails or not d > 0
+        root = math.sqrt(d) if d > 0 else 1.0
+        column = [0.0] * (k + 1) + [lower[i][k] / root for i in range(k + 1, n)]
+        exact = [Fraction(c) for c in column]
+        for i in range(k + 1, n):
+            for j in range(k + 1, i + 1):
+                if column[i] and column[j]:
+                    lower[i][j] = float(Fraction(lower[i][j]) - exact[i] * exact[j])
+    return fails
+
+
+@pytest.mark.parametrize("sides", [(3, 1), (18, 1), (2, 3), (3, 4), (4, 5), (5, 6), (6, 7), (7, 8),
+                                   (8, 9), (9, 10), (4, 4, 4), (6, 4, 4), (7, 5, 3)])
+@pytest.mark.parametrize("random", [False, True])
+def test_dense_inverse_flags_singular_operators_by_the_factor(cuda, sides, random):
+    """Neumann Laplacians, singular but for rounding: whether one is refused as not
+    SPD follows the sign of the last pivot in the Cholesky factor."""
+    import torch
+    s = harness.poisson(*sides, *[1] * (4 - len(sides)), random, True)
+    a = L.upload(s)
+    inv = torch.empty(s.n * s.n, dtype=torch.float64, device="cuda")
+    flag = torch.full((1,), 7.0, dtype=torch.float64, device="cuda")
+    L.dense_inverse(a, inv, flag)
+    dense = np.zeros((s.n, s.n))
+    dense[np.repeat(np.arange(s.n), np.diff(s.row_ptr)), s.col] = s.val.astype(np.float32)
+    assert flag.item() == float(_cholesky_fails(dense))
+
+
 def _shuffled(s, seed):
     import scipy.sparse as sp
     rng = np.random.default_rng(seed)
