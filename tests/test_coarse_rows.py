@@ -127,3 +127,37 @@ def test_solve_beyond_the_split_guard(cuda, scale):
     got = x.cpu().numpy().astype(np.float64)
     assert (st.iterations, st.converged) == (o.iterations, o.converged)
     assert np.linalg.norm(got - o.x) <= 1e-5 * np.linalg.norm(o.x.astype(np.float64))
+
+
+@pytest.mark.gpu
+def test_updates_queued_past_the_end_are_skipped(cuda):
+    """Updates that a batch still queues after the one that converged load their
+    operators ahead, but form no products: on 1,572,864 tets such an update costs
+    half of a running one, and three quarters where the sweeps are worked out."""
+    import time
+    import torch
+    s = harness.box_system(64, 64, 64, tet=True, seed=1)
+    a = L.upload(s)
+    b = torch.from_numpy(s.b).cuda()
+
+    def first_solve(interval):
+        times, iterations = [], 0
+        for _ in range(4):
+            solver = L.make_amg_solver(L.SolverKind.AmgPcg, s, L.AmgOptions(
+                structure=M, pre_sweeps=2, post_sweeps=2))
+            solver.refresh(a)
+            x = torch.zeros(s.n, device="cuda")
+            torch.cuda.synchronize()
+            start = time.perf_counter()
+            st = solver.solve(a, x, b, L.SolveControl(1e-3, 1e-30, 500, interval))
+            torch.cuda.synchronize()
+            times.append(time.perf_counter() - start)
+            assert st.converged and iterations in (0, st.iterations)
+            iterations = st.iterations
+        return min(times), iterations
+
+    count = first_solve(1)[1]
+    exact, same = first_solve(count)
+    longer, again = first_solve(count + 40)
+    assert same == again == count
+    assert (longer - exact) / 40 < 0.62 * exact / count
