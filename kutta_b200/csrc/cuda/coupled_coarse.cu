@@ -224,8 +224,9 @@ __device__ __forceinline__ int entry_of(const int* __restrict__ rows, const int*
 }
 
 // Appends term `value` to entry e's list: counts it, or (terms set) places it.
-__device__ __forceinline__ int add_term(const CoupledLevel& l, int e, int value, int* count,
-                                        int* terms) {
+template <class Term>
+__device__ __forceinline__ int add_term(const CoupledLevel& l, int e, Term value, int* count,
+                                        Term* terms) {
   const int at = count[e]++;
   if (!terms) return 0;
   terms[l.term_at[e] + at] = value;
@@ -234,15 +235,16 @@ __device__ __forceinline__ int add_term(const CoupledLevel& l, int e, int value,
 
 // One thread owns a coarse row and visits its contributions in the reference's
 // order (fv_coupled.kern.h:424-524): members, then each one's faces or entries.
+template <class Term>
 __global__ void k_cpl_terms_fine(CoupledLevel l, CoupledTransfer t, int cells,
                                  const int* __restrict__ offsets, const int* __restrict__ adjacent,
-                                 const int* __restrict__ faces, int* count, int* terms,
+                                 const int* __restrict__ faces, int* count, Term* terms,
                                  int* term_faces) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= l.n) return;
   for (int mm = t.offsets[i]; mm < t.offsets[i + 1]; ++mm) {
     const int q = t.members[mm];
-    add_term(l, l.diag[i], ~q, count, terms);
+    add_term(l, l.diag[i], ~static_cast<Term>(q), count, terms);
     int slot = 0;
     for (int j = offsets[q]; j < offsets[q + 1]; ++j) {
       const int other = adjacent[j];
@@ -250,25 +252,26 @@ __global__ void k_cpl_terms_fine(CoupledLevel l, CoupledTransfer t, int cells,
       const int target = t.aggregate[other];
       const int e = target == i ? l.diag[i] : entry_of(l.rows, l.cols, i, target);
       if (e >= 0) {
-        const int at = add_term(l, e, slot * cells + q, count, terms);
+        const int at = add_term(l, e, static_cast<Term>(slot) * cells + q, count, terms);
         if (terms) term_faces[at] = faces[j];
       }
       ++slot;
     }
   }
 }
+template <class Term>
 __global__ void k_cpl_terms_coarse(CoupledLevel l, CoupledTransfer t, CoupledLevel f, int* count,
-                                   int* terms) {
+                                   Term* terms) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= l.n) return;
   for (int mm = t.offsets[i]; mm < t.offsets[i + 1]; ++mm) {
     const int row = t.members[mm];
-    add_term(l, l.diag[i], ~row, count, terms);
+    add_term(l, l.diag[i], ~static_cast<Term>(row), count, terms);
     for (int j = f.rows[row]; j < f.rows[row + 1]; ++j) {
       const int target = t.aggregate[f.cols[j]];
       const bool diagonal = j == f.diag[row];
       const int e = diagonal || target == i ? l.diag[i] : entry_of(l.rows, l.cols, i, target);
-      if (e >= 0) add_term(l, e, 2 * j + (diagonal ? 1 : 0), count, terms);
+      if (e >= 0) add_term(l, e, 2 * static_cast<Term>(j) + (diagonal ? 1 : 0), count, terms);
     }
   }
 }
@@ -276,8 +279,10 @@ __global__ void k_cpl_terms_coarse(CoupledLevel l, CoupledTransfer t, CoupledLev
 // Where a contribution's coefficient lies. Fine level: the packed records of
 // the ELL slot (the coefficients fv_coupled.kern.h:424-488 forms again: a, G, the
 // negative Rhie-Chow coefficient, and H as share times face area).
+template <class Term>
 struct FromFine {
   CoupledFine op;
+  const Term* terms;
   const int* faces;
   const float* cell;
   std::size_t cells;
@@ -285,7 +290,7 @@ struct FromFine {
   // Coefficient k of a term: a, gx, gy, gz, c, hx, hy, hz.
   // The face of a term comes from a list of its own beside the terms, so that
   // its load does not wait for the slot's link.
-  __device__ __forceinline__ float value(int term, int at, int k) const {
+  __device__ __forceinline__ float value(Term term, int at, int k) const {
     if (k < 4) return reinterpret_cast<const float*>(op.edge)[4 * static_cast<std::size_t>(term) + k];
     const float* face =
         reinterpret_cast<const float*>(op.face) + 4 * static_cast<std::size_t>(faces[at]);
@@ -297,18 +302,20 @@ struct FromFine {
     return k < 4 ? v : wc * v;
   }
   // Whether a term adds to the momentum sums.
-  static __device__ __forceinline__ bool momentum(int) { return true; }
+  static __device__ __forceinline__ bool momentum(Term) { return true; }
   static constexpr bool kOwnsAll = true;  // own() covers all ten sums
 };
+template <class Term>
 struct FromLevel {
   CoupledLevel f;
-  __device__ __forceinline__ float value(int term, int, int k) const {
+  const Term* terms;
+  __device__ __forceinline__ float value(Term term, int, int k) const {
     return reinterpret_cast<const float*>(f.entry)[8 * static_cast<std::size_t>(term >> 1) + k];
   }
   __device__ __forceinline__ float own(int row, int k) const {
     return f.d[k * static_cast<std::size_t>(f.n) + row];
   }
-  static __device__ __forceinline__ bool momentum(int term) { return (term & 1) == 0; }
+  static __device__ __forceinline__ bool momentum(Term term) { return (term & 1) == 0; }
   static constexpr bool kOwnsAll = false;  // only u, v, w
 };
 
@@ -317,12 +324,12 @@ struct FromLevel {
 template <class From>
 __device__ __forceinline__ void sum_entry(const CoupledLevel& l, const From& from, int e, int k) {
   const int begin = l.term_at[e], end = l.term_at[e + 1];
-  if (begin < end && l.terms[begin] < 0) return;  // a diagonal entry
+  if (begin < end && from.terms[begin] < 0) return;  // a diagonal entry
   float sum = 0.0f;
   for (int j = begin; j < end; j += 4) {
     float v[4];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) v[u] = j + u < end ? from.value(l.terms[j + u], j + u, k) : 0.0f;
+    for (int u = 0; u < 4; ++u) v[u] = j + u < end ? from.value(from.terms[j + u], j + u, k) : 0.0f;
 #pragma unroll
     for (int u = 0; u < 4; ++u)
       if (j + u < end) sum += v[u];
@@ -346,10 +353,10 @@ __device__ __forceinline__ void sum_diagonal(const CoupledLevel& l, const From& 
     for (int u = 0; u < 4; ++u) {
       add[u] = j + u < end;
       if (!add[u]) continue;
-      const int term = l.terms[j + u];
+      const auto term = from.terms[j + u];
       if (term < 0) {
         add[u] = From::kOwnsAll || k < 3;
-        if (add[u]) v[u] = from.own(~term, k);
+        if (add[u]) v[u] = from.own(static_cast<int>(~term), k);
       } else {
         add[u] = k >= 3 || From::momentum(term);
         if (add[u]) v[u] = from.value(term, j + u, which);
@@ -629,28 +636,47 @@ void coarse_rows(const CoupledLevel& l, const float4* x, const float4* b, float4
 
 namespace launch {
 
+template <class Term>
 void cpl_terms_fine(const CoupledLevel& l, const CoupledTransfer& t, const CoupledMeshDevice& m,
-                    int* count, int* terms, int* term_faces, cudaStream_t s) {
+                    int* count, Term* terms, int* term_faces, cudaStream_t s) {
   if (l.n <= 0) return;
   ++counter;
-  k_cpl_terms_fine<<<blocks_of(l.n, kBlock), kBlock, 0, s>>>(
+  k_cpl_terms_fine<Term><<<blocks_of(l.n, kBlock), kBlock, 0, s>>>(
       l, t, m.n, m.offsets, m.adjacent, m.faces, count, terms, term_faces);
 }
 
+template <class Term>
 void cpl_terms_coarse(const CoupledLevel& l, const CoupledTransfer& t, const CoupledLevel& f,
-                      int* count, int* terms, cudaStream_t s) {
+                      int* count, Term* terms, cudaStream_t s) {
   if (l.n <= 0) return;
   ++counter;
-  k_cpl_terms_coarse<<<blocks_of(l.n, kBlock), kBlock, 0, s>>>(l, t, f, count, terms);
+  k_cpl_terms_coarse<Term><<<blocks_of(l.n, kBlock), kBlock, 0, s>>>(l, t, f, count, terms);
 }
+
+template void cpl_terms_fine<int>(const CoupledLevel&, const CoupledTransfer&,
+                                  const CoupledMeshDevice&, int*, int*, int*, cudaStream_t);
+template void cpl_terms_fine<long long>(const CoupledLevel&, const CoupledTransfer&,
+                                        const CoupledMeshDevice&, int*, long long*, int*,
+                                        cudaStream_t);
+template void cpl_terms_coarse<int>(const CoupledLevel&, const CoupledTransfer&,
+                                    const CoupledLevel&, int*, int*, cudaStream_t);
+template void cpl_terms_coarse<long long>(const CoupledLevel&, const CoupledTransfer&,
+                                          const CoupledLevel&, int*, long long*, cudaStream_t);
 
 void cpl_galerkin_fine(const CoupledLevel& l, const CoupledFine& op, const float* cell, int cells,
                        float wc, cudaStream_t s) {
-  galerkin(l, FromFine{op, l.term_faces, cell, static_cast<std::size_t>(cells), wc}, s);
+  const std::size_t n = static_cast<std::size_t>(cells);
+  if (l.long_terms != nullptr)
+    galerkin(l, FromFine<long long>{op, l.long_terms, l.term_faces, cell, n, wc}, s);
+  else
+    galerkin(l, FromFine<int>{op, l.terms, l.term_faces, cell, n, wc}, s);
 }
 
 void cpl_galerkin_coarse(const CoupledLevel& l, const CoupledLevel& f, cudaStream_t s) {
-  galerkin(l, FromLevel{f}, s);
+  if (l.long_terms != nullptr)
+    galerkin(l, FromLevel<long long>{f, l.long_terms}, s);
+  else
+    galerkin(l, FromLevel<int>{f, l.terms}, s);
 }
 
 void cpl_coarse_prepare(const CoupledLevel& l, float* scratch, cudaStream_t s) {

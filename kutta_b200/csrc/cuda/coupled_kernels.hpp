@@ -65,7 +65,9 @@ struct CoupledLevel {
   // ~row says that a member row's own data comes next (diagonal entries only,
   // whose lists begin with one).
   const int* term_at = nullptr;
+  // Where the numbers of terms pass 31 bits, long_terms holds them instead.
   const int* terms = nullptr;
+  const long long* long_terms = nullptr;
   const int* term_faces = nullptr;  // from the fine level: each term's face
 };
 
@@ -109,11 +111,13 @@ void cpl_galerkin_fine(const CoupledLevel& l, const CoupledFine& op, const float
 void cpl_galerkin_coarse(const CoupledLevel& l, const CoupledLevel& f, cudaStream_t s);
 // The term lists, a thread per coarse row: first each entry's count of terms,
 // then (after an exclusive scan into term_at) the terms. Fine level: its
-// adjacency through the mesh; coarse: the level above's CSR.
+// adjacency through the mesh; coarse: the level above's CSR. Term is int or long long.
+template <class Term>
 void cpl_terms_fine(const CoupledLevel& l, const CoupledTransfer& t, const CoupledMeshDevice& m,
-                    int* count, int* terms, int* term_faces, cudaStream_t s);
+                    int* count, Term* terms, int* term_faces, cudaStream_t s);
+template <class Term>
 void cpl_terms_coarse(const CoupledLevel& l, const CoupledTransfer& t, const CoupledLevel& f,
-                      int* count, int* terms, cudaStream_t s);
+                      int* count, Term* terms, cudaStream_t s);
 // |G| row sums into scratch (3n), then cs and the block inverse.
 void cpl_coarse_prepare(const CoupledLevel& l, float* scratch, cudaStream_t s);
 

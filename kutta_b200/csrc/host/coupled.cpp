@@ -318,25 +318,27 @@ void CoupledSolver::precondition(const float4* rhs, float4*& out) {
   fine_smooth(out, rhs, options_.post_sweeps, false);
 }
 
-// The contributions of every Galerkin entry, listed once for the pattern.
+// The contributions of every Galerkin entry, listed once for the pattern. The
+// fine level numbers its terms by ELL slot, a coarse one by 2 x entry: in 64 bits
+// where those pass 31 (KUTTA_B200_COUPLED_LONG_TERMS=1: always, the same results).
 void CoupledSolver::build_terms(cudaStream_t s) {
+  const char* set = std::getenv("KUTTA_B200_COUPLED_LONG_TERMS");
+  const bool always = set && std::string(set) == "1";
   for (std::size_t k = 0; k < levels_.size(); ++k) {
     auto& l = levels_[k];
     const auto& t = transfers_[k].view;
     const std::size_t entries = l.op.nnz;
-    // The fine level numbers its terms by ELL slot, a coarse one by 2 x entry.
-    KB2_REQUIRE(k == 0 ? static_cast<long long>(width_) * n_ <= 0x7fffffffLL
-                       : levels_[k - 1].op.nnz < (1 << 30),
-                "coupled: operator exceeds the 32-bit index range");
+    const long long numbers =
+        k == 0 ? static_cast<long long>(width_) * n_ : 2LL * levels_[k - 1].op.nnz;
     DArray<int> count(entries + 1), scratch(launch::scan_scratch(l.op.nnz));
-    const auto list = [&](int* terms) {
+    const auto list = [&](auto* terms) {
       cuda_check(cudaMemsetAsync(count.get(), 0, (entries + 1) * sizeof(int), s), "memset");
       if (k == 0)
         launch::cpl_terms_fine(l.op, t, mesh_, count.get(), terms, l.term_faces.get(), s);
       else
         launch::cpl_terms_coarse(l.op, t, levels_[k - 1].op, count.get(), terms, s);
     };
-    list(nullptr);
+    list(static_cast<int*>(nullptr));
     own(l.term_at, entries + 1);
     launch::exclusive_scan(l.op.nnz, count.get(), l.term_at.get(), scratch.get(), s);
     l.op.term_at = l.term_at.get();
@@ -345,11 +347,17 @@ void CoupledSolver::build_terms(cudaStream_t s) {
                                cudaMemcpyDeviceToHost, s),
                "readback");
     wait(s);
-    own(l.terms, static_cast<std::size_t>(total));
     if (k == 0) own(l.term_faces, static_cast<std::size_t>(total));
-    list(l.terms.get());
-    l.op.terms = l.terms.get();
     l.op.term_faces = l.term_faces.get();
+    if (always || numbers > 0x7fffffffLL) {
+      own(l.long_terms, static_cast<std::size_t>(total));
+      list(l.long_terms.get());
+      l.op.long_terms = l.long_terms.get();
+    } else {
+      own(l.terms, static_cast<std::size_t>(total));
+      list(l.terms.get());
+      l.op.terms = l.terms.get();
+    }
     wait(s);  // count and scratch are released here
   }
 }

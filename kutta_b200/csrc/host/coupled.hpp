@@ -77,6 +77,7 @@ class CoupledSolver {
   struct Level {
     CoupledLevel op;
     DArray<int> rows, cols, diag, term_at, terms, term_faces;
+    DArray<long long> long_terms;
     DArray<float4> entry;
     DArray<float> d;
     DArray<float4> b, store[2];

@@ -106,3 +106,66 @@ def test_galerkin_sums_match_their_order(cuda):
     got = np.concatenate([[c["a"], c["c"]], c["g"].reshape(3, cz), c["h"].reshape(3, cz)])
     assert np.array_equal(bits(got), bits(want))
     assert np.array_equal(bits(c["d"][:3 * nc]), bits(momentum.reshape(-1)))
+
+
+def test_long_term_lists_change_no_bits(cuda, monkeypatch):
+    """The Galerkin terms numbered in 64 bits, on every level."""
+    want = _solved("tet")
+    monkeypatch.setenv("KUTTA_B200_COUPLED_LONG_TERMS", "1")
+    got = _solved("tet")
+    for k in range(1, want.levels()):
+        a, b = want.level(k), got.level(k)
+        for key in a:
+            assert np.array_equal(a[key], b[key]), (k, key)
+    assert np.array_equal(bits(want.copy("x")), bits(got.copy("x")))
+
+
+def _hub_mesh(n):
+    """A closed ring of n cells, each with a face to one cell more: connectivity
+    only, the cells' places random and the areas along the distances."""
+    rng = np.random.default_rng(1)
+    centroid = rng.uniform(-1, 1, (n + 1, 3))
+    ring = np.arange(n - 1)
+    owner = np.concatenate([ring, [0], np.arange(n)])
+    neighbour = np.concatenate([ring + 1, [n - 1], np.full(n, n)])
+    order = np.lexsort((neighbour, owner))
+    owner, neighbour = owner[order], neighbour[order]
+    d = centroid[neighbour] - centroid[owner]
+    area = d / np.linalg.norm(d, axis=1)[:, None] * np.where(neighbour == n, 1e-7, 1e-3)[:, None]
+    fc = 0.5 * (centroid[owner] + centroid[neighbour])
+    return H._mesh_arrays(centroid, np.full(n + 1, 1e-6), owner, neighbour, area, fc,
+                          np.zeros(0, np.int64))
+
+
+@pytest.mark.parametrize("n", [500, 46_345])
+def test_galerkin_operator_of_a_hub_cell(cuda, n):
+    """One cell that borders all others makes the fine slots cells x cells: 60 GB
+    and more than 2^31 of them at the larger size. The first coarse operator is the
+    fine one between prolongation and restriction, whose float sums of up to n terms
+    are within 1e-4 of each other's."""
+    import torch
+    if n > 1000 and torch.cuda.mem_get_info()[0] < 80 << 30:
+        pytest.skip("80 GB of device memory")
+    mesh = _hub_mesh(n)
+    fields = H.flow_fields(mesh, 3, reference=0)
+    dev = {k: torch.from_numpy(v).cuda() if isinstance(v, np.ndarray) else v
+           for k, v in fields.items()}
+    s = L.CoupledSolver(mesh, 0, L.CoupledOptions())
+    rows, diag = (torch.from_numpy(mesh[k]).cuda() for k in ("pattern_row_ptr", "pattern_diag"))
+    for k, c in enumerate("uvw"):
+        s.capture_diagonal(k, rows, diag, dev["momentum_" + c], dev["physical_" + c])
+    s.solve(dev, L.SolveControl(0.1, 1e-12, 2))
+    coarse = s.level(1)
+    nc = len(coarse["diag"])
+    x = torch.randn(4 * nc, device="cuda", generator=torch.Generator("cuda").manual_seed(1))
+    zero, product = torch.zeros_like(x), torch.zeros_like(x)
+    s.level_apply(1, "residual", x, zero, product)
+    fine = torch.zeros(4 * (n + 1), device="cuda")
+    s.level_apply(1, "prolong", x, None, fine)
+    y, want = torch.zeros_like(fine), torch.zeros_like(x)
+    s.apply("spmv", fine, None, y)
+    s.level_apply(1, "restrict", y, None, want)
+    got, want = -product.view(-1, 4).double(), want.view(-1, 4).double()
+    assert nc > 48 and torch.isfinite(got).all()
+    for k in range(4):
+        assert (got - want)[:, k].norm() <= 1e-4 * want[:, k].norm()
