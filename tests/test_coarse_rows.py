@@ -72,13 +72,58 @@ CASES = {
     # Rows at and around a block's 32, 64 and 128, and one small level only.
     **{f"poisson{n}": lambda n=n: harness.poisson(n, 1) for n in (25, 33, 64, 65, 129, 257)},
     "poisson2d": lambda: harness.poisson(47, 43, 1, 100.0),
-    # The one-block levels' edges: 2,048 and 2,049 rows below the fine level.
+    # A smallest level too large for one block, and two that fit one.
     "hex": lambda: harness.box_system(27, 23, 26, tet=False, seed=4),
     "tet": lambda: harness.box_system(13, 17, 11, tet=True, seed=5),
     # Rows longer than what a block stages at once (1,024 and 2,048 entries).
     "hub_small": lambda: _hub(3_000, 1_400, 3, 1),
     "hub_large": lambda: _hub(20_000, 5_000, 4, 2),
 }
+
+
+# (system, coarse_rows, the rows and entries of some levels below the fine one).
+ONE_BLOCK = {
+    # The most rows a level in one block has, and one more; on the way down levels
+    # of 256, 32 and 4 rows, or of 257, 33 and 5.
+    "rows2048": (lambda: harness.poisson(16384, 1), 24, {1: (2048, 6142), 3: (32, 94)}),
+    "rows2049": (lambda: harness.poisson(16392, 1), 24, {1: (2049, 6145), 3: (33, 97)}),
+    # Coarsest levels about 24 rows, up to which a launch of its own takes the
+    # coarsest, and 32, up to which a warp of the one block does.
+    **{f"coarsest{c}": (lambda c=c: harness.poisson(8 * c, 1), c, {1: (c, 3 * c - 2)})
+       for c in (24, 25, 32, 33)},
+    # Two tet levels below and above 16,384 entries, the most one in a block has.
+    "entries11452": (lambda: harness.box_system(14, 14, 12, tet=True, seed=5), 24,
+                     {2: (1384, 11452), 3: (988, 6352)}),
+    "entries16696": (lambda: harness.box_system(16, 15, 14, tet=True, seed=5), 24,
+                     {2: (1984, 16696), 3: (1426, 9532)}),
+}
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("post", [3, 1])
+@pytest.mark.parametrize("name", ONE_BLOCK)
+def test_one_block_edges_match_oracle(cuda, name, post):
+    """At the limits of the levels that run in one block, AMG-BiCGStab (whose
+    sweeps down and up may differ) as below."""
+    import torch
+    make, coarse_rows, sizes = ONE_BLOCK[name]
+    s = make()
+    a = L.upload(s)
+    solver = L.make_amg_solver(L.SolverKind.AmgBicgstab, s, L.AmgOptions(
+        pre_sweeps=3, post_sweeps=post, coarse_rows=coarse_rows))
+    solver.refresh(a)
+    levels = solver.levels()
+    for k, (rows, entries) in sizes.items():
+        assert (levels[k][0], len(levels[k][2])) == (rows, entries), [lv[0] for lv in levels]
+    x = torch.zeros(s.n, device="cuda")
+    b = s.b.astype(f32)
+    st = solver.solve(a, x, torch.from_numpy(b).cuda(), L.SolveControl(1e-4, 1e-38, 200))
+    o = O.solve(s, O.AMG_BICGSTAB, b=b, rel_tol=1e-4, abs_tol=1e-38, max_iter=200,
+                opts=O.options(O.AMG_BICGSTAB, pre_sweeps=3, post_sweeps=post,
+                               coarse_rows=coarse_rows))
+    got = x.cpu().numpy().astype(np.float64)
+    assert (st.iterations, st.converged) == (o.iterations, o.converged)
+    assert np.linalg.norm(got - o.x) <= 1e-5 * np.linalg.norm(o.x.astype(np.float64))
 
 
 @pytest.mark.gpu

@@ -24,18 +24,21 @@ def bits(a):
     return np.ascontiguousarray(a, f32).view(np.uint32)
 
 
-def _solved(name):
+def _solve(mesh, fields, reference=-1, options=None, max_iter=20):
     import torch
-    mesh = BOXES[name]()
-    fields = H.flow_fields(mesh, 3)
     dev = {k: torch.from_numpy(v).cuda() if isinstance(v, np.ndarray) else v
            for k, v in fields.items()}
-    s = L.CoupledSolver(mesh, -1, L.CoupledOptions())
+    s = L.CoupledSolver(mesh, reference, options or L.CoupledOptions())
     rows, diag = (torch.from_numpy(mesh[k]).cuda() for k in ("pattern_row_ptr", "pattern_diag"))
     for k, c in enumerate("uvw"):
         s.capture_diagonal(k, rows, diag, dev["momentum_" + c], dev["physical_" + c])
-    s.solve(dev, L.SolveControl(0.1, 1e-12, 20))
+    s.solve(dev, L.SolveControl(0.1, 1e-12, max_iter))
     return s
+
+
+def _solved(name):
+    mesh = BOXES[name]()
+    return _solve(mesh, H.flow_fields(mesh, 3))
 
 
 @pytest.mark.parametrize("name", BOXES)
@@ -58,6 +61,74 @@ def test_level_rows_match_oracle(cuda, name):
             s.level_apply(k, op, dx, db, y)
             got = y.cpu().numpy().reshape(n, 4).T.reshape(-1)
             assert np.array_equal(bits(got), bits(w)), (k, op)
+
+
+class Cycle:
+    """The V-cycle on the oracle's row kernels, with the device's operators."""
+
+    def __init__(self, s, mesh, fields, o):
+        self.mesh, self.o = mesh, o
+        self.wc = f32(fields["density"] * fields["velocity_scale"])
+        self.cell, self.coefficient = s.copy("cell"), s.copy("coefficient")
+        self.edge = O.fine_coefficients(mesh, self.cell, fields["viscosity"], fields["mass"],
+                                        fields["face_weights"], self.wc)
+        self.levels = [s.level(k) for k in range(1, s.levels())]
+
+    def fine_row(self, x):
+        return O.fine_row(self.mesh, self.cell, self.edge, self.coefficient, x, self.wc)
+
+    def sweeps(self, k, x, b, count, first):
+        for q in range(count):
+            zero = first and q == 0
+            if k == 0:
+                x = O.fine_smooth(self.mesh, self.cell, self.edge, self.coefficient, x, b, self.wc,
+                                  self.o.smoother_damping, zero)
+            else:
+                x = O.coarse_smooth(self.levels[k - 1], x, b, self.o.smoother_damping, zero)
+        return x
+
+    def __call__(self, b, k=0):
+        if k == len(self.levels):
+            return self.sweeps(k, None, b, self.o.coarsest_sweeps, True)
+        n = len(b) // 4
+        x = self.sweeps(k, None, b, self.o.pre_sweeps, True)
+        r = b - (self.fine_row(x) if k == 0 else O.coarse_row(self.levels[k - 1], x))
+        aggregate = self.levels[k]["aggregate"]
+        members = np.argsort(aggregate, kind="stable").astype(np.int32)
+        offsets = np.concatenate([[0], np.cumsum(np.bincount(aggregate))])
+        c = self(O.restrict(offsets, members, r.astype(f32), n), k + 1).reshape(4, -1)
+        x = (x.reshape(4, n) + c[:, aggregate]).reshape(-1)
+        return self.sweeps(k, x, b, self.o.post_sweeps, False)
+
+
+@pytest.mark.parametrize("tail", ["1", "0"], ids=["tail", "separate"])
+@pytest.mark.parametrize("post", [0, 1, 2])
+@pytest.mark.parametrize("name", BOXES)
+def test_one_update_follows_the_oracle(cuda, name, post, tail, monkeypatch):
+    """The first BiCGStab update with the whole V-cycle, its folded transfers and
+    first sweeps among it, on a coarse level above 16,384 rows and those below: the
+    cycle rounds as the oracle's, and FP64 dots give the two coefficients, so x
+    differs by float roundings only."""
+    monkeypatch.setenv("KUTTA_B200_COUPLED_TAIL", tail)
+    mesh = BOXES[name]()
+    fields, o = H.flow_fields(mesh, 3), L.CoupledOptions(post_sweeps=post)
+    s = _solve(mesh, fields, options=o, max_iter=1)
+    cycle = Cycle(s, mesh, fields, o)
+    n = len(cycle.levels[0]["diag"])
+    assert (n > 16384) == (name == "hex") and len(cycle.levels[1]["diag"]) < 16384
+    r = s.copy("rhs")
+
+    def dot(a, b):
+        return a.astype(np.float64) @ b.astype(np.float64)
+
+    z = cycle(r)
+    v = cycle.fine_row(z)
+    alpha = dot(r, r) / dot(r, v)
+    sv = (r - f32(alpha) * v).astype(f32)
+    zs = cycle(sv)
+    t = cycle.fine_row(zs)
+    want = alpha * z.astype(np.float64) + dot(t, sv) / dot(t, t) * zs
+    assert np.linalg.norm(s.copy("x") - want) <= 1e-6 * np.linalg.norm(want)
 
 
 def _add(sum_, error, value):
@@ -147,14 +218,7 @@ def test_galerkin_operator_of_a_hub_cell(cuda, n):
     if n > 1000 and torch.cuda.mem_get_info()[0] < 80 << 30:
         pytest.skip("80 GB of device memory")
     mesh = _hub_mesh(n)
-    fields = H.flow_fields(mesh, 3, reference=0)
-    dev = {k: torch.from_numpy(v).cuda() if isinstance(v, np.ndarray) else v
-           for k, v in fields.items()}
-    s = L.CoupledSolver(mesh, 0, L.CoupledOptions())
-    rows, diag = (torch.from_numpy(mesh[k]).cuda() for k in ("pattern_row_ptr", "pattern_diag"))
-    for k, c in enumerate("uvw"):
-        s.capture_diagonal(k, rows, diag, dev["momentum_" + c], dev["physical_" + c])
-    s.solve(dev, L.SolveControl(0.1, 1e-12, 2))
+    s = _solve(mesh, H.flow_fields(mesh, 3, reference=0), reference=0, max_iter=2)
     coarse = s.level(1)
     nc = len(coarse["diag"])
     x = torch.randn(4 * nc, device="cuda", generator=torch.Generator("cuda").manual_seed(1))
