@@ -34,11 +34,17 @@ inline void raise_shared_limit(const void* kernel, int bytes,
 // kernel's end and the next one's start is a large share of the time. Every
 // solve-path kernel is launched with programmatic stream serialization: the
 // next kernel may be scheduled while the current one drains, and it waits
-// (griddepcontrol.wait, its very first instruction) until the previous grid
-// has completed and its memory is visible before touching any memory. So the
-// ordering of every read and write is exactly that of ordinary stream order;
-// only the launch latency overlaps. After its own wait a kernel lets its
-// dependents be scheduled.
+// (griddepcontrol.wait) until the previous grid has completed and its memory is
+// visible. After its own wait a kernel lets its dependents be scheduled, so a
+// kernel that starts early knows every grid but the previous one to be complete.
+//
+// Most kernels wait before touching any memory: their reads and writes are
+// ordered as in an ordinary stream, and only the launch latency overlaps. The
+// coarse levels' kernels (coarse_rows.cu, coupled_coarse.cu, mixed_tail.cu) load
+// before the wait what a solve does not change: patterns, operators, inverses.
+// Such an operand must not be written by the kernel directly before: it comes
+// from setup or a refresh, behind a host wait or at least one kernel earlier.
+// Vectors, scalars and the status are read after the wait only.
 __device__ __forceinline__ void pdl_entry() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

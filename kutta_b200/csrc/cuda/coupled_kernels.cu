@@ -261,7 +261,9 @@ __global__ void __launch_bounds__(kBlock, 8) k_cpl_fine_spmv(int n, int width, C
 
 // y = J x with the BiCGStab's reduction of y fused in: w.y and alpha, or (kDual)
 // y.y, y.w and omega. The FP64 sums need more than 32 registers, so the grid is
-// sized for six blocks per SM (still one wave).
+// sized for six blocks per SM (still one wave). A cell's four products are added
+// before the running sum, a component at a time in the separate reduction, so the
+// two may differ in the last bits of FP64.
 constexpr int kDotBlocks = 6;
 template <bool kDual>
 __global__ void __launch_bounds__(kBlock, kDotBlocks)

@@ -595,7 +595,7 @@ __global__ void k_dense_copy(std::size_t count, const double* __restrict__ from,
 // the current row of X, which their owners put into shared memory as they
 // update them for the next step, and one barrier. `L` (global) is not used. (A
 // Cholesky factor and a separate substitution in shared memory, five barriers,
-// a root and a column of divisions per step, took 231 us at 94 rows; this 118.)
+// a root and a column of divisions per step, took 231 us at 107 rows; this 118.)
 constexpr int kSharedDense = 112;
 constexpr int kDenseThreads = 1024;
 constexpr int kDenseTile = 4;  // elements of a thread in each direction

@@ -167,9 +167,7 @@ class Solver {
   std::size_t tail_start_ = 0;
   double tail_bytes_ = 0;
   launch::TailPlan tail_{};
-  // The plain V-cycle's choice of row kernels per level, and its smallest
-  // levels (>= plain_tail_start_, 0: none) in one block.
-  // The mixed solve's: levels >= mixed_tail_start_ (0: none) in one block.
+  // The mixed solve's smallest levels (>= mixed_tail_start_, 0: none) in one block.
   void plan_mixed_tail(cudaStream_t s);
   launch::MixedTail mixed_tail_{};
   std::vector<launch::MixedTail::Values> mixed_tail_values_;
@@ -177,6 +175,8 @@ class Solver {
   std::size_t mixed_tail_start_ = 0;
   double mixed_tail_bytes_ = 0;
   static bool near_columns(const DevLevel& l, cudaStream_t s);
+  // The plain cycle's choice of row kernels per level, and the V-cycle's smallest
+  // levels (>= plain_tail_start_, 0: none) in one block.
   void plan_plain(cudaStream_t s);
   static std::vector<int> row_pointers(const DevLevel& l, cudaStream_t s);
   std::size_t plain_tail_start_ = 0;
