@@ -73,6 +73,7 @@ __global__ void __launch_bounds__(kBlock) k_staged_rows(
     const int* __restrict__ aggregate, const float* __restrict__ coarse,
     const int* __restrict__ order) {
   constexpr int kStage = kPer * kBlock;
+  static_assert(kStage == launch::kStagedEntries * (kRows / launch::kStagedRows), "adds_too_long");
   constexpr bool kProlong = kMode == Rows::SmoothProlonged;
   __shared__ float2 staged[kStage];
   const int tid = threadIdx.x;

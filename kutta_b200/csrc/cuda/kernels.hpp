@@ -159,6 +159,9 @@ void level_rows(int n, const int* rows, const int* diag, float* vals, const Leve
 // kStagedSmall rows take blocks of 64 rows, more take 128 (see staged()).
 // With order, rows [128 k, 128 k + 128) are taken in that order (longest first).
 constexpr int kStagedSmall = 16384, kStagedHub = 64;
+// Rows of a block and the entries that it stages at a time (twice these for more
+// than kStagedSmall rows).
+constexpr int kStagedRows = 64, kStagedEntries = 1024;
 void staged_residual(int n, const int* rows, const int* cols, const float* vals, const float* x,
                      const float* b, float* r, const int* status, const int* order,
                      cudaStream_t s);

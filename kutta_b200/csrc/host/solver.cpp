@@ -162,7 +162,7 @@ Solver::Solver(Kind kind, const CsrView& a, const Options& options,
     if (options_.fused_tail && options_.coarse_bf16 && !nullspace_) plan_tail();
     if (options_.packed_fine) plan_packed(a, s);
   } else if (amg()) {
-    plan_plain(s);
+    plan_plain(a, s);
   }
   for (std::size_t i = 0; amg() && i < levels_.size(); ++i) {
     surplus(i);  // allocated here rather than in the first refresh
@@ -190,21 +190,70 @@ std::vector<int> Solver::row_pointers(const DevLevel& l, cudaStream_t s) {
 // with a longest of 165: 3.8 against 18.4 us; 48,848 with 123: 5.2 against 18.8
 // us) and, above, on levels whose longest row has more than 8 entries (159,785
 // rows of up to 18: 5.6 against 8.6 us). Short rows on many threads are faster
-// direct (262,144 rows of up to 7: 5.0 against 6.7 us). The one-block tail takes
+// direct (262,144 rows of up to 7: 5.0 against 6.7 us), and so are levels where
+// many long rows share a block (adds_too_long). The one-block tail takes
 // the levels from the first with at most kPlainTailRows rows and
 // kPlainTailSlots entries: beyond that one SM is slower than a launch per
 // sweep.
-void Solver::plan_plain(cudaStream_t s) {
+
+// A staged block adds the entries that it has staged with a thread per row, so it
+// takes as many additions one after the other as the longest of those rows has
+// there, summed over what it stages in turn; a thread that walks its row takes the
+// row's entries, each some twelve additions' time. Rows of 190 entries: 37 us a
+// sweep staged against 45 direct (6,000 rows), of 251: 58.7 against 59.3, of 372:
+// 119 against 84; 8,211 rows of a graph with hubs beside one another (44 on
+// average, longest 988): 240 against 155.
+bool Solver::adds_too_long(const int* rows, int n) {
+  const bool few = n <= launch::kStagedSmall;
+  const int block = few ? launch::kStagedRows : 2 * launch::kStagedRows;
+  const int stage = few ? launch::kStagedEntries : 2 * launch::kStagedEntries;
+  long long most = 0;
+  int longest = 0;
+  for (int i0 = 0; i0 < n; i0 += block) {
+    long long additions = 0;
+    int i = i0;
+    const int i1 = std::min(n, i0 + block), last = rows[i1];
+    for (int base = rows[i0]; base < last;) {
+      const int end = last - base > stage ? base + stage : last;
+      int here = 0;
+      while (i < i1) {
+        here = std::max(here, std::min(rows[i + 1], end) - std::max(rows[i], base));
+        if (rows[i + 1] > end) break;  // goes on in the next stage
+        ++i;
+      }
+      additions += here;
+      base = end;
+    }
+    most = std::max(most, additions);
+    for (int r = i0; r < i1; ++r) longest = std::max(longest, rows[r + 1] - rows[r]);
+  }
+  return most > 14LL * longest;
+}
+
+void Solver::plan_plain(const CsrView& a, cudaStream_t s) {
   constexpr int kDirectRows = 1 << 16, kDirectLongest = 8;
+  // The levels' row pointers, read back together.
+  std::vector<std::vector<int>> pointers(levels_.size());
+  for (std::size_t i = 1; i < levels_.size(); ++i) {
+    const auto& l = levels_[i];
+    pointers[i].resize(static_cast<std::size_t>(l.n) + 1);
+    cuda_check(cudaMemcpyAsync(pointers[i].data(), l.row_ptr.get(),
+                               sizeof(int) * pointers[i].size(), cudaMemcpyDeviceToHost, s),
+               "row lengths");
+  }
+  wait(s);
   for (std::size_t i = 0; i < levels_.size(); ++i) {
     auto& l = levels_[i];
+    const int* rows = i == 0 ? a.row_ptr : pointers[i].data();
     l.staged = l.n <= kDirectRows;
-    if (i == 0 || l.n <= launch::kStagedSmall) continue;
-    const std::vector<int> rows = row_pointers(l, s);
+    if (i == 0 || l.n <= launch::kStagedSmall) {
+      l.staged = l.staged && !adds_too_long(rows, l.n);
+      continue;
+    }
     int longest = 0;
     for (int k = 0; k < l.n; ++k) longest = std::max(longest, rows[k + 1] - rows[k]);
-    l.staged = l.staged || longest > kDirectLongest;
-    if (longest < launch::kStagedHub) continue;
+    l.staged = (l.staged || longest > kDirectLongest) && !adds_too_long(rows, l.n);
+    if (!l.staged || longest < launch::kStagedHub) continue;
     std::vector<int> order(static_cast<std::size_t>(l.n));
     std::iota(order.begin(), order.end(), 0);
     for (int k = 0; k < l.n; k += 128)
@@ -226,7 +275,7 @@ void Solver::plan_plain(cudaStream_t s) {
     auto& l = levels_[start - 1];
     if (l.n > launch::kPlainTailRows || l.nnz > launch::kPlainTailSlots) break;
     // Rows in order of length, their entries in slices of 32 rows.
-    const std::vector<int> rows = row_pointers(l, s);
+    const std::vector<int>& rows = pointers[start - 1];
     std::vector<int> order(static_cast<std::size_t>(l.n)), first(order.size());
     std::iota(order.begin(), order.end(), 0);
     std::stable_sort(order.begin(), order.end(), [&](int p, int q) {

@@ -177,7 +177,8 @@ class Solver {
   static bool near_columns(const DevLevel& l, cudaStream_t s);
   // The plain cycle's choice of row kernels per level, and the V-cycle's smallest
   // levels (>= plain_tail_start_, 0: none) in one block.
-  void plan_plain(cudaStream_t s);
+  void plan_plain(const CsrView& a, cudaStream_t s);
+  static bool adds_too_long(const int* rows, int n);
   static std::vector<int> row_pointers(const DevLevel& l, cudaStream_t s);
   std::size_t plain_tail_start_ = 0;
   double plain_tail_bytes_ = 0;

@@ -68,6 +68,25 @@ def _hub(n, degree, hubs, seed):
     return harness.HostSystem(row_ptr, col, diag, val, rng.standard_normal(n).astype(f32))
 
 
+def _long_rows(n, length, seed):
+    """An M-matrix of rows of about `length` entries."""
+    rng = np.random.default_rng(seed)
+    i = np.repeat(np.arange(n), length // 2)
+    j = (i + rng.integers(1, n, len(i))) % n
+    pairs = np.unique(np.minimum(i, j).astype(np.int64) * n + np.maximum(i, j))
+    i, j = pairs // n, pairs % n
+    w = rng.uniform(0.1, 1, len(i)).astype(f32).astype(np.float64)
+    total = np.bincount(np.concatenate([i, j]), np.concatenate([w, w]), n) * 1.01 + 1e-3
+    row = np.concatenate([i, j, np.arange(n)])
+    col = np.concatenate([j, i, np.arange(n)])
+    val = np.concatenate([-w, -w, np.nextafter(total.astype(f32), f32(np.inf))])
+    order = np.lexsort((col, row))
+    row, col, val = row[order], col[order].astype(np.int32), val[order].astype(np.float64)
+    row_ptr = np.concatenate([[0], np.cumsum(np.bincount(row, minlength=n))]).astype(np.int32)
+    diag = np.nonzero(row == col)[0].astype(np.int32)
+    return harness.HostSystem(row_ptr, col, diag, val, rng.standard_normal(n).astype(f32))
+
+
 CASES = {
     # Rows at and around a block's 32, 64 and 128, and one small level only.
     **{f"poisson{n}": lambda n=n: harness.poisson(n, 1) for n in (25, 33, 64, 65, 129, 257)},
@@ -78,6 +97,8 @@ CASES = {
     # Rows longer than what a block stages at once (1,024 and 2,048 entries).
     "hub_small": lambda: _hub(3_000, 1_400, 3, 1),
     "hub_large": lambda: _hub(20_000, 5_000, 4, 2),
+    # Many long rows in a block: formed by the block (150), a thread per row (400).
+    **{f"rows{k}": lambda k=k: _long_rows(1_500, k, 3) for k in (150, 400)},
 }
 
 
@@ -206,3 +227,40 @@ def test_updates_queued_past_the_end_are_skipped(cuda):
     longer, again = first_solve(count + 40)
     assert same == again == count
     assert (longer - exact) / 40 < 0.62 * exact / count
+
+
+@pytest.mark.gpu
+def test_levels_of_long_rows_are_not_slower_than_a_thread_per_row(cuda):
+    """2,000 rows of some 480 entries, where a block would add the entries of a few
+    rows at a time: a sweep of the solve takes no more than 1.3 times the sweep that
+    amg_smooth launches, a thread per row (167 against 99 us when a block did)."""
+    import time
+    import torch
+    s = _long_rows(2_000, 480, 1)
+    a = L.upload(s)
+    b = torch.from_numpy(s.b).cuda()
+
+    def best(run):
+        times = []
+        for _ in range(5):
+            torch.cuda.synchronize()
+            start = time.perf_counter()
+            run()
+            torch.cuda.synchronize()
+            times.append(time.perf_counter() - start)
+        return min(times)
+
+    def solve(sweeps):
+        solver = L.make_amg_solver(L.SolverKind.AmgPcg, s, L.AmgOptions(
+            coarse_sweeps=sweeps, max_levels=1, setup=L.Setup.Host))
+        solver.refresh(a)
+        x = torch.zeros_like(b)
+        return best(lambda: solver.solve(a, x.zero_(), b, L.SolveControl(1e-30, 1e-38, 1)))
+
+    x, y, inverse = torch.zeros_like(b), torch.zeros_like(b), torch.ones_like(b)
+
+    def direct():
+        for _ in range(100):
+            L.amg_smooth(a, x, b, inverse, y)
+
+    assert (solve(300) - solve(100)) / 200 <= 1.3 * best(direct) / 100
