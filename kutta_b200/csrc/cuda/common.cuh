@@ -306,17 +306,26 @@ __device__ __forceinline__ void row_values(const float* vals, int begin, int end
 
 // krylov_diagonal's row (src/kutta/kernels/linalg.kern.h:52-70): the inverse
 // (L1) diagonal of row i into inverse[i]; returns its invalid flag (0 valid,
-// 1 zero diagonal, 2 nonfinite, 3 negative diagonal under L1).
+// 1 zero diagonal, 2 nonfinite, 3 negative diagonal under L1). kBatched: the
+// row's loads issued together, which pays among a longer pass; in a kernel of its
+// own the entries one by one are 0.8 us faster (4.7 against 5.5 at 17,500 rows).
+template <bool kBatched = true>
 __device__ __forceinline__ float diagonal_row(int i, const int* __restrict__ rows,
                                               const int* __restrict__ diag,
                                               const float* vals, float* inverse, int use_l1) {
   const int at = diag[i];
   const float d = vals[at];
   float off = 0.0f, bad = 0.0f;
-  row_values(vals, rows[i], rows[i + 1], [&](int j, float v) {
+  const auto add = [&](int j, float v) {
     if (v - v != 0.0f) bad = 1.0f;
     if (j != at) off += fabsf(v);
-  });
+  };
+  if constexpr (kBatched) {
+    row_values(vals, rows[i], rows[i + 1], add);
+  } else {
+    const int end = rows[i + 1];
+    for (int j = rows[i]; j < end; ++j) add(j, vals[j]);
+  }
   return diagonal_value(d, off, bad, use_l1, inverse[i]);
 }
 // amg_m_matrix_diagonal's share of fine row i (src/kutta/kernels/amg.kern.h:44-58):

@@ -376,7 +376,7 @@ __global__ void k_diagonal(int n, const int* __restrict__ rows, const int* __res
                            int use_l1, DeviceReducer red, double* check, int slot) {
   pdl_entry();
   double worst = 0;
-  ROWS(i, n) worst = nan_max(worst, diagonal_row(i, rows, diag, vals, inverse, use_l1));
+  ROWS(i, n) worst = nan_max(worst, diagonal_row<false>(i, rows, diag, vals, inverse, use_l1));
   finish_max(as_reducer(red), worst, check, slot);
 }
 
@@ -396,9 +396,13 @@ __global__ void k_prolong(int nf, const int* __restrict__ aggregate,
 // amg_galerkin :27-38: Neumaier sum over the coarse entry's fine entries. An
 // off-diagonal entry has one to a few of them, a diagonal some thirty, and a
 // warp walks as far as its longest list; so the diagonals, marked in `diagonal`
-// (a bit per entry), are summed by blocks of their own, a thread per row, or not
-// at all where the M-matrix diagonal replaces them (kDiagonals false).
-template <bool kDiagonals>
+// (a bit per entry), are summed by blocks of their own, a thread per row
+// (Diagonals::Apart), or not at all where the M-matrix diagonal replaces them
+// (Diagonals::Left). Levels of at most kApartEntries take all entries alike
+// (Diagonals::Along): 86,950 entries 4.3 us against 5.2, 251,223 6.5 against 5.3.
+enum class Diagonals { Left, Apart, Along };
+constexpr int kApartEntries = 1 << 17;
+template <Diagonals kDiagonals>
 __global__ void k_galerkin(int n_c, int nnz_c, const int* __restrict__ offsets,
                            const int* __restrict__ entries, const unsigned* __restrict__ diagonal,
                            const int* __restrict__ diag, const float* __restrict__ fine,
@@ -411,14 +415,14 @@ __global__ void k_galerkin(int n_c, int nnz_c, const int* __restrict__ offsets,
     coarse[e] = sum + error;
   };
   const int block = static_cast<int>(blockIdx.x) - diagonal_blocks;
-  if (kDiagonals && block < 0) {
+  if (kDiagonals == Diagonals::Apart && block < 0) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n_c) sum_list(diag[i]);
     return;
   }
   const int stride = (gridDim.x - diagonal_blocks) * blockDim.x;
   for (int e = block * blockDim.x + threadIdx.x; e < nnz_c; e += stride)
-    if (!(diagonal[e >> 5] >> (e & 31) & 1u)) sum_list(e);
+    if (kDiagonals == Diagonals::Along || !(diagonal[e >> 5] >> (e & 31) & 1u)) sum_list(e);
 }
 
 // The bits of the diagonal entries (words zeroed before).
@@ -872,13 +876,16 @@ void galerkin(int n_c, int nnz_c, const int* offsets, const int* entries, const 
               const int* diag, bool diagonals, const float* fine, float* coarse, cudaStream_t s) {
   if (nnz_c <= 0) return;
   ++counter;
-  const int own = diagonals ? (n_c + kBlock - 1) / kBlock : 0;
-  if (diagonals)
-    pdl(k_galerkin<true>, own + blocks(nnz_c), kBlock, 0, s, n_c, nnz_c, offsets, entries, diagonal,
-        diag, fine, coarse, own);
-  else
-    pdl(k_galerkin<false>, blocks(nnz_c), kBlock, 0, s, n_c, nnz_c, offsets, entries, diagonal, diag,
+  const auto go = [&](auto kernel, int own) {
+    pdl(kernel, own + blocks(nnz_c), kBlock, 0, s, n_c, nnz_c, offsets, entries, diagonal, diag,
         fine, coarse, own);
+  };
+  if (!diagonals)
+    go(k_galerkin<Diagonals::Left>, 0);
+  else if (nnz_c > kApartEntries)
+    go(k_galerkin<Diagonals::Apart>, (n_c + kBlock - 1) / kBlock);
+  else
+    go(k_galerkin<Diagonals::Along>, 0);
 }
 void mark_diagonals(int n, const int* diag, unsigned* words, cudaStream_t s) {
   if (n <= 0) return;

@@ -1207,8 +1207,12 @@ void Solver::refresh_levels(const float* val, bool fine_done, cudaStream_t s) {
       if (l.bf16()) p.store = l.bf16_store();
       matrix = l.val.get();
     }
+    if (i == 0 && fine_done) continue;
     // Without members the pass writes no values, so the caller's stay untouched.
-    if (i > 0 || !fine_done)
+    if (p.members == nullptr && p.surplus == nullptr && p.store.scale == nullptr)
+      launch::diagonal(l.n, l.row_ptr.get(), l.diag.get(), matrix, p.inverse, 1, reducer(),
+                       values_.get(), static_cast<int>(i), s);
+    else
       launch::level_rows(l.n, l.row_ptr.get(), l.diag.get(), const_cast<float*>(matrix), p,
                          reducer(), values_.get(), static_cast<int>(i), s);
   }

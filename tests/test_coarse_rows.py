@@ -230,6 +230,31 @@ def test_updates_queued_past_the_end_are_skipped(cuda):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("sides", [(200, 180, 1), (60, 60, 60)])
+def test_general_refresh(cuda, sides):
+    """A refresh without the M-matrix diagonal, with the first coarse level below and
+    above 131,072 entries, where its diagonals are summed apart: the oracle's values
+    bit for bit, in two launches a level and one for the levels in one block."""
+    s = harness.poisson(*sides)
+    a = L.upload(s)
+    solver = L.make_amg_solver(L.SolverKind.AmgPcg, s, L.AmgOptions())
+    solver.refresh(a)
+    launches = L.kernel_launches()
+    solver.refresh(a)
+    launches = L.kernel_launches() - launches
+    levels = solver.levels()
+    assert launches <= 2 * len(levels)
+    assert (len(levels[1][2]) > 1 << 17) == (sides[2] > 1)
+    o = O.Solver(s, O.options(O.AMG_PCG))
+    o.refresh(s.val.astype(f32))
+    want = o.levels()
+    for k, (got, ref) in enumerate(zip(levels, want, strict=True)):
+        assert np.array_equal(got[4].view(np.uint32), ref["l1"].view(np.uint32)), k
+        if k > 0:
+            assert np.array_equal(got[3].view(np.uint32), ref["val"].view(np.uint32)), k
+
+
+@pytest.mark.gpu
 def test_levels_of_long_rows_are_not_slower_than_a_thread_per_row(cuda):
     """2,000 rows of some 480 entries, where a block would add the entries of a few
     rows at a time: a sweep of the solve takes no more than 1.3 times the sweep that
