@@ -40,26 +40,62 @@ struct Assembly {
   int reference;
 };
 
-// Row i's values into `values`; returns its right-hand side.
+// Faces of a cell whose loads are issued together.
+constexpr int kFaces = 4;
+
+// Row i's values into `values`; returns its right-hand side. Bound by the loads'
+// latency, the more so as the registers of register_row leave five blocks on an SM:
+// one face after another, 1,000,000 rows took 266 us (11 entries on average) and
+// 342 (13) in a kernel of its own, 294 and 368 beside register_row, and 227 and 280
+// with four faces' loads issued together.
 __device__ __forceinline__ float assemble_row(int i, const Assembly& a,
                                               float* __restrict__ values) {
   UpperSum ap{0.0f, 0.0f};
   float b = 0.0f;
-  for (int j = a.offsets[i]; j < a.offsets[i + 1]; ++j)
-    if (a.adjacent[j] >= 0) values[a.entry[j]] = 0.0f;
-  for (int j = a.offsets[i]; j < a.offsets[i + 1]; ++j) {
-    const int f = a.faces[j], nb = a.adjacent[j];
-    const float d = a.coefficient[f];
-    b -= a.sign[j] * a.flux[f];
-    // Boundary faces and the eliminated reference cell anchor the diagonal.
-    if (nb < 0 || nb == a.reference) ap = upper_add(ap, d);
-    if (nb >= 0 && nb != a.reference && i != a.reference) values[a.entry[j]] -= d;
+  const int begin = __ldg(a.offsets + i), end = __ldg(a.offsets + i + 1);
+  for (int first = begin; first < end; first += kFaces) {
+    int entry[kFaces];
+#pragma unroll
+    for (int u = 0; u < kFaces; ++u)
+      entry[u] = first + u < end && __ldg(a.adjacent + first + u) >= 0
+                     ? __ldg(a.entry + first + u)
+                     : -1;
+#pragma unroll
+    for (int u = 0; u < kFaces; ++u)
+      if (entry[u] >= 0) values[entry[u]] = 0.0f;
+  }
+  for (int first = begin; first < end; first += kFaces) {
+    int face[kFaces], nb[kFaces], entry[kFaces];
+    float sign[kFaces], d[kFaces], flux[kFaces];
+#pragma unroll
+    for (int u = 0; u < kFaces; ++u) {
+      const bool in = first + u < end;
+      face[u] = in ? __ldg(a.faces + first + u) : -1;
+      nb[u] = in ? __ldg(a.adjacent + first + u) : -1;
+      entry[u] = in ? __ldg(a.entry + first + u) : -1;
+      sign[u] = in ? __ldg(a.sign + first + u) : 0.0f;
+    }
+#pragma unroll
+    for (int u = 0; u < kFaces; ++u) {
+      d[u] = face[u] >= 0 ? __ldg(a.coefficient + face[u]) : 0.0f;
+      flux[u] = face[u] >= 0 ? __ldg(a.flux + face[u]) : 0.0f;
+    }
+#pragma unroll
+    for (int u = 0; u < kFaces; ++u) {
+      if (face[u] < 0) continue;
+      b -= sign[u] * flux[u];
+      // Boundary faces and the eliminated reference cell anchor the diagonal.
+      if (nb[u] < 0 || nb[u] == a.reference) ap = upper_add(ap, d[u]);
+      if (nb[u] >= 0 && nb[u] != a.reference && i != a.reference) values[entry[u]] -= d[u];
+    }
   }
   // The stored off-diagonals once each (faces may share an entry), upward
   // rounded: the row stays weakly diagonally dominant.
-  for (int j = a.rows[i]; j < a.rows[i + 1]; ++j)
-    if (j != a.diag[i]) ap = upper_add(ap, -values[j]);
-  values[a.diag[i]] = i == a.reference ? 1.0f : upper_value(ap);
+  const int at = a.diag[i];
+  row_values(values, a.rows[i], a.rows[i + 1], [&](int j, float v) {
+    if (j != at) ap = upper_add(ap, -v);
+  });
+  values[at] = i == a.reference ? 1.0f : upper_value(ap);
   return i == a.reference ? 0.0f : b;
 }
 
@@ -72,7 +108,7 @@ __device__ __forceinline__ float assemble_row(int i, const Assembly& a,
 // 127 us at 1,572,864 tetrahedra with the fused parts, this 72, for 220 MB that
 // have to move. (Rows of at most six faces only: 117, as one cell in twenty there
 // has more and its warp then runs both forms.)
-constexpr int kRow = 6, kFaces = 4;
+constexpr int kRow = 6;
 template <bool kFused>
 __device__ __forceinline__ float register_row(int i, int begin, int count, int at,
                                               const Assembly& a, float* __restrict__ values,

@@ -54,7 +54,8 @@ def _device_fv(c):
 
 
 @pytest.mark.parametrize("reference", [-1, 100])
-@pytest.mark.parametrize("degree, duplicate", [(3, 0.0), (4, 0.3), (5, 0.1), (6, 0.2), (8, 0.0)])
+@pytest.mark.parametrize("degree, duplicate", [(3, 0.0), (4, 0.3), (5, 0.1), (6, 0.2), (8, 0.0),
+                                               (13, 0.2)])
 def test_assembly_rows_match_oracle_and_refresh(cuda, degree, duplicate, reference):
     """Faces below, at and above six per row, some sharing an entry, some
     entries without a face (they keep their value), some faces naming the
